@@ -38,6 +38,17 @@ extern "C" const char *qp3d_strerror(int code)
 
 extern "C" const char *qp3d_ctx_last_error(const qp3d_ctx *ctx) { return ctx ? ctx->err : ""; }
 
+static void free_defer(qp3d_ctx *ctx)
+{
+    if (ctx->dkey) cudaFree(ctx->dkey);
+    if (ctx->dval) cudaFree(ctx->dval);
+    if (ctx->dcount) cudaFree(ctx->dcount);
+    ctx->dkey = nullptr;
+    ctx->dval = nullptr;
+    ctx->dcount = nullptr;
+    ctx->defer_entries = ctx->defer_segs = 0;
+}
+
 static void free_shot(qp3d_ctx *ctx)
 {
     cudaSetDevice(ctx->device);
@@ -45,24 +56,16 @@ static void free_shot(qp3d_ctx *ctx)
                       &ctx->R8,    &ctx->W1[0], &ctx->W1[1], &ctx->W1[2], &ctx->W3[0],
                       &ctx->W3[1], &ctx->W3[2], &ctx->P[0],  &ctx->P[1],  &ctx->P[2],
                       &ctx->W21[0], &ctx->W21[1], &ctx->record, &ctx->gmax, &ctx->snap_dev,
-                      &ctx->win,   &ctx->spec_err, &ctx->am2, &ctx->av};
+                      &ctx->win,   &ctx->spec_err};
     for (float **b : bufs) {
         if (*b) cudaFree(*b);
         *b = nullptr;
     }
     if (ctx->redo) cudaFree(ctx->redo);
     if (ctx->alt_count) cudaFree(ctx->alt_count);
-    if (ctx->amask) cudaFree(ctx->amask);
-    if (ctx->apml) cudaFree(ctx->apml);
-    ctx->apml = nullptr;
-    if (ctx->alist) cudaFree(ctx->alist);
-    if (ctx->fix_count) cudaFree(ctx->fix_count);
-    ctx->fix_count = nullptr;
     ctx->redo = nullptr;
     ctx->alt_count = nullptr;
-    ctx->amask = nullptr;
-    ctx->alist = nullptr;
-    ctx->alist_cap = 0;
+    free_defer(ctx);
     __half **halves[] = {&ctx->h_vp, &ctx->h_eps, &ctx->h_del};
     for (__half **h : halves) {
         if (*h) cudaFree(*h);
@@ -162,17 +165,11 @@ static int check_geom(qp3d_ctx *ctx, const qp3d_geom *g)
     return QP3D_OK;
 }
 
-static int make_tmap(qp3d_ctx *ctx, float *base, CUtensorMap *tm)
+static int make_tmap(qp3d_ctx *ctx, float *base, TileMaps *tm)
 {
     const qp3d_geom &g = ctx->g;
-    cuuint64_t dims[3] = {(cuuint64_t)g.ny, (cuuint64_t)g.nx, (cuuint64_t)g.nz};
-    cuuint64_t strides[2] = {(cuuint64_t)ctx->ldy * 4, (cuuint64_t)ctx->plane * 4};
-    cuuint32_t box[3] = {(cuuint32_t)kBoxY, (cuuint32_t)(ctx->tile_x + 2 * kRadius), 1};
-    cuuint32_t es[3] = {1, 1, 1};
-    CUresult r = ctx->encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, es,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult r = encode_tile_maps(ctx->encode, base, g.nx, g.ny, g.nz, ctx->ldy,
+                                        ctx->tile_x, tm);
     if (r != CUDA_SUCCESS) return ctx_fail(ctx, QP3D_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return QP3D_OK;
 }
@@ -181,21 +178,37 @@ static void plan_launch(qp3d_ctx *ctx)
 {
     const qp3d_geom &g = ctx->g;
     int ncx = g.nx - 2 * kRadius;
-    int ntx = (ncx + kMaxTileX - 1) / kMaxTileX;
+    int ntx = (ncx + kStepTileX - 1) / kStepTileX;
     ctx->tile_x = (ncx + ntx - 1) / ntx;
-    if (ctx->tune_tile_x > 0) ctx->tile_x = std::min(ctx->tune_tile_x, kMaxTileX);
+    if (ctx->tune_tile_x > 0) ctx->tile_x = std::min(ctx->tune_tile_x, kStepTileX);
     ctx->nxt = (ncx + ctx->tile_x - 1) / ctx->tile_x;
     ctx->nyt = (g.ny - kRadius - 1) / kTileY + 1;   // last tile starts below ny-5
     int ncz = g.nz - 2 * kRadius;
     long long tiles = (long long)ctx->nxt * ctx->nyt;
-    long long target = 18ll * ctx->nsm;              // ~9 waves at 2 CTAs/SM
-    int nch = (int)((target + tiles - 1) / tiles);
-    int maxch = std::max(1, ncz / 24);
-    nch = std::max(1, std::min(nch, maxch));
+    ctx->smem = plane_smem_bytes(ctx->tile_x, g.pml, ctx->fuse_sources ? ctx->n_fused : 0);
+    int nch = plan_chunks(tiles, ncz, plane_threads(ctx->tile_x), ctx->smem, ctx->nsm);
     if (ctx->tune_chunks > 0) nch = std::min(ctx->tune_chunks, ncz);
     ctx->chunk_z = (ncz + nch - 1) / nch;
     ctx->nchunks = (ncz + ctx->chunk_z - 1) / ctx->chunk_z;
-    ctx->smem = plane_smem_bytes(ctx->tile_x, g.pml, ctx->fuse_sources ? ctx->n_fused : 0);
+}
+
+// Room for the deferred cells of the current launch plan: a segment per tile
+// column, a quarter of its cells (more make the step re-run exactly).  The
+// context's stream is idle when the plan changes.
+static int ensure_defer(qp3d_ctx *ctx)
+{
+    const size_t segs = (size_t)ctx->nyt * ctx->nxt * ctx->nchunks;
+    ctx->dcap = (unsigned)(ctx->tile_x * kTileY / 4 * ctx->chunk_z);
+    const size_t n = segs * ctx->dcap;
+    if (n <= ctx->defer_entries && segs <= ctx->defer_segs) return QP3D_OK;
+    CK(cudaStreamSynchronize(ctx->stream));
+    free_defer(ctx);
+    CK(cudaMalloc(&ctx->dkey, n * sizeof(uint2)));
+    CK(cudaMalloc(&ctx->dval, n * sizeof(float4)));
+    CK(cudaMalloc(&ctx->dcount, segs * sizeof(unsigned)));
+    ctx->defer_entries = n;
+    ctx->defer_segs = segs;
+    return QP3D_OK;
 }
 
 static int alloc_vol(qp3d_ctx *ctx, float **p)
@@ -243,6 +256,12 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
     ctx->vol = ctx->plane * g->nz;
     ctx->hx = g->nx - 2 * g->pml;
     ctx->hy = g->ny - 2 * g->pml;
+    // the kernels index cells with 32 bits; the state of 2^32 cells (14 volumes
+    // and the parameters) is more than the device holds anyway
+    if (ctx->vol >= (1ll << 32)) {
+        free_shot(ctx);
+        return ctx_fail(ctx, QP3D_ERR_NOMEM, "grid of %lld padded cells", ctx->vol);
+    }
 
     if (!same) {
         float **vols[] = {&ctx->U[0],  &ctx->U[1],  &ctx->U[2],  &ctx->W1[0], &ctx->W1[1],
@@ -266,21 +285,10 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
         CK(cudaMalloc(&ctx->layers, sizeof(float4) * 3 * std::max(g->pml, 1)));
         if (!ctx->errword) CK(cudaMalloc(&ctx->errword, sizeof(unsigned)));
         size_t ntb = (size_t)std::max(g->nt, 1);
-        CK(cudaMalloc(&ctx->win, 3 * ntb * sizeof(float)));
+        CK(cudaMalloc(&ctx->win, kWinFloats * ntb * sizeof(float)));
         CK(cudaMalloc(&ctx->redo, ntb * sizeof(int)));
         CK(cudaMalloc(&ctx->alt_count, ntb * sizeof(unsigned)));
         CK(cudaMalloc(&ctx->spec_err, kSpecHist * sizeof(float)));
-        // deferred cells of a speculative step: one bit per cell (vol is a
-        // multiple of 32), m2 and the alternative value at the cell's index
-        CK(cudaMalloc(&ctx->amask, (size_t)defer_mask_words(ctx->vol) * sizeof(unsigned)));
-        CK(cudaMalloc(&ctx->am2, (size_t)ctx->vol * sizeof(float)));
-        CK(cudaMalloc(&ctx->av, (size_t)ctx->vol * sizeof(float)));
-        CK(cudaMalloc(&ctx->apml, (size_t)ctx->vol * sizeof(float4)));
-        CK(cudaMalloc(&ctx->fix_count, ntb * sizeof(unsigned)));
-        // compacted list: a quarter of the cells (more deferred cells than
-        // that make the step re-run exactly)
-        ctx->alist_cap = (unsigned)std::min<long long>(std::max(1ll << 16, ctx->vol / 4), 0x7fffffff);
-        CK(cudaMalloc(&ctx->alist, (size_t)ctx->alist_cap * sizeof(unsigned)));
     }
     // vp, eps, delta go to the device in one piece each (the wavefield buffers
     // serve as staging; the reset below zeroes them) and are laid out pitched
@@ -342,6 +350,7 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
     ctx->rec_fused = g->pml >= kRadius && g->sz >= kRadius && g->sz < g->nz - kRadius &&
                      ctx->fuse_sources && ctx->n_band == 0;
     plan_launch(ctx);   // after the sources: the per-CTA source list is in shared memory
+    if ((rc = ensure_defer(ctx))) return rc;
     for (int i = 0; i < 3; ++i)
         if ((rc = make_tmap(ctx, ctx->U[i], &ctx->tm[i]))) return rc;
     ctx->loaded = true;
@@ -359,12 +368,9 @@ extern "C" int qp3d_shot_reset(qp3d_ctx *ctx)
                      ctx->W21[0], ctx->W21[1]};
     for (float *p : zero) CK(cudaMemsetAsync(p, 0, vb, ctx->stream));
     size_t ntb = (size_t)std::max(ctx->g.nt, 1);
-    CK(cudaMemsetAsync(ctx->win, 0, 3 * ntb * sizeof(float), ctx->stream));
+    CK(cudaMemsetAsync(ctx->win, 0, kWinFloats * ntb * sizeof(float), ctx->stream));
     CK(cudaMemsetAsync(ctx->redo, 0, ntb * sizeof(int), ctx->stream));
     CK(cudaMemsetAsync(ctx->alt_count, 0, ntb * sizeof(unsigned), ctx->stream));
-    CK(cudaMemsetAsync(ctx->fix_count, 0, ntb * sizeof(unsigned), ctx->stream));
-    CK(cudaMemsetAsync(ctx->amask, 0, (size_t)defer_mask_words(ctx->vol) * sizeof(unsigned),
-                       ctx->stream));
     // error history: no prediction yet (1.0 opens the widest window once)
     static const float first[kSpecHist] = {1.0f};
     CK(cudaMemcpyAsync(ctx->spec_err, first, sizeof(first), cudaMemcpyHostToDevice, ctx->stream));
@@ -376,6 +382,7 @@ extern "C" int qp3d_shot_reset(qp3d_ctx *ctx)
     ctx->step = 0;
     ctx->cur = 0;
     ctx->prev = 1;
+    ctx->win_step = -1;
     return QP3D_OK;
 }
 
@@ -385,8 +392,7 @@ constexpr int kSpecFirstStep = 3;
 
 static bool use_spec(const qp3d_ctx *ctx, int k)
 {
-    return ctx->threshold_mode == 1 && ctx->dec_mode == 0 && k >= kSpecFirstStep &&
-           ctx->vol < (1ll << 32);
+    return ctx->threshold_mode == 1 && ctx->dec_mode == 0 && k >= kSpecFirstStep;
 }
 
 // Enqueue one time step.  ev_* are optional events bracketing the main step
@@ -437,30 +443,30 @@ static int enqueue_step(qp3d_ctx *ctx, cudaEvent_t ev_g0, cudaEvent_t ev_g1, cud
 
     if (use_spec(ctx, k)) {
         p.spec = 1;
-        p.win = ctx->win + 3 * (size_t)k;
+        p.win = ctx->win + kWinFloats * (size_t)k;
+        p.win_ready = ctx->win_step == k && ctx->win_delta == ctx->delta_min &&
+                      ctx->win_bias == ctx->spec_bias;
+        p.win_next = k + 1 < g.nt ? p.win + kWinFloats : nullptr;
+        ctx->win_step = k + 1;
+        ctx->win_delta = ctx->delta_min;
+        ctx->win_bias = ctx->spec_bias;
         p.spec_err = ctx->spec_err;
         p.spec_bias = ctx->spec_bias;
-        p.amask = ctx->amask;
-        p.am2 = ctx->am2;
-        p.av = ctx->av;
-        p.apml = ctx->apml;
+        p.gate = ctx->redo + k;
+        p.dkey = ctx->dkey;
+        p.dval = ctx->dval;
+        p.dcount = ctx->dcount;
+        p.dcap = ctx->dcap;
         p.alt_count = ctx->alt_count + k;
-        p.alist = ctx->alist;
-        p.alist_cap = ctx->alist_cap;
-        p.fix_count = ctx->fix_count + k;
         if (ev_s0) CK(cudaEventRecord(ev_s0, ctx->stream));
         CKL(launch_step(ctx->tm[a], p, grid, ctx->smem, ctx->stream));
         if (ev_s1) CK(cudaEventRecord(ev_s1, ctx->stream));
         if (ev_g0) CK(cudaEventRecord(ev_g0, ctx->stream));
-        CKL(launch_compact(p, ctx->redo + k, ctx->spec_err, ctx->stream));
-        PlaneParams pe = p;
-        pe.spec = 0;
-        pe.gate = ctx->redo + k;
-        CKL(launch_fix_or_rerun(ctx->tm[a], pe, ctx->nsm, ctx->smem, ctx->stream));
+        CKL(launch_fix_or_rerun(ctx->tm[a], p, ctx->spec_err, ctx->nsm, ctx->smem, ctx->stream));
         if (ev_g1) CK(cudaEventRecord(ev_g1, ctx->stream));
     } else {
         if (ev_g0) CK(cudaEventRecord(ev_g0, ctx->stream));
-        CKL(launch_gradmax(ctx->tm[a], p, grid, ctx->smem, ctx->stream, ctx->gradmax_variant));
+        CKL(launch_gradmax(ctx->tm[a], p, grid, ctx->stream));
         if (ev_g1) CK(cudaEventRecord(ev_g1, ctx->stream));
         if (ev_s0) CK(cudaEventRecord(ev_s0, ctx->stream));
         CKL(launch_step(ctx->tm[a], p, grid, ctx->smem, ctx->stream));
@@ -522,11 +528,11 @@ int qp3d_internal_restore_step(qp3d_ctx *ctx, int step)
     if (step < 0 || step >= ctx->g.nt) return ctx_fail(ctx, QP3D_ERR_ARG, "bad step %d", step);
     const size_t n = (size_t)(ctx->g.nt - step);
     CK(cudaMemsetAsync(ctx->gmax + step, 0, n * sizeof(float), ctx->stream));
-    CK(cudaMemsetAsync(ctx->win + 3 * (size_t)step, 0, 3 * n * sizeof(float), ctx->stream));
+    CK(cudaMemsetAsync(ctx->win + kWinFloats * (size_t)step, 0, kWinFloats * n * sizeof(float), ctx->stream));
     CK(cudaMemsetAsync(ctx->redo + step, 0, n * sizeof(int), ctx->stream));
     CK(cudaMemsetAsync(ctx->alt_count + step, 0, n * sizeof(unsigned), ctx->stream));
-    CK(cudaMemsetAsync(ctx->fix_count + step, 0, n * sizeof(unsigned), ctx->stream));
     ctx->step = step;
+    ctx->win_step = -1;
     ctx->cur = (3 - step % 3) % 3;
     ctx->prev = (ctx->cur + 1) % 3;
     return QP3D_OK;
@@ -535,7 +541,7 @@ int qp3d_internal_restore_step(qp3d_ctx *ctx, int step)
 extern "C" int qp3d_shot_launches_per_step(const qp3d_ctx *ctx)
 {
     if (!ctx || !ctx->loaded) return 0;
-    int n = use_spec(ctx, ctx->step) ? 3 : 2;   // step, compaction, fix-up or re-run
+    int n = 2;   // the step kernel, and the gradmax before or the resolution after it
     if (ctx->fuse_sources) n += ctx->n_band > 0 ? 1 : 0;
     else n += ctx->n_all > 0 ? 1 : 0;
     if (!ctx->rec_fused) n += 1;
@@ -668,6 +674,7 @@ extern "C" int qp3d_shot_write_state(qp3d_ctx *ctx, int step, const float *u_pre
     CK(cudaSetDevice(ctx->device));
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->step = step;
+    ctx->win_step = -1;
     int rc;
     if (u_prev && (rc = upload_vol(ctx, ctx->U[ctx->prev], u_prev))) return rc;
     if (u_cur && (rc = upload_vol(ctx, ctx->U[ctx->cur], u_cur))) return rc;
@@ -1060,7 +1067,8 @@ extern "C" int qp3d_tune(qp3d_ctx *ctx, const char *key, int value)
         CK(cudaSetDevice(ctx->device));
         CK(cudaStreamSynchronize(ctx->stream));
         plan_launch(ctx);
-        int rc;
+        int rc = ensure_defer(ctx);
+        if (rc) return rc;
         for (int i = 0; i < 3; ++i)
             if ((rc = make_tmap(ctx, ctx->U[i], &ctx->tm[i]))) return rc;
     }

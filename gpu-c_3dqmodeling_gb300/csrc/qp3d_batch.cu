@@ -5,8 +5,9 @@
 // its own, so a shot of ~10 M cells leaves most of the GPU idle between the
 // short launches of each step.  Here all shots that fit in device memory are
 // resident at once.  Per time step there is one launch of each plane kernel
-// for all of them; its persistent CTAs take work items (one tile column of one
-// shot) from a device queue, so shots of uneven size share the SMs.  The
+// for all of them, one CTA per work item (one tile column of one shot), so
+// shots of uneven size share the SMs.  (Persistent CTAs that took the items
+// from a queue needed 164 registers, one CTA per SM, or spilled 80 bytes.)  The
 // per-step parameters of every shot are written on the device
 // (qp3d_batch_prepare_kernel), so one step is the same sequence of launches
 // for every k and the speculative steps are replayed from a captured graph.
@@ -34,9 +35,9 @@ struct Cand {
     int tile_rows;   // largest tile height (x rows)
     int zblocks;     // z blocks per tile column
 };
-constexpr Cand kCands[] = {{32, 1}, {32, 2}, {32, 4}, {16, 1}, {16, 2}};
+constexpr Cand kCands[] = {{32, 1}, {32, 2}, {32, 4}, {32, 8}, {16, 2}};
 constexpr int kNumCands = (int)(sizeof(kCands) / sizeof(kCands[0]));
-constexpr int kDefaultCand = 4;   // 16 rows: three CTAs per SM
+constexpr int kDefaultCand = 2;
 constexpr int kTuneSteps = 2;       // steps per candidate and pass (two passes)
 constexpr int kGraphSteps = 8;      // steps per captured graph
 constexpr int kSpecFirst = 3;       // as the single-shot path
@@ -49,6 +50,7 @@ struct Plan {
     long long plane = 0, vol = 0;
     std::vector<SrcEntry> src;
     size_t bytes = 0;               // device bytes of this shot
+    size_t defer_entries = 0;
     BatchShot d{};                  // device pointers, filled per group
 };
 
@@ -63,7 +65,9 @@ struct BatchState {
     int *d_ctr = nullptr;           // [0] step counter, [4..8) work queues
     WorkItem *d_work[kNumCands] = {};
     size_t work_cap[kNumCands] = {};
-    CUtensorMap *d_tm[kNumCands] = {};
+    unsigned *d_count = nullptr;    // deferred cells per work item
+    size_t count_cap = 0;
+    TileMaps *d_tm[kNumCands] = {};
     size_t tm_cap[kNumCands] = {};
     std::map<std::string, int> tuned;
     qp3d_batch_stats stats{};
@@ -76,6 +80,7 @@ void batch_free(BatchState *b)
     if (b->d_shots) cudaFree(b->d_shots);
     if (b->d_pp) cudaFree(b->d_pp);
     if (b->d_ctr) cudaFree(b->d_ctr);
+    if (b->d_count) cudaFree(b->d_count);
     for (int c = 0; c < kNumCands; ++c) {
         if (b->d_work[c]) cudaFree(b->d_work[c]);
         if (b->d_tm[c]) cudaFree(b->d_tm[c]);
@@ -115,21 +120,19 @@ void carve(Plan &s, Carver &c, size_t *zero_bytes)
     for (int i = 0; i < 2; ++i) d.W21[i] = c.take<float>(vol);
     d.record = c.take<float>(nt * s.hx * s.hy);
     d.gmax = c.take<float>(nt);
-    d.win = c.take<float>(3 * nt);
+    d.win = c.take<float>(kWinFloats * nt);
     d.redo = c.take<int>(nt);
     d.alt_count = c.take<unsigned>(nt);
-    d.fix_count = c.take<unsigned>(nt);
-    d.amask = c.take<unsigned>((size_t)defer_mask_words((long long)vol));
     if (zero_bytes) *zero_bytes = c.off - start;
     d.VP = c.take<float>(vol);
     d.E2 = c.take<float>(vol);
     d.R8 = c.take<float>(vol);
     d.spec_err = c.take<float>(kSpecHist);
-    d.am2 = c.take<float>(vol);
-    d.av = c.take<float>(vol);
-    d.apml = c.take<float4>(vol);
-    d.alist_cap = (unsigned)std::min<size_t>(std::max<size_t>(1u << 16, vol / 4), 0x7fffffff);
-    d.alist = c.take<unsigned>(d.alist_cap);
+    // deferred cells: a quarter of the cells of every tile column, whatever the
+    // tile height (columns reach at most one tile past the volume)
+    s.defer_entries = (size_t)(s.g.nx + kMaxTileX) * s.ldy / 4 * s.g.nz;
+    d.dkey = c.take<uint2>(s.defer_entries);
+    d.dval = c.take<float4>(s.defer_entries);
     d.layers = c.take<float4>(3 * (size_t)std::max(s.g.pml, 1));
     d.wavelet = c.take<float>(nt);
     d.src = c.take<SrcEntry>(std::max<size_t>(s.src.size(), 1));
@@ -142,16 +145,10 @@ int tile_height(int nx, int rows)
     return (ncx + ntx - 1) / ntx;
 }
 
-int make_tmap(qp3d_ctx *ctx, const Plan &s, float *base, int tile_x, CUtensorMap *tm)
+int make_tmap(qp3d_ctx *ctx, const Plan &s, float *base, int tile_x, TileMaps *tm)
 {
-    cuuint64_t dims[3] = {(cuuint64_t)s.g.ny, (cuuint64_t)s.g.nx, (cuuint64_t)s.g.nz};
-    cuuint64_t strides[2] = {(cuuint64_t)s.ldy * 4, (cuuint64_t)s.plane * 4};
-    cuuint32_t box[3] = {(cuuint32_t)kBoxY, (cuuint32_t)(tile_x + 2 * kRadius), 1};
-    cuuint32_t es[3] = {1, 1, 1};
-    CUresult r = ctx->encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, es,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult r = encode_tile_maps(ctx->encode, base, s.g.nx, s.g.ny, s.g.nz, s.ldy, tile_x,
+                                        tm);
     if (r != CUDA_SUCCESS)
         return ctx_fail(ctx, QP3D_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return QP3D_OK;
@@ -186,11 +183,10 @@ class Runner {
     BatchState *B;
     Launch L[kNumCands];
     int nshots = 0;
-    long long max_words = 0;   // largest deferred-cell bitmask of the group
     Coefs coefs{};
 
     int build_candidate(int c, std::vector<Plan *> &G);
-    BatchArgs args(int c, int queue) const
+    BatchArgs args(int c, int queue, bool spec) const
     {
         BatchArgs a;
         a.k = coefs;
@@ -198,6 +194,9 @@ class Runner {
         a.tm = B->d_tm[c];
         a.work = B->d_work[c];
         a.nwork = L[c].nwork;
+        a.dcount = B->d_count;
+        a.nshots = nshots;
+        a.spec = spec ? 1 : 0;
         a.queue = B->d_ctr + 4 + queue;
         a.arith = ctx->arith;
         return a;
@@ -208,7 +207,7 @@ class Runner {
 int Runner::build_candidate(int c, std::vector<Plan *> &G)
 {
     std::vector<WorkItem> items;
-    std::vector<CUtensorMap> tms(3 * G.size());
+    std::vector<TileMaps> tms(3 * G.size());
     int max_tile = 1;
     size_t smem = 0;
     for (size_t s = 0; s < G.size(); ++s) {
@@ -221,6 +220,7 @@ int Runner::build_candidate(int c, std::vector<Plan *> &G)
         const int ncz = P.g.nz - 2 * kRadius;
         const int zb = std::min(kCands[c].zblocks, ncz);
         const int cz = (ncz + zb - 1) / zb;
+        size_t dbase = 0;
         for (int z0 = kRadius; z0 < P.g.nz - kRadius; z0 += cz)
             for (int xt = 0; xt < nxt; ++xt)
                 for (int yt = 0; yt < nyt; ++yt) {
@@ -231,8 +231,13 @@ int Runner::build_candidate(int c, std::vector<Plan *> &G)
                     w.x0 = kRadius + xt * tx;
                     w.z0 = z0;
                     w.z1 = std::min(z0 + cz, P.g.nz - kRadius);
+                    w.dcap = (unsigned)(tx * kTileY / 4 * (w.z1 - w.z0));
+                    w.dbase = (unsigned)dbase;
+                    dbase += w.dcap;
                     items.push_back(w);
                 }
+        if (dbase > P.defer_entries)
+            return ctx_fail(ctx, QP3D_ERR_STATE, "deferred-cell list too small");
         for (int i = 0; i < 3; ++i) {
             int rc = make_tmap(ctx, P, P.d.U[i], tx, &tms[3 * s + i]);
             if (rc) return rc;
@@ -244,20 +249,18 @@ int Runner::build_candidate(int c, std::vector<Plan *> &G)
     });
     int rc;
     if ((rc = ensure(ctx, &B->d_work[c], &B->work_cap[c], items.size())) ||
+        (rc = ensure(ctx, &B->d_count, &B->count_cap, items.size())) ||
         (rc = ensure(ctx, &B->d_tm[c], &B->tm_cap[c], tms.size())))
         return rc;
     CK(cudaMemcpyAsync(B->d_work[c], items.data(), items.size() * sizeof(WorkItem),
                        cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(B->d_tm[c], tms.data(), tms.size() * sizeof(CUtensorMap),
+    CK(cudaMemcpyAsync(B->d_tm[c], tms.data(), tms.size() * sizeof(TileMaps),
                        cudaMemcpyHostToDevice, ctx->stream));
     Launch &l = L[c];
     l.nwork = (int)items.size();
-    l.threads = batch_plane_threads(max_tile);
+    l.threads = plane_threads(max_tile);
     l.smem = smem;
-    int per_sm = 0;
-    CK(batch_ctas_per_sm(2, ctx->arith, l.threads, l.smem, &per_sm));
-    if (per_sm < 1) return ctx_fail(ctx, QP3D_ERR_CUDA, "batched step kernel does not fit an SM");
-    l.grid = std::max(1, std::min(l.nwork, per_sm * ctx->nsm));
+    l.grid = 2 * ctx->nsm;   // what one wave of the resolution holds
     return QP3D_OK;
 }
 
@@ -267,14 +270,11 @@ int Runner::enqueue_step(int c, bool spec)
     CKL(launch_batch_prepare(B->d_shots, nshots, B->d_pp, B->d_ctr, B->d_ctr + 4, spec ? 1 : 0,
                              ctx->stream));
     if (spec) {
-        CKL(launch_batch_plane(2, args(c, 1), l.grid, l.threads, l.smem, ctx->stream));
-        const int per_shot = std::max(2, 8 * ctx->nsm / std::max(nshots, 1));
-        CKL(launch_batch_fixup(args(c, 1), nshots, per_shot, max_words, ctx->stream));
-        ctx->launches += 1;   // compaction and fix-up
-        CKL(launch_batch_plane(1, args(c, 2), l.grid, l.threads, l.smem, ctx->stream));
+        CKL(launch_batch_plane(2, args(c, 1, true), l.threads, l.smem, ctx->stream));
+        CKL(launch_batch_resolve(args(c, 2, true), l.grid, l.threads, l.smem, ctx->stream));
     } else {
-        CKL(launch_batch_plane(0, args(c, 0), l.grid, l.threads, l.smem, ctx->stream));
-        CKL(launch_batch_plane(1, args(c, 1), l.grid, l.threads, l.smem, ctx->stream));
+        CKL(launch_batch_plane(0, args(c, 0, false), l.threads, l.smem, ctx->stream));
+        CKL(launch_batch_plane(1, args(c, 1, false), l.threads, l.smem, ctx->stream));
     }
     return QP3D_OK;
 }
@@ -284,8 +284,6 @@ int Runner::run_group(std::vector<Plan *> &G, const Coefs &kc, const qp3d_shot *
     int rc;
     nshots = (int)G.size();
     coefs = kc;
-    max_words = 0;
-    for (Plan *p : G) max_words = std::max(max_words, defer_mask_words(p->vol));
     // ---- device memory: one arena for the group
     size_t total = 0;
     for (Plan *p : G) total += p->bytes;

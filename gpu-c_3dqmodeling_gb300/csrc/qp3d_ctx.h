@@ -18,18 +18,13 @@ struct AdjState;                   // qp3d_adjoint.cu
 void adjoint_free(AdjState *s);
 }  // namespace qp3d
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 struct qp3d_ctx {
     int device = 0;
     int nsm = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;   // record pieces to page-locked host memory
     cudaEvent_t copy_ev = nullptr;
-    EncodeTiledFn encode = nullptr;
+    qp3d::EncodeTiledFn encode = nullptr;
     char err[512] = {0};
 
     // shot
@@ -49,22 +44,24 @@ struct qp3d_ctx {
     float *record = nullptr;
     float *gmax = nullptr;
     // speculative threshold: per-step window, re-run flags, deferred-cell counts
-    float *win = nullptr;
+    float *win = nullptr;            // kWinFloats per step
+    int win_step = -1;               // the step whose window the last one left behind,
+    float win_delta = 0.0f, win_bias = 0.0f;   // under these settings
     int *redo = nullptr;
     unsigned *alt_count = nullptr;
     float *spec_err = nullptr;
-    unsigned *amask = nullptr;       // deferred-cell bits, vol / 32 words
-    float *am2 = nullptr, *av = nullptr;
-    float4 *apml = nullptr;
-    unsigned *fix_count = nullptr;   // per step: deferred cells below the threshold
-    unsigned *alist = nullptr;       // compacted deferred cells
-    unsigned alist_cap = 0;
+    // deferred cells of a speculative step, one segment per tile column
+    uint2 *dkey = nullptr;
+    float4 *dval = nullptr;
+    unsigned *dcount = nullptr;      // lengths of the segments
+    unsigned dcap = 0;               // entries per segment
+    size_t defer_entries = 0, defer_segs = 0;   // allocated
     float4 *layers = nullptr;
     qp3d::SrcEntry *src_fused = nullptr, *src_band = nullptr, *src_all = nullptr;
     int n_fused = 0, n_band = 0, n_all = 0;
     bool fuse_sources = true;
     unsigned *errword = nullptr;
-    CUtensorMap tm[3];
+    qp3d::TileMaps tm[3];
     qp3d::Coefs coefs{};
     std::vector<float> wavelet;
     int step = 0;

@@ -27,22 +27,27 @@ constexpr int kRadius = 5;        // 10th-order stencil (M/2 with M = 10)
 constexpr int kTileY = 32;        // y cells per tile = 8 quads of 4 cells
 constexpr int kQuadsY = kTileY / 4;
 constexpr int kHaloY = 8;         // y halo rounded up to 16 bytes
-constexpr int kBoxY = kTileY + 2 * kHaloY;   // 48 floats per staged row
-// Planes loaded ahead of use.  One is enough to cover the TMA latency; every
-// further slot costs 8 KB of shared memory per CTA, and the L1 share of the
-// SM (where the per-cell global loads wait for DRAM) shrinks with it: two
-// CTAs of 32-row tiles with a 12-slot ring fit the 196 KiB shared-memory
-// carveout (60 KiB left for L1), a 13-slot ring needs the 228 KiB carveout
-// (28 KiB of L1) and runs the step about 17% slower.
-constexpr int kPrefetch = 1;
-constexpr int kRing = 2 * kRadius + 1 + kPrefetch;   // staged planes
+constexpr int kBoxY = kTileY + 2 * kHaloY;   // 48 floats per staged halo row
+// Load groups in flight or in use: the current plane's and two ahead.  One
+// ahead leaves the load's latency open whenever the warps of a CTA drift.
+constexpr int kGroups = 2;
+constexpr int kRingZ = 2 * kRadius + kGroups;   // own-cell planes staged
 constexpr int kMaxTileX = 32;
 constexpr int kThreads = kQuadsY * kMaxTileX;        // 256
+constexpr int kStepTileX = 32;   // largest tile height of the step kernels
+constexpr int kStepThreads = kQuadsY * kStepTileX;
 constexpr int kMaxFusedSources = 64;
 // Relative prediction errors of the step max kept for the speculative window
 // (most recent first).
 constexpr int kSpecHist = 8;
 constexpr int kMaxPml = 256;
+constexpr int kWinFloats = 5;
+
+// The two tensor maps of a wavefield buffer: boxes of the tile's own cells and
+// of the tile with its halo.
+struct TileMaps {
+    CUtensorMap z, c;
+};
 
 // Error bits written to the device error word.
 constexpr unsigned kErrWaitTimeout = 1u;
@@ -71,11 +76,6 @@ struct SrcEntry {
     int x, y, z;
     float v;
 };
-
-// Words of the deferred-cell bitmask of a volume of vol cells (vol is a
-// multiple of 32), rounded up to a multiple of 4 for 16-byte loads; the
-// padding words stay zero.
-__host__ __device__ inline long long defer_mask_words(long long vol) { return ((vol >> 5) + 3) & ~3ll; }
 
 struct PlaneParams {
     // geometry
@@ -110,9 +110,10 @@ struct PlaneParams {
     const SrcEntry *src;      // sources inside the updated box, fused
     int nsrc;
     unsigned *err;
-    // threshold decisions of the step, one bit per cell in the layout of amask
-    // (exact steps only): written to dec_out, or read from dec_in instead of
-    // being taken (the gradient's recomputation replays the forward's)
+    // threshold decisions of the step, one bit per cell, 32 y cells a word
+    // (word = pitched index / 32; exact steps only): written to dec_out, or
+    // read from dec_in instead of being taken (the gradient's recomputation
+    // replays the forward's)
     unsigned *dec_out;
     const unsigned *dec_in;
     unsigned long long wait_ns;   // limit of every bounded device wait (0: 2 s)
@@ -120,23 +121,25 @@ struct PlaneParams {
                               // never loaded, so its waits run out (0: none)
     // threshold handling of the step kernel
     int spec;                 // 1: predicted window, own max, deferred cells
-    const int *gate;          // exact mode: run only if *gate != 0 (null: always)
-    float *win;               // spec: &win[3*step] = (M_lo, M_hi, M_pred)
+    const int *gate;          // spec: set to 1 when the step has to be re-run (null: not
+                              // speculative)
+    float *win;               // spec: kWinFloats of the step: M_lo, M_hi, M_pred and the
+                              // thresholds of m2 at M_lo and M_hi
+    int win_ready;            // 1: all five are there already
+    float *win_next;          // where the resolution leaves the next step's (or null)
     const float *spec_err;    // kSpecHist last relative prediction errors of the max
     float delta_min;          // smallest half-width of the window
     float spec_bias;          // relative shift of the window (test hook, 0)
-    // Cells whose decision waits for the exact max of the step ("deferred"):
-    // one bit per cell, 32 y-cells per word (word = pitched index / 32), and
-    // at the cell's own index its m2 and its alternative value: u(k+1) with
-    // S = 1 (source included); a PML cell also keeps the split-field outputs
-    // of S = 1 {w13, w21, w33, p3} in apml.
-    unsigned *amask;
-    float *am2, *av;
-    float4 *apml;
-    unsigned *alt_count;      // &alt_count[step]: deferred cells (compaction)
-    unsigned *fix_count;      // &fix_count[step]: of them below the threshold
-    unsigned *alist;          // their pitched indices (compaction -> fix-up)
-    unsigned alist_cap;
+    // Cells whose decision waits for the exact max of the step ("deferred"),
+    // listed by the column that holds them in a segment of its own: pitched
+    // index and m2, and what gives the cell its S = 1 results: u(k+1) with
+    // S = 1 without the source, or of a PML cell the three derivative terms of
+    // its update (its other inputs are still in place).
+    uint2 *dkey;
+    float4 *dval;
+    unsigned *dcount;         // cells listed per column (grid launches)
+    unsigned dcap;            // entries per segment (grid launches)
+    unsigned *alt_count;      // &alt_count[step]: deferred cells
     // batched launches only
     int ucur;                 // index of u(k) among the shot's three buffers
     int active;               // 0 once the shot has run all its steps
@@ -158,16 +161,12 @@ struct BatchShot {
     const SrcEntry *src;
     int nsrc;
     const float *wavelet;     // nt samples
-    float *win;               // 3 * nt
+    float *win;               // kWinFloats * nt
     int *redo;                // nt
     unsigned *alt_count;      // nt
     float *spec_err;
-    unsigned *amask;          // vol / 32 words
-    float *am2, *av;          // vol each
-    float4 *apml;             // vol
-    unsigned *fix_count;      // nt
-    unsigned *alist;          // alist_cap entries
-    unsigned alist_cap;
+    uint2 *dkey;              // deferred cells (see PlaneParams), all columns
+    float4 *dval;
     float spec_bias;
     unsigned *err;
 };
@@ -175,6 +174,7 @@ struct BatchShot {
 // A unit of work of a batched launch: one tile column of one shot.
 struct WorkItem {
     int shot, tile_x, y0, x0, z0, z1;
+    unsigned dcap, dbase;     // its segment of the shot's deferred-cell list
 };
 
 // Kernel arguments of the batched plane kernels.  The coefficient tables are
@@ -182,9 +182,11 @@ struct WorkItem {
 struct BatchArgs {
     Coefs k;
     const PlaneParams *pp;    // per shot, the current step
-    const CUtensorMap *tm;    // per shot three maps (one per u buffer)
+    const TileMaps *tm;       // per shot three pairs of maps (one per u buffer)
     const WorkItem *work;
     int nwork;
+    unsigned *dcount;         // deferred cells per work item
+    int nshots, spec;
     int *queue;               // next work item (zeroed by the prepare kernel)
     int arith;                // Arith of every shot of the batch
 };
@@ -220,18 +222,15 @@ cudaError_t launch_from_bf16(const __nv_bfloat16 *h, float *a, long long n, cuda
 
 // Launchers (qp3d_kernels.cu).  All enqueue on `stream` and return the
 // launch error.
-cudaError_t launch_gradmax(const CUtensorMap &tm_u, const PlaneParams &p,
-                           dim3 grid, size_t smem, cudaStream_t stream, int variant);
-cudaError_t launch_step(const CUtensorMap &tm_u, const PlaneParams &p,
-                        dim3 grid, size_t smem, cudaStream_t stream);
-// Speculative step resolution: compaction of the deferred-cell bitmask into a
-// list, then the fix-up of the listed cells.
-// resolution and compaction of a speculative step, then its fix-up or (when
-// the max fell outside the window) its exact re-run, a persistent grid of
-// nsm CTAs
-cudaError_t launch_compact(const PlaneParams &p, int *redo, float *spec_err, cudaStream_t stream);
-cudaError_t launch_fix_or_rerun(const CUtensorMap &tm_u, const PlaneParams &p, int nsm,
-                                size_t smem, cudaStream_t stream);
+cudaError_t launch_gradmax(const TileMaps &tm, const PlaneParams &p, dim3 grid,
+                           cudaStream_t stream);
+cudaError_t launch_step(const TileMaps &tm, const PlaneParams &p, dim3 grid, size_t smem,
+                        cudaStream_t stream);
+// resolution of a speculative step: the fix-up of its deferred cells or (when
+// the max fell outside the window) its exact re-run, a persistent grid of nsm
+// CTAs
+cudaError_t launch_fix_or_rerun(const TileMaps &tm, const PlaneParams &p, float *spec_err,
+                                int nsm, size_t smem, cudaStream_t stream);
 cudaError_t launch_band_sources(float *u_new, const float *u_cur,
                                 const SrcEntry *src, int n, long long plane,
                                 int ldy, float w, cudaStream_t stream);
@@ -257,25 +256,56 @@ cudaError_t launch_to_half_dense(const float *a, __half *h, int nx, int ny, int 
 // Every non-zero sample of a dense [nz][nx][ny] source volume, in index order
 // (z, then x, then y), scanned by several host threads.
 void scan_source_volume(const float *s, int nx, int ny, int nz, std::vector<SrcEntry> &out);
-// Dynamic shared memory of a plane kernel; nsrc = fused sources of the shot
-// (the per-CTA source list has room for all of them).
-size_t plane_smem_bytes(int tile_x, int pml, int nsrc = kMaxFusedSources);
+// Dynamic shared memory of a step kernel; nsrc = fused sources of the shot
+// (the per-CTA source list has room for all of them); and of a gradmax kernel.
+size_t plane_smem_bytes(int tile_x, int pml, int nsrc);
+size_t gradmax_smem_bytes(int tile_x);
+// The tensor maps of a pitched [nz][nx][ldy] wavefield for tiles of tile_x
+// rows (cuTensorMapEncodeTiled's result).
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
+                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline CUresult encode_tile_maps(EncodeTiledFn encode, const float *base, int nx, int ny, int nz,
+                                 int ldy, int tile_x, TileMaps *tm)
+{
+    cuuint64_t dims[3] = {(cuuint64_t)ny, (cuuint64_t)nx, (cuuint64_t)nz};
+    cuuint64_t strides[2] = {(cuuint64_t)ldy * 4, (cuuint64_t)ldy * 4 * nx};
+    cuuint32_t zbox[3] = {(cuuint32_t)kTileY, (cuuint32_t)tile_x, 1};
+    cuuint32_t cbox[3] = {(cuuint32_t)kBoxY, (cuuint32_t)(tile_x + 2 * kRadius), 1};
+    cuuint32_t es[3] = {1, 1, 1};
+    CUresult r = CUDA_SUCCESS;
+    for (int i = 0; i < 2 && r == CUDA_SUCCESS; ++i)
+        r = encode(i ? &tm->c : &tm->z, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
+                   const_cast<float *>(base), dims, strides, i ? cbox : zbox, es,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r;
+}
 
-// Batched launches (persistent CTAs pulling work items).  kind: 0 gradmax,
-// 1 exact step (gated per shot), 2 speculative step.
+// Batched launches.  kind: 0 gradmax, 1 exact step, 2 speculative step; the
+// resolution of a speculative step runs on grid persistent CTAs.
 size_t batch_smem_bytes(int tile_x, int pml, int nsrc);
 cudaError_t launch_batch_prepare(const BatchShot *shots, int nshots, PlaneParams *pp, int *ctr,
                                  int *queues, int spec, cudaStream_t stream);
-cudaError_t launch_batch_plane(int kind, const BatchArgs &b, int grid, int threads, size_t smem,
+cudaError_t launch_batch_plane(int kind, const BatchArgs &b, int threads, size_t smem,
                                cudaStream_t stream);
-cudaError_t launch_batch_fixup(const BatchArgs &b, int nshots, int blocks_per_shot,
-                               long long max_words, cudaStream_t stream);
-int batch_plane_threads(int tile_x);
-cudaError_t batch_ctas_per_sm(int kind, int arith, int threads, size_t smem, int *n);
-cudaError_t configure_gradmax_partial();
-cudaError_t launch_gradmax_partial(const CUtensorMap &tm_u, const PlaneParams &p, dim3 grid,
-                                   size_t smem, cudaStream_t stream, float *partial,
-                                   unsigned nblocks, float *out);
+cudaError_t launch_batch_resolve(const BatchArgs &b, int grid, int threads, size_t smem,
+                                 cudaStream_t stream);
+// max|grad u| in one launch: sc starts zero and is left zero, out receives the
+// maximum (NaN on a timed-out wait) and *host_flags (mapped) the error bits.
+struct GradmaxScratch {
+    unsigned max_bits, done, err;
+};
+cudaError_t configure_gradmax_single();
+cudaError_t launch_gradmax_single(const TileMaps &tm, const PlaneParams &p, dim3 grid,
+                                  cudaStream_t stream, GradmaxScratch *sc, float *out,
+                                  unsigned *host_flags);
+// threads of a plane kernel's CTA: whole warps; rows past tile_x are idle, so
+// every warp collective sees 32 lanes
+__host__ __device__ inline int plane_threads(int tile_x) { return (kQuadsY * tile_x + 31) & ~31; }
+// z chunks of a plane kernel's grid
+int plan_chunks(long long tiles, int ncz, int threads, size_t smem, int nsm);
 cudaError_t configure_kernels();
 
 }  // namespace qp3d

@@ -18,20 +18,28 @@
 //                         updated: either qp3d_gradmax_kernel computes it
 //                         first (GPU_kernel.cu:14-33 + CPU_function.c:10-22),
 //                         or the step runs speculatively with a predicted
-//                         window and qp3d_resolve / compact / fixup_kernel
-//                         settle the cells whose decision waited (a gated
-//                         exact re-run when the prediction missed).
+//                         window and qp3d_fix_or_rerun_kernel settles the
+//                         cells whose decision waited (an exact re-run when
+//                         the prediction missed).
 //
-// The same tile bodies run in the batched persistent kernels (many shots per
-// launch), and the adjoint kernels at the end of the file transpose the step.
+// The same tile bodies run in the batched kernels (many shots per launch),
+// and the adjoint kernels at the end of the file transpose the step.
 //
 // Both kernels march along z.  A CTA owns a tile of tile_x rows (x) by 32
 // cells (y) and a chunk of z planes.  Each thread owns one row and four
-// consecutive y cells (a "quad", one float4).  Planes of u(k), with a 5-row
-// and 8-column halo, are staged into a ring of kRing shared-memory slots by
-// TMA (cp.async.bulk.tensor.3d) and completed on one mbarrier per slot; the
-// stencil reads all 30 taps from shared memory.  Loads of the next planes
-// overlap the arithmetic of the current one.
+// consecutive y cells (a "quad", one float4).  Planes of u(k) are staged by
+// TMA (cp.async.bulk.tensor.3d) into two rings in shared memory, the tile's
+// own cells for the z taps and the current plane with its halo for the x and
+// y taps (see Pipe); the stencil reads all 30 taps from shared memory.
+//
+// What bounds the step: instruction issue and its latencies at 16 warps an SM
+// (128 registers a thread), beside HBM on large grids.  Instructions per warp
+// and plane (four rows by 32 cells; 240x240x190 cells, 20-cell shell) went
+// from 764 to 652, 582 on a grid with a 6-cell shell, of which the stencil is
+// 240: the shell's update has a loop body of its own, per axis and in FP32x2
+// pairs; the threshold decides warps before cells; deferred cells are listed
+// on the side; the sources and the receiver plane are handled after the loop.
+// 460x460x360: 623 -> 531 us a step kernel (75% of the DRAM peak by ncu).
 //
 // Arithmetic.  The 1/h factors of the reference (each tap divided by dx or
 // dx*dx, CPU_function.c:314-316,393-395) are folded into the coefficient
@@ -45,6 +53,9 @@
 #include "qp3d_exact.h"
 
 #include <math.h>
+
+#include <algorithm>
+#include <type_traits>
 
 namespace qp3d {
 
@@ -121,6 +132,34 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *tm, in
         : "memory");
 }
 
+// 16 (8) bytes global -> shared, past L1, for the thread's own use after
+// cp_async_wait
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// Programmatic dependent launch: the kernels of a time step are launched with
+// cudaLaunchAttributeProgrammaticStreamSerialization.  Each lets its successor
+// start as soon as its own CTAs have, and waits for its predecessor to finish
+// before it touches anything a step writes; what comes before the wait may
+// only read data that no step changes.
+__device__ __forceinline__ void pdl_trigger()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ float4 lds4(const float *p)
 {
     return *reinterpret_cast<const float4 *>(p);
@@ -132,36 +171,81 @@ __device__ __forceinline__ float f4(const float4 &v, int j)
 }
 
 // ---------------------------------------------------------------------------
-// Shared-memory layout of both plane kernels
+// Shared-memory layout of the plane kernels
 // ---------------------------------------------------------------------------
 struct SmemLayout {
-    size_t slot_floats;   // one staged plane, padded to 128 B
-    size_t ring_bytes;
-    size_t bar_off;       // kRing mbarriers
-    size_t tab_off;       // 3 * pml float4 layer coefficients
+    int zslot, cslot;     // floats of one own-cell plane and one halo plane
+    size_t c_off;         // halo planes (the own-cell planes start at 0)
+    size_t own_off;       // per-thread stream slots (step kernels)
+    size_t bar_off;       // kGroups mbarriers
+    size_t cnt_off;       // kGroups arrival counters, then the issued count
+    size_t tab_off;       // layer coefficients: [3][pml] float4 (x, y, z faces)
+    size_t ytab_off;      // those of the tile's y cells, [4][kTileY] floats
     size_t src_off;       // fused source entries of this CTA
     size_t misc_off;      // scalars
     size_t total;
 };
 
-__host__ __device__ inline SmemLayout smem_layout(int tile_x, int pml,
-                                                  int nsrc = kMaxFusedSources)
+// streams: 16-byte slots per thread (0 for the gradmax kernels)
+__host__ __device__ inline SmemLayout smem_layout(int tile_x, int pml, int nsrc, int streams)
 {
     SmemLayout L;
-    size_t box = (size_t)(tile_x + 2 * kRadius) * kBoxY;
-    L.slot_floats = (box + 31) & ~(size_t)31;
-    L.ring_bytes = L.slot_floats * 4 * kRing;
-    L.bar_off = L.ring_bytes;
-    L.tab_off = L.bar_off + 16 * kRing;   // full[kRing], empty[kRing]
-    L.tab_off = (L.tab_off + 15) & ~(size_t)15;
-    L.src_off = L.tab_off + 16 * 3 * (size_t)(pml > 0 ? pml : 1);
-    L.misc_off = L.src_off + sizeof(SrcEntry) * (size_t)(nsrc > 0 ? nsrc : 1);
+    L.zslot = tile_x * kTileY;
+    L.cslot = ((tile_x + 2 * kRadius) * kBoxY + 31) & ~31;
+    L.c_off = (size_t)L.zslot * 4 * kRingZ;
+    L.own_off = L.c_off + (size_t)L.cslot * 4 * kGroups;
+    L.bar_off = L.own_off + (size_t)plane_threads(tile_x) * 16 * streams;
+    L.cnt_off = L.bar_off + 8 * kGroups;
+    L.tab_off = (L.cnt_off + 4 * (kGroups + 1) + 15) & ~(size_t)15;
+    L.ytab_off = L.tab_off + (streams ? 16 * 3 * (size_t)(pml > 0 ? pml : 1) : 0);
+    L.src_off = L.ytab_off + (streams ? 16 * kTileY : 0);
+    L.misc_off = L.src_off + (streams ? sizeof(SrcEntry) * (size_t)(nsrc > 0 ? nsrc : 1) : 0);
     L.misc_off = (L.misc_off + 15) & ~(size_t)15;
     L.total = L.misc_off + 64;
     return L;
 }
 
-size_t plane_smem_bytes(int tile_x, int pml, int nsrc) { return smem_layout(tile_x, pml, nsrc).total; }
+// Streams of the step kernels: u(k-1), vp, 2 eps, 8 (eps - delta), and where
+// there is a PML shell the seven split-field values a PML cell reads.
+__host__ __device__ inline int step_streams(int pml) { return pml > 0 ? 11 : 4; }
+
+size_t plane_smem_bytes(int tile_x, int pml, int nsrc)
+{
+    return smem_layout(tile_x, pml, nsrc, step_streams(pml)).total;
+}
+
+size_t gradmax_smem_bytes(int tile_x) { return smem_layout(tile_x, 0, 0, 0).total; }
+
+// The number of z chunks of a plane kernel's grid: tiles columns of ncz planes,
+// smem bytes a CTA.  A CTA's march over its planes is a serial chain (2-3 us a
+// plane when two CTAs share an SM), so a grid too small to fill the SMs takes
+// as long as its longest chunk, and one that fills them a little more than
+// once takes two of them.  The estimate below, in planes, follows what was
+// measured on 140^3, 191x127x105, 240x240x190 and 460x460x360 cells over 4 to
+// 26 chunks: half-filled SMs run a plane 0.7 times as long; up to one wave
+// costs its chunk and 1.5 planes of start-up; more waves overlap, at half a
+// plane each and a third of a wave for the uneven end; the last factor is the
+// re-read of ten planes a chunk.  Before (24 planes or more a chunk, 18 CTAs
+// an SM) 140^3 took 63 us a step, now 43.
+int plan_chunks(long long tiles, int ncz, int threads, size_t smem, int nsm)
+{
+    const int per_sm = std::max(1, std::min((int)(227 * 1024 / (smem + 1024)), 512 / threads));
+    const double slots = (double)per_sm * nsm;
+    int best = 1;
+    double best_t = 0.0;
+    for (int n = 1; n <= ncz && (n == 1 || tiles * n <= 64 * (long long)slots); ++n) {
+        const int chunk = (ncz + n - 1) / n;
+        if ((ncz + chunk - 1) / chunk != n) continue;   // the same chunks with fewer
+        const double w = (double)tiles * n / slots;
+        const double waves = w <= 0.5 ? 0.7 : (w <= 1.0 ? 1.0 : w + 0.35);
+        const double t = waves * (chunk + (w <= 1.0 ? 1.5 : 0.5)) * (1.0 + 0.5 / chunk);
+        if (n == 1 || t < best_t) {
+            best = n;
+            best_t = t;
+        }
+    }
+    return best;
+}
 
 // ---------------------------------------------------------------------------
 // Threshold of the scalar operator, GPU_kernel.cu:99.
@@ -197,15 +281,6 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b)
     return __fadd2_rn(a, make_float2(-b.x, -b.y));
 }
 
-// slot of staged plane (base + d), base already reduced modulo kRing
-__device__ __forceinline__ int slot_add(int s, int d)
-{
-    s += d;
-    if (s >= kRing) s -= kRing;
-    if (s < 0) s += kRing;
-    return s;
-}
-
 // One second-difference tap in the reference's form, (u[+m] - 2u) + u[-m]
 // (CPU_function.c:393-395), two cells at a time.  Summing c2[m] times these
 // keeps a constant field's Laplacian exactly zero; the form with the centre
@@ -218,23 +293,31 @@ __device__ __forceinline__ float2 lap_tap2(float2 a, float2 b, float2 u0)
     return __fadd2_rn(__ffma2_rn(make_float2(-2.0f, -2.0f), u0, a), b);
 }
 
+// Where a quad finds its taps: pc, its first cell in the halo plane of the
+// current z (x and y taps), and za, its first cell in the own-cell plane z - 5
+// (z taps); the planes after it follow at zslot floats each, those past the
+// last slot (from the wrap-th on) one ring length (zlen) back.
+struct Taps {
+    const float *pc, *za;
+    int wrap, zslot, zlen;
+};
+
+__device__ __forceinline__ float4 ztap(const Taps &T, int j)   // plane z - 5 + j
+{
+    return lds4((j < T.wrap ? T.za : T.za - T.zlen) + j * T.zslot);
+}
+
 template <bool SECOND>
-__device__ __forceinline__ void quad_derivs(const float *ring, size_t slot_floats, int t, int rc,
-                                            const Coefs &k, float Ux[4], float Uy[4],
-                                            float Uz[4], float Uxx[4], float Uyy[4],
+__device__ __forceinline__ void quad_derivs(const Taps &T, const Coefs &k, float Ux[4],
+                                            float Uy[4], float Uz[4], float Uxx[4], float Uyy[4],
                                             float Uzz[4], float u0[4])
 {
-    const int sc = (t + kRadius) % kRing;
-    const float *pc = ring + (size_t)sc * slot_floats;
-    // the z taps: planes sc +- (m + 1) of the ring, wrapped by one ring length
-    const float *pcr = pc + rc;
-    const float *pcr_lo = pcr - kRing * (int)slot_floats;
-    const float *pcr_hi = pcr + kRing * (int)slot_floats;
+    const float *pc = T.pc;
     // y taps: columns c-8 .. c+11 of the centre plane
     float Y[20];
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
-        float4 v = lds4(pc + rc - 8 + 4 * b);
+        float4 v = lds4(pc - 8 + 4 * b);
         Y[4 * b] = v.x; Y[4 * b + 1] = v.y; Y[4 * b + 2] = v.z; Y[4 * b + 3] = v.w;
     }
 #pragma unroll
@@ -261,8 +344,8 @@ __device__ __forceinline__ void quad_derivs(const float *ring, size_t slot_float
     float2 gx[2] = {f2(0.f, 0.f), f2(0.f, 0.f)}, lx[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
 #pragma unroll
     for (int m = 0; m < kRadius; ++m) {
-        const float4 a = lds4(pc + rc + (m + 1) * kBoxY);
-        const float4 b = lds4(pc + rc - (m + 1) * kBoxY);
+        const float4 a = lds4(pc + (m + 1) * kBoxY);
+        const float4 b = lds4(pc - (m + 1) * kBoxY);
         const float2 a2[2] = {f2(a.x, a.y), f2(a.z, a.w)}, b2[2] = {f2(b.x, b.y), f2(b.z, b.w)};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -275,13 +358,12 @@ __device__ __forceinline__ void quad_derivs(const float *ring, size_t slot_float
     }
     Ux[0] = gx[0].x; Ux[1] = gx[0].y; Ux[2] = gx[1].x; Ux[3] = gx[1].y;
     if (SECOND) { Uxx[0] = lx[0].x; Uxx[1] = lx[0].y; Uxx[2] = lx[1].x; Uxx[3] = lx[1].y; }
-    // z taps: planes t+5 +- m
+    // z taps
     float2 gz[2] = {f2(0.f, 0.f), f2(0.f, 0.f)}, lz[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
 #pragma unroll
     for (int m = 0; m < kRadius; ++m) {
-        const int d = (m + 1) * (int)slot_floats;
-        const float4 a = lds4((sc + m + 1 < kRing ? pcr : pcr_lo) + d);
-        const float4 b = lds4((sc >= m + 1 ? pcr : pcr_hi) - d);
+        const float4 a = ztap(T, kRadius + m + 1);
+        const float4 b = ztap(T, kRadius - m - 1);
         const float2 a2[2] = {f2(a.x, a.y), f2(a.z, a.w)}, b2[2] = {f2(b.x, b.y), f2(b.z, b.w)};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -316,18 +398,16 @@ __device__ __forceinline__ void tap2(float2 a, float2 b, float2 u0, float2 c, fl
     l = __fadd2_rn(l, div2(__fmul2_rn(c2, lap_tap2(a, b, u0)), h2));
 }
 
-__device__ __forceinline__ void quad_derivs_ref(const float *ring, size_t slot_floats, int t,
-                                                int rc, const Coefs &k, float Ux[4], float Uy[4],
-                                                float Uz[4], float Uxx[4], float Uyy[4],
-                                                float Uzz[4], float u0[4])
+__device__ __forceinline__ void quad_derivs_ref(const Taps &T, const Coefs &k, float Ux[4],
+                                                float Uy[4], float Uz[4], float Uxx[4],
+                                                float Uyy[4], float Uzz[4], float u0[4])
 {
-    const int sc = (t + kRadius) % kRing;
-    const float *pc = ring + (size_t)sc * slot_floats;
+    const float *pc = T.pc;
     const float2 zero = make_float2(0.0f, 0.0f);
     float Y[20];
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
-        float4 v = lds4(pc + rc - 8 + 4 * b);
+        float4 v = lds4(pc - 8 + 4 * b);
         Y[4 * b] = v.x; Y[4 * b + 1] = v.y; Y[4 * b + 2] = v.z; Y[4 * b + 3] = v.w;
     }
     float2 c0[2];
@@ -348,8 +428,8 @@ __device__ __forceinline__ void quad_derivs_ref(const float *ring, size_t slot_f
     float2 gx[2] = {zero, zero}, lx[2] = {zero, zero};
 #pragma unroll
     for (int m = 0; m < kRadius; ++m) {
-        const float4 a = lds4(pc + rc + (m + 1) * kBoxY);
-        const float4 b = lds4(pc + rc - (m + 1) * kBoxY);
+        const float4 a = lds4(pc + (m + 1) * kBoxY);
+        const float4 b = lds4(pc - (m + 1) * kBoxY);
         const float2 a2[2] = {f2(a.x, a.y), f2(a.z, a.w)}, b2[2] = {f2(b.x, b.y), f2(b.z, b.w)};
 #pragma unroll
         for (int h = 0; h < 2; ++h)
@@ -360,10 +440,8 @@ __device__ __forceinline__ void quad_derivs_ref(const float *ring, size_t slot_f
     float2 gz[2] = {zero, zero}, lz[2] = {zero, zero};
 #pragma unroll
     for (int m = 0; m < kRadius; ++m) {
-        const float *pp = ring + (size_t)slot_add(sc, m + 1) * slot_floats;
-        const float *pm = ring + (size_t)slot_add(sc, -m - 1) * slot_floats;
-        const float4 a = lds4(pp + rc);
-        const float4 b = lds4(pm + rc);
+        const float4 a = ztap(T, kRadius + m + 1);
+        const float4 b = ztap(T, kRadius - m - 1);
         const float2 a2[2] = {f2(a.x, a.y), f2(a.z, a.w)}, b2[2] = {f2(b.x, b.y), f2(b.z, b.w)};
 #pragma unroll
         for (int h = 0; h < 2; ++h)
@@ -374,17 +452,15 @@ __device__ __forceinline__ void quad_derivs_ref(const float *ring, size_t slot_f
 }
 
 // First derivatives only, for the gradmax kernels.
-__device__ __forceinline__ void quad_grad_ref(const float *ring, size_t slot_floats, int t, int rc,
-                                              const Coefs &k, float Ux[4], float Uy[4],
-                                              float Uz[4])
+__device__ __forceinline__ void quad_grad_ref(const Taps &T, const Coefs &k, float Ux[4],
+                                              float Uy[4], float Uz[4])
 {
-    const int sc = (t + kRadius) % kRing;
-    const float *pc = ring + (size_t)sc * slot_floats;
+    const float *pc = T.pc;
     const float2 zero = make_float2(0.0f, 0.0f);
     float Y[20];
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
-        float4 v = lds4(pc + rc - 8 + 4 * b);
+        float4 v = lds4(pc - 8 + 4 * b);
         Y[4 * b] = v.x; Y[4 * b + 1] = v.y; Y[4 * b + 2] = v.z; Y[4 * b + 3] = v.w;
     }
 #pragma unroll
@@ -402,10 +478,10 @@ __device__ __forceinline__ void quad_grad_ref(const float *ring, size_t slot_flo
     float2 gx[2] = {zero, zero}, gz[2] = {zero, zero};
 #pragma unroll
     for (int m = 0; m < kRadius; ++m) {
-        const float4 a = lds4(pc + rc + (m + 1) * kBoxY);
-        const float4 b = lds4(pc + rc - (m + 1) * kBoxY);
-        const float4 za = lds4(ring + (size_t)slot_add(sc, m + 1) * slot_floats + rc);
-        const float4 zb = lds4(ring + (size_t)slot_add(sc, -m - 1) * slot_floats + rc);
+        const float4 a = lds4(pc + (m + 1) * kBoxY);
+        const float4 b = lds4(pc - (m + 1) * kBoxY);
+        const float4 za = ztap(T, kRadius + m + 1);
+        const float4 zb = ztap(T, kRadius - m - 1);
         const float2 a2[2] = {f2(a.x, a.y), f2(a.z, a.w)}, b2[2] = {f2(b.x, b.y), f2(b.z, b.w)};
         const float2 za2[2] = {f2(za.x, za.y), f2(za.z, za.w)},
                      zb2[2] = {f2(zb.x, zb.y), f2(zb.z, zb.w)};
@@ -420,57 +496,76 @@ __device__ __forceinline__ void quad_grad_ref(const float *ring, size_t slot_flo
 }
 
 // ---------------------------------------------------------------------------
-// Plane pipeline.  Staged plane i of a chunk holds z = zfirst + i, in slot
-// s = i % kRing.  full[s] completes when the TMA load of a plane into s has
-// landed (one arrival + transaction bytes); empty[s] completes when every
-// consumer warp has finished with the plane in s.  Plane i is last read by
-// iteration t = i (as the z-5 tap of plane z = zfirst + i + 5), so warps
-// release slot t % kRing after iteration t and thread 0 refills it with plane
-// t + kRing.  No CTA-wide barrier in the plane loop.
+// Plane pipeline.  The taps of a quad come from two rings.  The z taps need
+// eleven planes, but of each only the tile's own cells: 4 KB a plane at 32
+// rows.  The x and y taps need the 5-row, 8-column halo, but of the current
+// plane only: 8 KB.  Iteration t (z = z0 + t) therefore waits for one group
+// of loads: own-cell plane t + 10 (iteration 0: planes 0..10; plane i holds
+// z = z0 - 5 + i, in slot i % kRingZ) and halo plane t (slot t % kGroups),
+// both completing on full[t % kGroups].  Keeping eleven halo planes instead,
+// 8 KB each, left room for one load ahead, whose latency every iteration then
+// waited for; this form keeps kGroups - 1 = 2 groups ahead in less memory.
+//
+// A warp that has finished iteration t adds one to cnt[t % kGroups]; the last
+// one to do so refills what the iteration freed with group t + kGroups (its
+// own-cell plane goes to the slot of plane t, its halo plane to that of halo
+// plane t).  No CTA barrier, no producer warp, and the load starts as soon as
+// its slots are free.
 // ---------------------------------------------------------------------------
 struct Pipe {
-    float *ring;
-    uint64_t *full, *empty;
-    size_t slot_floats;
-    unsigned box_bytes;
-    int nplanes;     // planes to stage for this chunk
-    int zfirst;      // z of staged plane 0
-    int c0, c1;      // TMA coordinates of the box (y, x)
-    int ncw;         // consumer warps
+    float *zr, *cr;
+    uint64_t *full;
+    unsigned *cnt;
+    int *issued;     // groups issued so far
+    int zslot, cslot;
+    unsigned zbytes, cbytes;
+    int ngroups;     // iterations of this column
+    int y0, x0, z0;
+    int ncw;         // warps
     unsigned long long wait_ns;   // limit of every wait
-    int hold;        // test hook: plane never issued (-1: none)
+    int hold;        // test hook: own-cell plane never loaded (-1: none)
 };
 
-__device__ __forceinline__ void pipe_issue(const Pipe &P, const CUtensorMap *tm, int i)
+__device__ __forceinline__ void pipe_issue(const Pipe &P, const TileMaps *tm, int g)
 {
-    if (i == P.hold) return;   // test hook: the waits for this plane run out
-    int s = i % kRing;
-    mbar_arrive_expect_tx(&P.full[s], P.box_bytes);
-    tma_load_3d(P.ring + (size_t)s * P.slot_floats, tm, P.c0, P.c1, P.zfirst + i, &P.full[s]);
+    const int s = g % kGroups;
+    uint64_t *bar = &P.full[s];
+    *P.issued = g + 1;
+    mbar_arrive_expect_tx(bar, P.cbytes + P.zbytes * (g == 0 ? 2 * kRadius + 1 : 1));
+    for (int i = g == 0 ? 0 : g + 2 * kRadius; i <= g + 2 * kRadius; ++i)
+        if (i != P.hold)   // test hook: the wait for this group runs out
+            tma_load_3d(P.zr + (i % kRingZ) * P.zslot, &tm->z, P.y0, P.x0, P.z0 - kRadius + i, bar);
+    tma_load_3d(P.cr + s * P.cslot, &tm->c, P.y0 - kHaloY, P.x0 - kRadius, P.z0 + g, bar);
 }
 
-__device__ __forceinline__ bool pipe_wait(const Pipe &P, int i)
+__device__ __forceinline__ bool pipe_wait(const Pipe &P, int g)
 {
-    return mbar_wait_bounded(&P.full[i % kRing], (unsigned)((i / kRing) & 1), P.wait_ns);
+    return mbar_wait_bounded(&P.full[g % kGroups], (unsigned)((g / kGroups) & 1), P.wait_ns);
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Consumer warp: release the slot of plane i.
-__device__ __forceinline__ void pipe_release(const Pipe &P, int i)
+// The end of a warp's iteration t (see above).
+__device__ __forceinline__ void pipe_release(const Pipe &P, const TileMaps *tm, int t)
 {
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(&P.empty[i % kRing]);
+    if ((threadIdx.x & 31) == 0 && t + kGroups < P.ngroups) {
+        unsigned old;
+        unsigned *c = &P.cnt[t % kGroups];
+        asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
+                     : "=r"(old) : "r"(smem_u32(c)) : "memory");
+        if (old == (unsigned)P.ncw - 1) {
+            *c = 0;   // next used after the group issued here has landed
+            fence_proxy_async();
+            pipe_issue(P, tm, t + kGroups);
+        }
+    }
 }
 
+// Thread 0, before a CTA barrier: barriers and counters, then the first groups.
 __device__ void pipe_init(const Pipe &P)
 {
-    for (int s = 0; s < kRing; ++s) {
+    for (int s = 0; s < kGroups; ++s) {
         mbar_init(&P.full[s], 1);
-        mbar_init(&P.empty[s], P.ncw);
+        P.cnt[s] = 0;
     }
     fence_barrier_init();
     // a CTA that takes another tile reuses shared memory its threads read
@@ -478,237 +573,103 @@ __device__ void pipe_init(const Pipe &P)
     fence_proxy_async();
 }
 
-// Refills, done by thread 0 of the CTA (which also computes).  Before
-// iteration t it issues every plane whose slot has been released, and blocks
-// only for the plane iteration t needs (t + 10) -- i.e. only when some warp
-// is more than two planes behind.  That wait needs planes <= t + 7, all
-// issued earlier, so it cannot deadlock.  Returns false on a timed-out wait.
-__device__ bool pipe_refill(const Pipe &P, const CUtensorMap *tm, int t, int &next_issue)
+__device__ void pipe_start(const Pipe &P, const TileMaps *tm)
 {
-    while (next_issue < P.nplanes) {
-        const int i = next_issue;
-        uint64_t *e = &P.empty[i % kRing];
-        const unsigned par = (unsigned)(((i - kRing) / kRing) & 1);
-        if (i <= t + 2 * kRadius) {
-            if (!mbar_wait_bounded(e, par, P.wait_ns)) return false;
-        } else if (!mbar_try_wait(e, par)) {
-            break;
-        }
-        fence_proxy_async();
-        pipe_issue(P, tm, i);
-        ++next_issue;
+    for (int g = 0; g < kGroups && g < P.ngroups; ++g) pipe_issue(P, tm, g);
+}
+
+// The end of a column: true if no wait ran out (the same in every thread).
+// Otherwise the loads still in flight are waited for (bounded), so that none
+// lands in shared memory after the CTA has exited.
+__device__ bool pipe_finish(const Pipe &P, bool ok, unsigned *err)
+{
+    if (__syncthreads_and(ok)) return true;
+    if (threadIdx.x == 0) {
+        atomicOr(err, kErrWaitTimeout);
+        for (int g = max(0, *P.issued - kGroups); g < *P.issued; ++g) (void)pipe_wait(P, g);
     }
-    return true;
+    return false;
 }
 
-// After an aborted loop (thread 0): wait, bounded, for the loads still in
-// flight so that none lands in shared memory after the CTA has exited.
-__device__ void pipe_drain(const Pipe &P, int next_issue)
+// hooks: the launch's wait limit (0: 2 s) and the plane-withholding test hook
+// apply (grid launches; the hook to the first CTA only)
+__device__ __forceinline__ void pipe_setup(Pipe &P, unsigned char *smem, const SmemLayout &L,
+                                           const PlaneParams &p, bool hooks, int tile_x, int y0,
+                                           int x0, int z0, int nzc)
 {
-    for (int j = max(0, next_issue - kRing); j < next_issue; ++j) (void)pipe_wait(P, j);
-}
-
-__device__ __forceinline__ void pipe_setup(Pipe &P, unsigned char *smem, int tile_x, int pml,
-                                           int y0, int x0, int z0, int nzc)
-{
-    const SmemLayout L = smem_layout(tile_x, pml);
-    P.ring = reinterpret_cast<float *>(smem);
+    P.zr = reinterpret_cast<float *>(smem);
+    P.cr = reinterpret_cast<float *>(smem + L.c_off);
     P.full = reinterpret_cast<uint64_t *>(smem + L.bar_off);
-    P.empty = P.full + kRing;
-    P.slot_floats = L.slot_floats;
-    P.box_bytes = (unsigned)((tile_x + 2 * kRadius) * kBoxY * 4);
-    P.nplanes = nzc + 2 * kRadius;
-    P.zfirst = z0 - kRadius;
-    P.c0 = y0 - kHaloY;
-    P.c1 = x0 - kRadius;
-    P.ncw = blockDim.x >> 5;   // every warp of the CTA releases every slot
+    P.cnt = reinterpret_cast<unsigned *>(smem + L.cnt_off);
+    P.issued = reinterpret_cast<int *>(P.cnt + kGroups);
+    P.zslot = L.zslot;
+    P.cslot = L.cslot;
+    P.zbytes = (unsigned)(tile_x * kTileY * 4);
+    P.cbytes = (unsigned)((tile_x + 2 * kRadius) * kBoxY * 4);
+    P.ngroups = nzc;
+    P.y0 = y0;
+    P.x0 = x0;
+    P.z0 = z0;
+    P.ncw = blockDim.x >> 5;   // every warp of the CTA releases every iteration
     P.wait_ns = 2000000000ull;
     P.hold = -1;
-}
-
-// The wait limit of the launch (0: 2 s) and the plane-withholding test hook,
-// which applies to the first CTA of a grid launch only.
-__device__ __forceinline__ void pipe_hooks(Pipe &P, const PlaneParams &p)
-{
-    if (p.wait_ns) P.wait_ns = p.wait_ns;
-    if (p.hold_plane > 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) P.hold = p.hold_plane - 1;
-}
-
-__device__ __forceinline__ void pipe_setup(Pipe &P, unsigned char *smem, const PlaneParams &p,
-                                           int y0, int x0, int z0, int nzc)
-{
-    pipe_setup(P, smem, p.tile_x, p.pml, y0, x0, z0, nzc);
-    pipe_hooks(P, p);
+    if (hooks) {
+        if (p.wait_ns) P.wait_ns = p.wait_ns;
+        if (p.hold_plane > 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0)
+            P.hold = p.hold_plane - 1;
+    }
 }
 
 // Before a CTA reuses its barriers for another tile (thread 0, after a CTA
 // barrier; every load of the previous tile has been waited for).
 __device__ void pipe_inval(const Pipe &P)
 {
-    for (int s = 0; s < kRing; ++s) {
+    for (int s = 0; s < kGroups; ++s)
         asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&P.full[s])) : "memory");
-        asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&P.empty[s])) : "memory");
-    }
 }
 
-// ---------------------------------------------------------------------------
-// gradmax kernel.  With QUEUE the thread keeps its own column of the last 11
-// planes in registers (loop unrolled by 11 so the queue never moves), which
-// leaves 16 shared-memory vector loads per quad and plane instead of 25.
-// ---------------------------------------------------------------------------
-template <bool QUEUE, int AR>
-__global__ void __launch_bounds__(kThreads, 2)
-    qp3d_gradmax_kernel(const __grid_constant__ CUtensorMap tm_u, const PlaneParams p)
+// The ring positions of iteration t, kept incrementally.
+__device__ __forceinline__ Taps taps_start(const Pipe &P, int r, int q)
 {
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int tid = threadIdx.x;
-    const int q = tid & (kQuadsY - 1), r = tid / kQuadsY;
-    const int y0 = blockIdx.x * kTileY, x0 = kRadius + blockIdx.y * p.tile_x;
-    const int z0 = kRadius + blockIdx.z * p.chunk_z;
-    const int z1 = min(z0 + p.chunk_z, p.nz - kRadius);
-    if (z0 >= z1) return;
-    const int nzc = z1 - z0;
-    Pipe P;
-    pipe_setup(P, smem, p, y0, x0, z0, nzc);
-    int next_issue = 0;
-    if (tid == 0) {
-        pipe_init(P);
-        next_issue = min(kRing, P.nplanes);
-        for (int i = 0; i < next_issue; ++i) pipe_issue(P, &tm_u, i);
-    }
-    __syncthreads();
-    const int x = x0 + r, yq = y0 + 4 * q;
-    const bool row_ok = (r < p.tile_x) && (x < p.nx - kRadius);
-    bool cell_ok[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) cell_ok[j] = row_ok && (yq + j >= kRadius) && (yq + j < p.ny - kRadius);
-    const int rc = (r + kRadius) * kBoxY + kHaloY + 4 * q;
-    const Coefs &k = p.k;
+    Taps T;
+    T.pc = P.cr + (r + kRadius) * kBoxY + kHaloY + 4 * q;
+    T.za = P.zr + r * kTileY + 4 * q;
+    T.wrap = kRingZ;
+    T.zslot = P.zslot;
+    T.zlen = kRingZ * P.zslot;
+    return T;
+}
 
-    float mx = 0.0f;
-    bool ok = true;
-    if (QUEUE) {
-        float4 zq[2 * kRadius + 1];
-#pragma unroll
-        for (int i = 0; i < 2 * kRadius; ++i) {
-            ok = ok && pipe_wait(P, i);
-            zq[i] = lds4(P.ring + (size_t)(i % kRing) * P.slot_floats + rc);
-        }
-        for (int t0 = 0; t0 < nzc && ok; t0 += 2 * kRadius + 1) {
-#pragma unroll
-            for (int u = 0; u < 2 * kRadius + 1; ++u) {
-                const int t = t0 + u;
-                if (t >= nzc) break;
-                if (tid == 0 && t >= kPrefetch + 1 && !pipe_refill(P, &tm_u, t, next_issue)) {
-                    ok = false;
-                    break;
-                }
-                if (!pipe_wait(P, t + 2 * kRadius)) {
-                    ok = false;
-                    break;
-                }
-                zq[(u + 2 * kRadius) % 11] =
-                    lds4(P.ring + (size_t)((t + 2 * kRadius) % kRing) * P.slot_floats + rc);
-                const float *pc = P.ring + (size_t)((t + kRadius) % kRing) * P.slot_floats;
-                if (row_ok) {
-                    float Ux[4], Uy[4], Uz[4];
-                    float Y[20];
-#pragma unroll
-                    for (int b = 0; b < 5; ++b) {
-                        float4 v = lds4(pc + rc - 8 + 4 * b);
-                        Y[4 * b] = v.x; Y[4 * b + 1] = v.y; Y[4 * b + 2] = v.z; Y[4 * b + 3] = v.w;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        float g = 0.0f;
-#pragma unroll
-                        for (int m = 0; m < kRadius; ++m) {
-                            float d = __fsub_rn(Y[8 + j + m + 1], Y[8 + j - m - 1]);
-                            g = (m == 0) ? __fmul_rn(k.cy[0], d) : fmaf(k.cy[m], d, g);
-                        }
-                        Uy[j] = g;
-                    }
-#pragma unroll
-                    for (int m = 0; m < kRadius; ++m) {
-                        float4 a = lds4(pc + rc + (m + 1) * kBoxY);
-                        float4 b = lds4(pc + rc - (m + 1) * kBoxY);
-                        float4 za = zq[(u + kRadius + m + 1) % 11];
-                        float4 zb = zq[(u + kRadius - m - 1 + 11) % 11];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            float dx_ = __fsub_rn(f4(a, j), f4(b, j));
-                            float dz_ = __fsub_rn(f4(za, j), f4(zb, j));
-                            Ux[j] = (m == 0) ? __fmul_rn(k.cx[0], dx_) : fmaf(k.cx[m], dx_, Ux[j]);
-                            Uz[j] = (m == 0) ? __fmul_rn(k.cz[0], dz_) : fmaf(k.cz[m], dz_, Uz[j]);
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (cell_ok[j])
-                            mx = fmaxf(mx, fmaxf(fabsf(Ux[j]), fmaxf(fabsf(Uy[j]), fabsf(Uz[j]))));
-                }
-                pipe_release(P, t);
-            }
-        }
-    } else {
-        int waited = 0;
-        for (int t = 0; t < nzc; ++t) {
-            if (tid == 0 && t >= kPrefetch + 1 && !pipe_refill(P, &tm_u, t, next_issue)) {
-                ok = false;
-                break;
-            }
-            while (ok && waited <= t + 2 * kRadius) {
-                ok = pipe_wait(P, waited);
-                if (ok) ++waited;
-            }
-            if (!ok) break;
-            if (row_ok) {
-                float Ux[4], Uy[4], Uz[4], Uxx[4], Uyy[4], Uzz[4], u0[4];
-                if (AR == kArithRef)
-                    quad_grad_ref(P.ring, P.slot_floats, t, rc, k, Ux, Uy, Uz);
-                else
-                    quad_derivs<false>(P.ring, P.slot_floats, t, rc, k, Ux, Uy, Uz, Uxx, Uyy,
-                                       Uzz, u0);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (cell_ok[j])
-                        mx = fmaxf(mx, fmaxf(fabsf(Ux[j]), fmaxf(fabsf(Uy[j]), fabsf(Uz[j]))));
-            }
-            pipe_release(P, t);
-        }
+__device__ __forceinline__ void taps_next(Taps &T, const Pipe &P, int t)   // from t to t + 1
+{
+    T.za += T.zslot;
+    if (--T.wrap == 0) {
+        T.za -= T.zlen;
+        T.wrap = kRingZ;
     }
-    if (!ok) {
-        atomicOr(p.err, kErrWaitTimeout);
-        if (tid == 0) pipe_drain(P, next_issue);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31) == 0 && mx > 0.0f)
-        atomicMax(reinterpret_cast<unsigned *>(p.gmax + p.step), __float_as_uint(mx));
+    T.pc += t % kGroups == kGroups - 1 ? -(kGroups - 1) * P.cslot : P.cslot;
 }
 
 // ---------------------------------------------------------------------------
-// gradmax of one tile column [z0, z1) for the batched launches: the
-// arithmetic of qp3d_gradmax_kernel<false>.  With REUSE the CTA's barriers
-// are invalidated at the end so that it can take another tile; the return
-// value (false: a wait timed out) is then the same in every thread.
+// max|grad u| over one tile column [z0, z1), a thread's own maximum in mx.
+// The grid kernels run one column per CTA; the batched kernel runs many
+// (REUSE: barriers invalidated at the end).  Returns false (in every thread)
+// when a wait timed out.
 // ---------------------------------------------------------------------------
-template <bool REUSE, int AR = kArithFast>
-__device__ __forceinline__ bool gradmax_tile(const CUtensorMap *tm, const PlaneParams &p,
+template <bool REUSE, int AR>
+__device__ __forceinline__ bool gradmax_tile(const TileMaps *tm, const PlaneParams &p,
                                              const Coefs &k, int tile_x, int y0, int x0, int z0,
-                                             int z1, unsigned char *smem)
+                                             int z1, unsigned char *smem, float &mx)
 {
     const int tid = threadIdx.x;
     const int q = tid & (kQuadsY - 1), r = tid / kQuadsY;
     const int nzc = z1 - z0;
+    const SmemLayout L = smem_layout(tile_x, 0, 0, 0);
     Pipe P;
-    pipe_setup(P, smem, tile_x, p.pml, y0, x0, z0, nzc);
-    if (!REUSE) pipe_hooks(P, p);
-    int next_issue = 0;
+    pipe_setup(P, smem, L, p, !REUSE, tile_x, y0, x0, z0, nzc);
     if (tid == 0) {
         pipe_init(P);
-        next_issue = min(kRing, P.nplanes);
-        for (int i = 0; i < next_issue; ++i) pipe_issue(P, tm, i);
+        pipe_start(P, tm);
     }
     __syncthreads();
     const int x = x0 + r, yq = y0 + 4 * q;
@@ -716,217 +677,124 @@ __device__ __forceinline__ bool gradmax_tile(const CUtensorMap *tm, const PlaneP
     bool cell_ok[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) cell_ok[j] = row_ok && (yq + j >= kRadius) && (yq + j < p.ny - kRadius);
-    const int rc = (r + kRadius) * kBoxY + kHaloY + 4 * q;
-    float mx = 0.0f;
+    Taps T = taps_start(P, r, q);
+    mx = 0.0f;
     bool ok = true;
-    int waited = 0;
-    for (int t = 0; t < nzc; ++t) {
-        if (tid == 0 && t >= kPrefetch + 1 && !pipe_refill(P, tm, t, next_issue)) ok = false;
-        while (ok && waited <= t + 2 * kRadius) {
-            ok = pipe_wait(P, waited);
-            if (ok) ++waited;
-        }
-        ok = __all_sync(0xffffffffu, ok);
+    for (int t = 0; t < nzc; taps_next(T, P, t), ++t) {
+        ok = __all_sync(0xffffffffu, pipe_wait(P, t));
         if (!ok) break;
         if (row_ok) {
             float Ux[4], Uy[4], Uz[4], Uxx[4], Uyy[4], Uzz[4], u0[4];
-            if (AR == kArithRef)
-                quad_grad_ref(P.ring, P.slot_floats, t, rc, k, Ux, Uy, Uz);
-            else
-                quad_derivs<false>(P.ring, P.slot_floats, t, rc, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
+            if (AR == kArithRef) quad_grad_ref(T, k, Ux, Uy, Uz);
+            else quad_derivs<false>(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 if (cell_ok[j])
                     mx = fmaxf(mx, fmaxf(fabsf(Ux[j]), fmaxf(fabsf(Uy[j]), fabsf(Uz[j]))));
         }
-        pipe_release(P, t);
+        pipe_release(P, tm, t);
     }
-    if (!ok) {
-        atomicOr(p.err, kErrWaitTimeout);
-        if (tid == 0) pipe_drain(P, next_issue);
-    }
+    ok = pipe_finish(P, ok, p.err);
+    if (REUSE && tid == 0 && ok) pipe_inval(P);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31) == 0 && mx > 0.0f)
-        atomicMax(reinterpret_cast<unsigned *>(p.gmax + p.step), __float_as_uint(mx));
-    if (REUSE) {
-        ok = __syncthreads_and(ok) != 0;
-        if (tid == 0 && ok) pipe_inval(P);
-    }
     return ok;
 }
 
-// ---------------------------------------------------------------------------
-// gradmax with per-CTA partial results: the same staging and arithmetic as
-// qp3d_gradmax_kernel<false>, but each CTA writes its own maximum to
-// partial[linear CTA index] (every CTA writes its slot, also when it has no
-// cell), for callers that supply the partial array themselves.
-// ---------------------------------------------------------------------------
+__device__ __forceinline__ void gradmax_publish(const PlaneParams &p, float mx)
+{
+    if ((threadIdx.x & 31) == 0 && mx > 0.0f)
+        atomicMax(reinterpret_cast<unsigned *>(p.gmax + p.step), __float_as_uint(mx));
+}
+
 template <int AR>
 __global__ void __launch_bounds__(kThreads, 2)
-    qp3d_gradmax_partial_kernel(const __grid_constant__ CUtensorMap tm_u, const PlaneParams p,
-                                float *partial)
+    qp3d_gradmax_kernel(const __grid_constant__ TileMaps tm, const PlaneParams p)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ float wmax[kThreads / 32];
-    const int tid = threadIdx.x;
-    const unsigned cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const int q = tid & (kQuadsY - 1), r = tid / kQuadsY;
-    const int y0 = blockIdx.x * kTileY, x0 = kRadius + blockIdx.y * p.tile_x;
+    pdl_trigger();
+    pdl_wait();
     const int z0 = kRadius + blockIdx.z * p.chunk_z;
     const int z1 = min(z0 + p.chunk_z, p.nz - kRadius);
-    if (z0 >= z1) {
-        if (tid == 0) partial[cta] = 0.0f;
-        return;
-    }
-    const int nzc = z1 - z0;
-    Pipe P;
-    pipe_setup(P, smem, p, y0, x0, z0, nzc);
-    int next_issue = 0;
-    if (tid == 0) {
-        pipe_init(P);
-        next_issue = min(kRing, P.nplanes);
-        for (int i = 0; i < next_issue; ++i) pipe_issue(P, &tm_u, i);
-    }
-    __syncthreads();
-    const int x = x0 + r, yq = y0 + 4 * q;
-    const bool row_ok = (r < p.tile_x) && (x < p.nx - kRadius);
-    bool cell_ok[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) cell_ok[j] = row_ok && (yq + j >= kRadius) && (yq + j < p.ny - kRadius);
-    const int rc = (r + kRadius) * kBoxY + kHaloY + 4 * q;
-    float mx = 0.0f;
-    bool ok = true;
-    int waited = 0;
-    for (int t = 0; t < nzc; ++t) {
-        if (tid == 0 && t >= kPrefetch + 1 && !pipe_refill(P, &tm_u, t, next_issue)) ok = false;
-        while (ok && waited <= t + 2 * kRadius) {
-            ok = pipe_wait(P, waited);
-            if (ok) ++waited;
-        }
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        if (row_ok) {
-            float Ux[4], Uy[4], Uz[4], Uxx[4], Uyy[4], Uzz[4], u0[4];
-            if (AR == kArithRef)
-                quad_grad_ref(P.ring, P.slot_floats, t, rc, p.k, Ux, Uy, Uz);
-            else
-                quad_derivs<false>(P.ring, P.slot_floats, t, rc, p.k, Ux, Uy, Uz, Uxx, Uyy, Uzz,
-                                   u0);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (cell_ok[j])
-                    mx = fmaxf(mx, fmaxf(fabsf(Ux[j]), fmaxf(fabsf(Uy[j]), fabsf(Uz[j]))));
-        }
-        pipe_release(P, t);
-    }
-    if (!ok) {
-        atomicOr(p.err, kErrWaitTimeout);
-        if (tid == 0) pipe_drain(P, next_issue);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31) == 0) wmax[tid / 32] = mx;
-    __syncthreads();
-    if (tid == 0) {
-        float m = 0.0f;
-        for (int w = 0; w < (int)blockDim.x / 32; ++w) m = fmaxf(m, wmax[w]);
-        partial[cta] = m;
-    }
-}
-
-// One block: out[0] = max(partial[0..n)), or NaN when *err is set.
-__global__ void qp3d_reduce_max_kernel(const float *partial, unsigned n, const unsigned *err,
-                                       float *out)
-{
-    __shared__ float wmax[32];
-    float m = 0.0f;
-    for (unsigned i = threadIdx.x; i < n; i += blockDim.x) m = fmaxf(m, partial[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x / 32] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float r = 0.0f;
-        for (int w = 0; w < (int)blockDim.x / 32; ++w) r = fmaxf(r, wmax[w]);
-        out[0] = (err && *err) ? __int_as_float(0x7fc00000) : r;
-    }
+    if (z0 >= z1) return;
+    float mx;
+    gradmax_tile<false, AR>(&tm, p, p.k, p.tile_x, blockIdx.x * kTileY,
+                            kRadius + blockIdx.y * p.tile_x, z0, z1, smem, mx);
+    gradmax_publish(p, mx);
 }
 
 // ---------------------------------------------------------------------------
-// PML update of one cell (GPU_kernel.cu:566-637 restated with per-layer
-// coefficients a1 = (d*dt+1)^2-3, a2 = 2*d*dt-1, a3 = 1-dt*d).  Face codes
-// L=0 R=1 F=2 Bk=3 T=4 Bo=5; the odd faces take the minus sign on the
-// dd*u_n term.  Written with selects only.
+// gradmax for a caller that supplies no buffer: the maximum, a count of the
+// CTAs that are done and the error word live in one small scratch that every
+// launch finds zero.  The last CTA delivers the result (NaN when a wait ran
+// out) and the error flags, and leaves the scratch zero again.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float pml_cell(int f, float4 lc, float KS, float e2, float Ux,
-                                          float Uy, float Uz, float Uxx, float Uyy, float Uzz,
-                                          float dt, float w11, float w12, float w21, float w31,
-                                          float w32, float p1, float p2, float &nw13,
-                                          float &nw21, float &nw33, float &np3)
+__global__ void __launch_bounds__(kThreads, 2)
+    qp3d_gradmax_single_kernel(const __grid_constant__ TileMaps tm, const PlaneParams p,
+                               GradmaxScratch *sc, float *out, unsigned *host_flags)
 {
-    const bool isx = f < 2, isz = f >= 4;
-    const float e2KS = __fmul_rn(e2, KS);
-    const float A = isz ? KS : e2KS;
-    const float Unn = isx ? Uxx : (isz ? Uzz : Uyy);
-    const float Un = isx ? Ux : (isz ? Uz : Uy);
-    const float Bt = isz ? e2KS : KS;
-    const float Tt = isz ? __fadd_rn(Uxx, Uyy) : fmaf(e2, isx ? Uyy : Uxx, Uzz);
-    const float a1 = lc.x, a2 = lc.y, a3 = lc.z, dd = lc.w;
-    nw13 = fmaf(A, Unn, fmaf(-a1, w12, __fmul_rn(a2, w11)));
-    float Ad = __fmul_rn(A, dd);
-    Ad = (f & 1) ? -Ad : Ad;
-    np3 = fmaf(Ad, Un, fmaf(-a1, p2, __fmul_rn(a2, p1)));
-    nw21 = fmaf(dt, np3, __fmul_rn(a3, w21));
-    nw33 = fmaf(Bt, Tt, fmaf(2.0f, w32, -w31));
-    return __fadd_rn(__fadd_rn(nw13, nw21), nw33);
-}
-
-// The same update with two scalar operators, KS and KS1 (S = 1): the terms
-// that do not depend on S are shared, and each result equals pml_cell's with
-// that operator bit for bit.  The second set of outputs goes to a1x.
-__device__ __forceinline__ float pml_cell2(int f, float4 lc, float KS, float KS1, float e2,
-                                           float Ux, float Uy, float Uz, float Uxx, float Uyy,
-                                           float Uzz, float dt, float w11, float w12, float w21,
-                                           float w31, float w32, float p1, float p2,
-                                           float &nw13, float &nw21, float &nw33, float &np3,
-                                           float &v1, float4 &a1x)
-{
-    const bool isx = f < 2, isz = f >= 4;
-    const float Unn = isx ? Uxx : (isz ? Uzz : Uyy);
-    const float Un = isx ? Ux : (isz ? Uz : Uy);
-    const float Tt = isz ? __fadd_rn(Uxx, Uyy) : fmaf(e2, isx ? Uyy : Uxx, Uzz);
-    const float a1 = lc.x, a2 = lc.y, a3 = lc.z, dd = lc.w;
-    const float X1 = fmaf(-a1, w12, __fmul_rn(a2, w11));
-    const float X2 = fmaf(-a1, p2, __fmul_rn(a2, p1));
-    const float X3 = fmaf(2.0f, w32, -w31);
-    const float W = __fmul_rn(a3, w21);
-    float out[2];
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        const float ks = s ? KS1 : KS;
-        const float e2KS = __fmul_rn(e2, ks);
-        const float A = isz ? ks : e2KS, Bt = isz ? e2KS : ks;
-        float Ad = __fmul_rn(A, dd);
-        Ad = (f & 1) ? -Ad : Ad;
-        const float n13 = fmaf(A, Unn, X1), n3 = fmaf(Ad, Un, X2);
-        const float n21 = fmaf(dt, n3, W), n33 = fmaf(Bt, Tt, X3);
-        out[s] = __fadd_rn(__fadd_rn(n13, n21), n33);
-        if (s) a1x = make_float4(n13, n21, n33, n3);
-        else nw13 = n13, nw21 = n21, nw33 = n33, np3 = n3;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int z0 = kRadius + blockIdx.z * p.chunk_z;
+    const int z1 = min(z0 + p.chunk_z, p.nz - kRadius);
+    if (z0 < z1) {
+        float mx;
+        gradmax_tile<false, kArithFast>(&tm, p, p.k, p.tile_x, blockIdx.x * kTileY,
+                                        kRadius + blockIdx.y * p.tile_x, z0, z1, smem, mx);
+        if ((threadIdx.x & 31) == 0 && mx > 0.0f) atomicMax(&sc->max_bits, __float_as_uint(mx));
     }
-    v1 = out[1];
-    return out[0];
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&sc->done, 1u) != gridDim.x * gridDim.y * gridDim.z - 1) return;
+    __threadfence();
+    const unsigned flags = atomicExch(&sc->err, 0u), bits = atomicExch(&sc->max_bits, 0u);
+    atomicExch(&sc->done, 0u);
+    out[0] = flags ? __int_as_float(0x7fc00000) : __uint_as_float(bits);
+    *host_flags = flags;
 }
 
-__device__ __forceinline__ float4 ldg4(const float *p)
+// ---------------------------------------------------------------------------
+// PML update of a quad in the fast arithmetic (GPU_kernel.cu:566-637 restated
+// with per-layer coefficients a1 = (d*dt+1)^2-3, a2 = 2*d*dt-1, a3 = 1-dt*d),
+// for faces normal to axis AX (0 x, 1 y, 2 z), two cells at a time with the
+// packed FP32x2 instructions.  na1 = -a1, and dd carries the sign of the odd
+// faces (R, Bk, Bo), so that every product and sum rounds as the scalar
+// expression does.  One body per axis: choosing the normal and tangential
+// derivatives of every cell by selects took about a third of the update's
+// instructions.
+// ---------------------------------------------------------------------------
+struct PmlOwn {   // what a PML quad reads of its split-field state
+    float4 w11, w12, w31, w32, p1, p2, w21;
+};
+struct PmlNew {
+    float2 w13[2], w21[2], w33[2], p3[2];
+};
+
+__device__ __forceinline__ float2 half2of(const float4 &v, int h)
 {
-    return __ldg(reinterpret_cast<const float4 *>(p));
+    return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
 }
 
-__device__ __forceinline__ float4 ld4(const float *p)
+template <int AX>
+__device__ __forceinline__ float2 pml_pair(float2 na1, float2 a2, float2 a3, float2 dd, float2 KS,
+                                           float2 e1, float2 Un, float2 Uxx, float2 Uyy,
+                                           float2 Uzz, float2 dt, const PmlOwn &o, int h,
+                                           PmlNew &n)
 {
-    return *reinterpret_cast<const float4 *>(p);
+    const float2 e2KS = __fmul2_rn(e1, KS);
+    const float2 A = AX == 2 ? KS : e2KS, Bt = AX == 2 ? e2KS : KS;
+    const float2 Unn = AX == 0 ? Uxx : AX == 1 ? Uyy : Uzz;
+    const float2 Tt = AX == 2 ? __fadd2_rn(Uxx, Uyy) : __ffma2_rn(e1, AX == 0 ? Uyy : Uxx, Uzz);
+    n.w13[h] = __ffma2_rn(A, Unn, __ffma2_rn(na1, half2of(o.w12, h),
+                                             __fmul2_rn(a2, half2of(o.w11, h))));
+    n.p3[h] = __ffma2_rn(__fmul2_rn(A, dd), Un, __ffma2_rn(na1, half2of(o.p2, h),
+                                                           __fmul2_rn(a2, half2of(o.p1, h))));
+    n.w21[h] = __ffma2_rn(dt, n.p3[h], __fmul2_rn(a3, half2of(o.w21, h)));
+    const float2 w31 = half2of(o.w31, h);
+    const float2 X3 = __ffma2_rn(make_float2(2.0f, 2.0f), half2of(o.w32, h),
+                                 make_float2(-w31.x, -w31.y));
+    n.w33[h] = __ffma2_rn(Bt, Tt, X3);
+    return __fadd2_rn(__fadd2_rn(n.w13[h], n.w21[h]), n.w33[h]);
 }
 
 // Face code and layer index of a cell from its x/y/z face parts (-1: none),
@@ -949,33 +817,35 @@ __device__ __forceinline__ void cell_face(int fx, int lix, int fy, int liy, int 
 //     in (T2(M_lo), T2(M_hi)] has an uncertain decision: the kernel computes
 //     it as "above", marks it in the deferred-cell bitmask with its m2 and
 //     S = 1 value, and reduces the true max of the step into gmax[step] on
-//     the way.  The resolution, compaction and fix-up kernels then give the
+//     the way.  The resolution kernel then gives the
 //     S = 1 result to the marked cells that turn out to be below the
 //     threshold, or ask for the exact re-run when the max fell outside the
 //     window.  The step never overwrites its inputs, so both are possible.
 //     Both modes write bit-identical results.
 // ---------------------------------------------------------------------------
-__device__ void spec_window(const PlaneParams &p, float &lo, float &hi, float &pred)
+// w = (M_lo, M_hi, M_pred) of step k, from the maxima of the two steps before
+// and the recent prediction errors.
+__device__ void spec_window(const PlaneParams &p, int k, const float *spec_err, float w[3])
 {
-    const int k = p.step;
     const float m1 = k >= 1 ? p.gmax[k - 1] : 0.0f;
     const float m0 = k >= 2 ? p.gmax[k - 2] : 0.0f;
     float r = (m0 > 0.0f) ? __fdiv_rn(m1, m0) : 1.0f;
     r = fminf(fmaxf(r, 0.5f), 2.0f);
     // half the last trend: late in a shot the max moves by a few tenths of a
     // percent per step with changing sign, which a full extrapolation doubles
-    pred = __fmul_rn(m1, fmaf(0.5f, __fsub_rn(r, 1.0f), 1.0f));
+    const float pred = __fmul_rn(m1, fmaf(0.5f, __fsub_rn(r, 1.0f), 1.0f));
     // cover both "the max keeps its trend" and "the max stays where it was",
     // widened by 1.5x the largest of the recent prediction errors
     float e = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kSpecHist; ++i) e = fmaxf(e, p.spec_err[i]);
+    for (int i = 0; i < kSpecHist; ++i) e = fmaxf(e, spec_err[i]);
     const float d = fminf(0.25f, fmaxf(p.delta_min, __fmul_rn(1.5f, e)));
-    lo = __fmul_rn(fminf(pred, m1), __fsub_rn(1.0f, d));
-    hi = __fmul_rn(fmaxf(pred, m1), __fadd_rn(1.0f, d));
+    w[0] = __fmul_rn(fminf(pred, m1), __fsub_rn(1.0f, d));
+    w[1] = __fmul_rn(fmaxf(pred, m1), __fadd_rn(1.0f, d));
+    w[2] = pred;
     if (p.spec_bias != 0.0f) {   // test hook: a window that misses on purpose
-        lo = __fmul_rn(lo, __fadd_rn(1.0f, p.spec_bias));
-        hi = __fmul_rn(hi, __fadd_rn(1.0f, p.spec_bias));
+        w[0] = __fmul_rn(w[0], __fadd_rn(1.0f, p.spec_bias));
+        w[1] = __fmul_rn(w[1], __fadd_rn(1.0f, p.spec_bias));
     }
 }
 
@@ -1053,140 +923,383 @@ __device__ __forceinline__ float4 fast_layer(float4 t)
     return make_float4(t.x, __fmaf_rn(2.0f, t.z, -1.0f), __fsub_rn(1.0f, t.z), t.w);
 }
 
+// The same with -a1 in place of a1, as the packed PML update takes it.
+__device__ __forceinline__ float4 step_layer(float4 t)
+{
+    const float4 l = fast_layer(t);
+    return make_float4(-l.x, l.y, l.z, l.w);
+}
+
+// The split-field update of one PML cell of face code f, layer li; v: its
+// pml_inputs, ks as in step_tile.
+template <int AR>
+__device__ __forceinline__ xr::PmlOut pml_cell(int f, float4 layer, float ks, float e1, float vp,
+                                               float4 v, float dt, float w11, float w12, float w21,
+                                               float w31, float w32, float p1, float p2)
+{
+    const bool isz = f >= 4;
+    if (AR == kArithRef) {
+        xr::PmlLayer Lr;
+        Lr.a1h = layer.x; Lr.a1l = layer.y;
+        Lr.a2 = __fmaf_rn(2.0f, layer.z, -1.0f);
+        Lr.a3 = __fsub_rn(1.0f, layer.z);
+        Lr.dd = layer.w;
+        return xr::pml_update(isz, (f & 1) != 0, ks, e1, __fmul_rn(vp, dt), v.x, v.y, v.z, dt, Lr,
+                              w11, w12, w21, w31, w32, p1, p2);
+    }
+    const float4 lc = step_layer(layer);
+    const float e2KS = __fmul_rn(e1, ks);
+    const float A = isz ? ks : e2KS, Bt = isz ? e2KS : ks;
+    xr::PmlOut o;
+    o.w13 = fmaf(A, v.x, fmaf(lc.x, w12, __fmul_rn(lc.y, w11)));
+    o.p3 = fmaf(__fmul_rn(A, (f & 1) ? -lc.w : lc.w), v.y, fmaf(lc.x, p2, __fmul_rn(lc.y, p1)));
+    o.w21 = fmaf(dt, o.p3, __fmul_rn(lc.z, w21));
+    o.w33 = fmaf(Bt, v.z, fmaf(2.0f, w32, -w31));
+    o.u3 = __fadd_rn(__fadd_rn(o.w13, o.w21), o.w33);
+    return o;
+}
+
+// Where the cells of one column that wait for the exact max are listed
+// ("deferred" cells): a segment of the shot's list, in no particular order,
+// with its length.
+struct DeferSeg {
+    size_t base;        // first entry of the segment
+    unsigned cap;       // its entries; more deferred cells make the step re-run
+    unsigned *count;
+};
+
+// The interior update, S of the cell as kS above: the reference's roundings, or
+// two fused multiply-adds.
+template <int AR>
+__device__ __forceinline__ float interior_cell(float u0, float u1, float Uxx, float Uyy, float Uzz,
+                                               float e1, float ks, float vp, float dt2)
+{
+    if (AR == kArithRef) return xr::interior_update(u0, u1, Uxx, Uyy, Uzz, e1, ks, vp, dt2);
+    const float Lp = fmaf(e1, __fadd_rn(Uxx, Uyy), Uzz);
+    return fmaf(ks, Lp, fmaf(2.0f, u0, -u1));
+}
+
+// Places in the segment for the deferred cells of a warp's quads (nib: a bit
+// per cell): the first place of this thread's.  *cnt: the segment's length so
+// far, in shared memory.
+__device__ __forceinline__ unsigned defer_places(unsigned *cnt, unsigned nib)
+{
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned c = __popc(nib);
+    unsigned incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (unsigned)o) incl += v;
+    }
+    unsigned first = 0;
+    if (lane == 31) first = atomicAdd(cnt, incl);
+    return __shfl_sync(0xffffffffu, first, 31) + incl - c;
+}
+
+// The derivatives the PML update of a face code f takes: along the normal
+// (second, first) and the tangential combination.
+template <int AR>
+__device__ __forceinline__ float4 pml_inputs(int f, float e1, float Ux, float Uy, float Uz,
+                                             float Uxx, float Uyy, float Uzz)
+{
+    const bool isx = f < 2, isz = f >= 4;
+    const float Ut = isx ? Uyy : Uxx;
+    float Tt;
+    if (isz) Tt = __fadd_rn(Uxx, Uyy);
+    else Tt = AR == kArithRef ? __fadd_rn(Uzz, __fmul_rn(e1, Ut)) : fmaf(e1, Ut, Uzz);
+    return make_float4(isx ? Uxx : (isz ? Uzz : Uyy), isx ? Ux : (isz ? Uz : Uy), Tt, 0.0f);
+}
+
+// Largest and smallest of four values, NaN if any is: a comparison with it is
+// then false, as the comparison with that value is.
+__device__ __forceinline__ float max4(const float v[4])
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(v[0]), "f"(v[1]), "f"(v[2]));
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(r), "f"(v[3]));
+    return r;
+}
+__device__ __forceinline__ float min4(const float v[4])
+{
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(v[0]), "f"(v[1]), "f"(v[2]));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(r), "f"(v[3]));
+    return r;
+}
+
+// The PML update of a quad, its interior results in out: the cells of pmlb get
+// the split-field ones, and n every new state (0, and the old w21, for cells
+// that are not of the shell).
+__device__ __forceinline__ void pml_quad_ref(
+    const PlaneParams &p, const float4 *tab, const float kS[4], const float e1[4], float4 Vv,
+    const float Ux[4], const float Uy[4], const float Uz[4], const float Uxx[4],
+    const float Uyy[4], const float Uzz[4], const PmlOwn &o, unsigned pmlb, int fx, int lix,
+    int yq, int fz, int liz, float out[4], PmlNew &n)
+{
+    const int pml = p.pml, ny = p.ny;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float *w13 = j & 1 ? &n.w13[j >> 1].y : &n.w13[j >> 1].x;
+        float *w21 = j & 1 ? &n.w21[j >> 1].y : &n.w21[j >> 1].x;
+        float *w33 = j & 1 ? &n.w33[j >> 1].y : &n.w33[j >> 1].x;
+        float *p3 = j & 1 ? &n.p3[j >> 1].y : &n.p3[j >> 1].x;
+        *w13 = *w33 = *p3 = 0.0f;
+        *w21 = f4(o.w21, j);
+        if (!((pmlb >> j) & 1u)) continue;
+        int f, li;
+        const int y = yq + j;
+        const int fy = y < pml ? 2 : (y >= ny - pml ? 3 : -1);
+        cell_face(fx, lix, fy, y < pml ? pml - y : y - ny + pml, fz, liz, f, li);
+        const xr::PmlOut v = pml_cell<kArithRef>(
+            f, tab[(f >> 1) * pml + li], kS[j], e1[j], f4(Vv, j),
+            pml_inputs<kArithRef>(f, e1[j], Ux[j], Uy[j], Uz[j], Uxx[j], Uyy[j], Uzz[j]), p.dt,
+            f4(o.w11, j), f4(o.w12, j), f4(o.w21, j), f4(o.w31, j), f4(o.w32, j), f4(o.p1, j),
+            f4(o.p2, j));
+        out[j] = v.u3;
+        *w13 = v.w13; *w21 = v.w21; *w33 = v.w33; *p3 = v.p3;
+    }
+}
+
+__device__ __forceinline__ void pml_quad_fast(
+    const PlaneParams &p, const float4 *tab, const float *ytab, const float kS[4],
+    const float e1[4], const float Ux[4], const float Uy[4], const float Uz[4],
+    const float Uxx[4], const float Uyy[4], const float Uzz[4], const PmlOwn &o, unsigned pmlb,
+    unsigned fyb, int fx, int lix, int fz, int liz, float out[4], PmlNew &n)
+{
+    const float2 dt = make_float2(p.dt, p.dt);
+    float2 v[2];
+#define QP3D_PML_PAIRS(AX, NA1, A2, A3, DD, UN)                                                   _Pragma("unroll") for (int h = 0; h < 2; ++h) {                                                   const int j0 = 2 * h, j1 = 2 * h + 1;                                                         v[h] = pml_pair<AX>(NA1, A2, A3, DD, f2(kS[j0], kS[j1]), f2(e1[j0], e1[j1]),                                      f2(UN[j0], UN[j1]), f2(Uxx[j0], Uxx[j1]), f2(Uyy[j0], Uyy[j1]),                               f2(Uzz[j0], Uzz[j1]), dt, o, h, n);                                   }
+    if (fx >= 0) {
+        const float4 lc = tab[lix];
+        const float dd = fx ? -lc.w : lc.w;
+        QP3D_PML_PAIRS(0, f2(lc.x, lc.x), f2(lc.y, lc.y), f2(lc.z, lc.z), f2(dd, dd), Ux)
+    } else if (fyb) {
+        const float4 c1 = lds4(ytab), c2 = lds4(ytab + kTileY), c3 = lds4(ytab + 2 * kTileY),
+                     c4 = lds4(ytab + 3 * kTileY);
+        QP3D_PML_PAIRS(1, half2of(c1, h), half2of(c2, h), half2of(c3, h), half2of(c4, h), Uy)
+        if (fyb != 15u && fz >= 0) {   // the quad's other cells are of the z face
+            const PmlNew y = n;
+            const float2 vy[2] = {v[0], v[1]};
+            const float4 lc = tab[2 * p.pml + liz];
+            const float dd = fz & 1 ? -lc.w : lc.w;
+            QP3D_PML_PAIRS(2, f2(lc.x, lc.x), f2(lc.y, lc.y), f2(lc.z, lc.z), f2(dd, dd), Uz)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (fyb >> (2 * h) & 1u) {
+                    v[h].x = vy[h].x;
+                    n.w13[h].x = y.w13[h].x; n.w21[h].x = y.w21[h].x;
+                    n.w33[h].x = y.w33[h].x; n.p3[h].x = y.p3[h].x;
+                }
+                if (fyb >> (2 * h + 1) & 1u) {
+                    v[h].y = vy[h].y;
+                    n.w13[h].y = y.w13[h].y; n.w21[h].y = y.w21[h].y;
+                    n.w33[h].y = y.w33[h].y; n.p3[h].y = y.p3[h].y;
+                }
+            }
+        }
+    } else {
+        const float4 lc = tab[2 * p.pml + liz];
+        const float dd = fz & 1 ? -lc.w : lc.w;
+        QP3D_PML_PAIRS(2, f2(lc.x, lc.x), f2(lc.y, lc.y), f2(lc.z, lc.z), f2(dd, dd), Uz)
+    }
+#undef QP3D_PML_PAIRS
+    if (pmlb == 15u) {
+        out[0] = v[0].x; out[1] = v[0].y; out[2] = v[1].x; out[3] = v[1].y;
+        return;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {   // cells of the interior or of the never-updated band
+        if (pmlb >> (2 * h) & 1u) {
+            out[2 * h] = v[h].x;
+        } else {
+            n.w13[h].x = n.w33[h].x = n.p3[h].x = 0.0f;
+            n.w21[h].x = half2of(o.w21, h).x;
+        }
+        if (pmlb >> (2 * h + 1) & 1u) {
+            out[2 * h + 1] = v[h].y;
+        } else {
+            n.w13[h].y = n.w33[h].y = n.p3[h].y = 0.0f;
+            n.w21[h].y = half2of(o.w21, h).y;
+        }
+    }
+}
+
 // One tile column [z0, z1) of the step.  The grid kernel below runs one per
 // CTA; the batched kernel runs many per CTA (REUSE: barriers invalidated at
 // the end, return value uniform over the CTA; false = a wait timed out).
 // AR: kArithRef (the reference CPU operators' roundings, qp3d_exact.h) or
 // kArithFast (folded coefficients, fused multiply-adds, one reciprocal in S).
 template <bool SPEC, bool REUSE, bool HALF = false, int AR = kArithFast>
-__device__ __forceinline__ bool step_tile(const CUtensorMap *tm, const PlaneParams &p,
+__device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams &p,
                                           const Coefs &k, int tile_x, int y0, int x0, int z0,
-                                          int z1, bool win_writer, unsigned char *smem)
+                                          int z1, bool win_writer, const DeferSeg &seg,
+                                          unsigned char *smem)
 {
-    const SmemLayout L = smem_layout(tile_x, p.pml, p.nsrc);
+    const SmemLayout L = smem_layout(tile_x, p.pml, p.nsrc, step_streams(p.pml));
     float4 *tab = reinterpret_cast<float4 *>(smem + L.tab_off);
+    float *ytab = reinterpret_cast<float *>(smem + L.ytab_off);
     SrcEntry *csrc = reinterpret_cast<SrcEntry *>(smem + L.src_off);
     float *misc = reinterpret_cast<float *>(smem + L.misc_off);
-    int *misc_i = reinterpret_cast<int *>(smem + L.misc_off + 16);
+    unsigned *misc_u = reinterpret_cast<unsigned *>(smem + L.misc_off + 16);
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int q = tid & (kQuadsY - 1), r = tid / kQuadsY;
     const int nzc = z1 - z0;
     Pipe P;
-    pipe_setup(P, smem, tile_x, p.pml, y0, x0, z0, nzc);
-    if (!REUSE) pipe_hooks(P, p);
+    pipe_setup(P, smem, L, p, !REUSE, tile_x, y0, x0, z0, nzc);
     const int nx = p.nx, ny = p.ny, nz = p.nz, pml = p.pml;
-    int next_issue = 0;
-    if (tid == 0) {
-        pipe_init(P);
-        next_issue = min(kRing, P.nplanes);
-        for (int i = 0; i < next_issue; ++i) pipe_issue(P, tm, i);
-        if (SPEC) {
-            float lo, hi, pred;
-            spec_window(p, lo, hi, pred);
-            misc[0] = threshold_m2(lo);
-            misc[1] = threshold_m2(hi);
-            if (win_writer) {
-                p.win[0] = lo;
-                p.win[1] = hi;
-                p.win[2] = pred;
-            }
-        } else {
-            misc[0] = misc[1] = threshold_m2(p.gmax[p.step]);
-        }
-        int n = 0;
-        for (int e = 0; e < p.nsrc; ++e) {
-            SrcEntry s = p.src[e];
-            if (s.x >= x0 && s.x < x0 + tile_x && s.y >= y0 && s.y < y0 + kTileY && s.z >= z0 &&
-                s.z < z1 && n < p.nsrc)
-                csrc[n++] = s;
-        }
-        misc_i[0] = n;
-    }
-    for (int i = tid; i < 3 * pml; i += blockDim.x) tab[i] = p.layers[i];
-    __syncthreads();
-    const float T2lo = misc[0], T2hi = misc[1];
-    const int ncsrc = misc_i[0];
-
     const int x = x0 + r, yq = y0 + 4 * q;
     const bool row_ok = (r < tile_x) && (x < nx - kRadius);
     // quads wholly in the row padding (y >= ny, the last y tile) neither load
     // nor store: their cells are not part of the volume
     const bool mem_ok = row_ok && (yq < ny);
-    bool cell_ok[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) cell_ok[j] = row_ok && (yq + j >= kRadius) && (yq + j < ny - kRadius);
-    const int rc = (r + kRadius) * kBoxY + kHaloY + 4 * q;
-    // x and y face parts, constant along z
-    const int fx = x < pml ? 0 : (x >= nx - pml ? 1 : -1);
-    const int lix = x < pml ? pml - x : x - nx + pml;
-    int fy[4], liy[4];
-    bool any_fy = false;
+    // bits per cell of the quad: updated; of a y face
+    unsigned okb = 0, fyb = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int y = yq + j;
-        fy[j] = y < pml ? 2 : (y >= ny - pml ? 3 : -1);
-        liy[j] = y < pml ? pml - y : y - ny + pml;
-        any_fy = any_fy || (cell_ok[j] && fy[j] >= 0);
+        if (row_ok && y >= kRadius && y < ny - kRadius) okb |= 1u << j;
+        if (y < pml || y >= ny - pml) fyb |= 1u << j;
     }
-    const bool xy_face = row_ok && (fx >= 0 || any_fy);
-    const int hy = ny - 2 * pml;
+    Taps T = taps_start(P, r, q);
+    // the x face part, constant along z
+    const int fx = x < pml ? 0 : (x >= nx - pml ? 1 : -1);
+    const int lix = x < pml ? pml - x : x - nx + pml;
+    const bool xy_face = row_ok && (fx >= 0 || (fyb & okb));
+    const bool xy_face_warp = __any_sync(0xffffffffu, xy_face);
+    // whether the tile reaches into the never-updated band or the row padding
+    const bool y_edge = y0 < kRadius || y0 + kTileY > ny - kRadius;
     const float dt = p.dt;
     const float dt2 = __fmul_rn(dt, dt);
     // the reference adds source * wavelet to every cell (CPU_function.c:326-338):
     // a cell without a source gets +-0, which turns a -0 into +0 when the
     // product is +0
     const float zw = __fmul_rn(0.0f, p.wavelet);
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 
+    // The cell's own values (u(k-1), the parameters, the PML state) are copied
+    // one plane ahead into the thread's slots by cp.async, and read after the
+    // stencil: they hold no registers while the stencil runs.
+    float4 *own = reinterpret_cast<float4 *>(smem + L.own_off) + tid;
+    const int nthr = plane_threads(tile_x);   // a batched CTA may have more
+    auto prefetch_params = [&](unsigned b) {
+        if (!mem_ok) return;
+        if (HALF) {
+            cp_async8(own + nthr, p.h_vp + b);
+            cp_async8(own + 2 * nthr, p.h_eps + b);
+            cp_async8(own + 3 * nthr, p.h_del + b);
+        } else {
+            cp_async16(own + nthr, p.prm_v + b);
+            cp_async16(own + 2 * nthr, p.prm_e + b);
+            cp_async16(own + 3 * nthr, p.prm_r + b);
+        }
+    };
+    auto prefetch_u = [&](unsigned b) {
+        if (mem_ok) cp_async16(own, p.u_prev + b);
+    };
+    auto prefetch_pml = [&](unsigned b, bool z_face) {
+        if (mem_ok && (xy_face || z_face)) {
+            cp_async16(own + 4 * nthr, p.w1o + b);
+            cp_async16(own + 5 * nthr, p.w1c + b);
+            cp_async16(own + 6 * nthr, p.w3o + b);
+            cp_async16(own + 7 * nthr, p.w3c + b);
+            cp_async16(own + 8 * nthr, p.po + b);
+            cp_async16(own + 9 * nthr, p.pc + b);
+            cp_async16(own + 10 * nthr, p.w21o + b);
+        }
+    };
+    auto face_of_z = [&](int z) { return z < pml ? 4 : (z >= nz - pml ? 5 : -1); };
     float mx = 0.0f;
-    bool ok = true;
-    int waited = 0;
-    long long base = (long long)z0 * p.plane + (long long)x * p.ldy + yq;
-    for (int t = 0; t < nzc; ++t, base += p.plane) {
-        const int z = z0 + t;
-        const int fz = z < pml ? 4 : (z >= nz - pml ? 5 : -1);
-        const int liz = z < pml ? pml - z : z - nz + pml;
-        const bool pml_quad = xy_face || (row_ok && fz >= 0);
-        float4 u1v = zero4, Vv = zero4, Ev = zero4, Rv = zero4;
-        uint2 hv = make_uint2(0u, 0u), he = hv, hd = hv;
-        if (mem_ok) {
-            u1v = ldg4(p.u_prev + base);
-            if (HALF) {   // widened after the stencil, when the loads have landed
-                hv = __ldg(reinterpret_cast<const uint2 *>(p.h_vp + base));
-                he = __ldg(reinterpret_cast<const uint2 *>(p.h_eps + base));
-                hd = __ldg(reinterpret_cast<const uint2 *>(p.h_del + base));
-            } else {
-                Vv = ldg4(p.prm_v + base);
-                Ev = ldg4(p.prm_e + base);
-                Rv = ldg4(p.prm_r + base);
+    unsigned base = (unsigned)((long long)z0 * p.plane + (long long)x * p.ldy + yq);
+    const unsigned plane = (unsigned)p.plane;
+
+    // Before the previous kernel has finished (grid launches): barriers, the
+    // parameters and the layer coefficients, which no step changes.
+    prefetch_params(base);
+    if (tid == 0) {
+        misc_u[0] = misc_u[1] = 0;   // sources of this column, deferred cells
+        pipe_init(P);
+    }
+    for (int i = tid; i < 3 * pml; i += blockDim.x)
+        tab[i] = AR == kArithRef ? p.layers[i] : step_layer(p.layers[i]);
+    if (AR == kArithFast && tid < kTileY) {   // layer coefficients of the tile's y cells
+        const int y = y0 + tid;
+        float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (y < pml) {
+            if (y > 0) c = step_layer(p.layers[pml + pml - y]);   // y = 0: never updated
+        } else if (y >= ny - pml && y < ny) {
+            c = step_layer(p.layers[pml + y - ny + pml]);
+            c.w = -c.w;
+        }
+        ytab[tid] = c.x;
+        ytab[kTileY + tid] = c.y;
+        ytab[2 * kTileY + tid] = c.z;
+        ytab[3 * kTileY + tid] = c.w;
+    }
+    if (!REUSE) pdl_wait();
+    if (tid == 0) pipe_start(P, tm);
+    prefetch_u(base);
+    if (xy_face_warp || face_of_z(z0) >= 0) prefetch_pml(base, face_of_z(z0) >= 0);
+    // The thresholds.  A speculative step finds them where the resolution of
+    // the step before left them; otherwise two threads of the last warp work
+    // them out while the first loads are on their way.
+    if (tid >> 5 == P.ncw - 1 && lane < 2) {
+        if (!SPEC) {
+            misc[lane] = threshold_m2(p.gmax[p.step]);
+        } else if (p.win_ready) {
+            misc[lane] = p.win[3 + lane];
+        } else {
+            float w[3];
+            spec_window(p, p.step, p.spec_err, w);
+            misc[lane] = threshold_m2(w[lane]);
+            if (win_writer && lane == 0) {
+                p.win[0] = w[0];
+                p.win[1] = w[1];
+                p.win[2] = w[2];
             }
         }
-        float4 w11 = zero4, w12 = zero4, w31 = zero4, w32 = zero4, p1 = zero4, p2 = zero4,
-               w21 = zero4;
-        if (pml_quad && mem_ok) {
-            w11 = ldg4(p.w1o + base); w12 = ldg4(p.w1c + base);
-            w31 = ldg4(p.w3o + base); w32 = ldg4(p.w3c + base);
-            p1 = ldg4(p.po + base);   p2 = ldg4(p.pc + base);
-            w21 = ldg4(p.w21o + base);
-        }
-        if (tid == 0 && t >= kPrefetch + 1 && !pipe_refill(P, tm, t, next_issue)) ok = false;
-        while (ok && waited <= t + 2 * kRadius) {
-            ok = pipe_wait(P, waited);
-            if (ok) ++waited;
-        }
-        ok = __all_sync(0xffffffffu, ok);   // warps stay converged for the collectives below
-        if (!ok) break;
+    }
+    __syncthreads();
+    for (int e = tid; e < p.nsrc; e += blockDim.x) {
+        const SrcEntry s = p.src[e];
+        if (s.x >= x0 && s.x < x0 + tile_x && s.y >= y0 && s.y < y0 + kTileY && s.z >= z0 &&
+            s.z < z1)
+            csrc[atomicAdd(&misc_u[0], 1u)] = s;
+    }
+    if (p.nsrc) __syncthreads();
+    const float T2lo = misc[0], T2hi = misc[1];
+    const int ncsrc = (int)misc_u[0];
+    bool ok = true;
+    // One plane of a warp.  PML: whether a cell of the warp is of the shell.
+    // The body exists twice, so that the warps of the interior carry nothing
+    // of the shell's update: sharing one body, with the update under a branch,
+    // cost them 160 of 650 instructions a plane.
+    auto plane_step = [&](int t, auto shell) {
+        constexpr bool PML = decltype(shell)::value;
+        const int z = z0 + t;
+        const int fz = PML ? face_of_z(z) : -1;
         float Ux[4], Uy[4], Uz[4], Uxx[4], Uyy[4], Uzz[4], u0[4];
-        if (AR == kArithRef)
-            quad_derivs_ref(P.ring, P.slot_floats, t, rc, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
-        else
-            quad_derivs<true>(P.ring, P.slot_floats, t, rc, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
-        if (HALF) quad_params_half(hv, he, hd, Vv, Ev, Rv);
-        // scalar operator, GPU_kernel.cu:93-111 / CPU_function.c:339-370
+        if (AR == kArithRef) quad_derivs_ref(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
+        else quad_derivs<true>(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
+        // a thread without a cell reads whatever its slots hold: it stores nothing
+        cp_async_wait();
+        const float4 u1v = own[0];
+        float4 Vv, Ev, Rv;
+        if (HALF) {
+            quad_params_half(*reinterpret_cast<const uint2 *>(own + nthr),
+                             *reinterpret_cast<const uint2 *>(own + 2 * nthr),
+                             *reinterpret_cast<const uint2 *>(own + 3 * nthr), Vv, Ev, Rv);
+        } else {
+            Vv = own[nthr];
+            Ev = own[2 * nthr];
+            Rv = own[3 * nthr];
+        }
+        if (t + 1 < nzc) {
+            prefetch_u(base + plane);
+            prefetch_params(base + plane);
+        }
+        // |grad u|^2, and the step's own max |grad u|
         float h2[4], m2[4];
-        bool above[4], amb[4];
-        bool any_above = false;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (AR == kArithRef) {
@@ -1196,377 +1309,410 @@ __device__ __forceinline__ bool step_tile(const CUtensorMap *tm, const PlanePara
                 h2[j] = fmaf(Uy[j], Uy[j], __fmul_rn(Ux[j], Ux[j]));
                 m2[j] = fmaf(Uz[j], Uz[j], h2[j]);
             }
-            if (SPEC && cell_ok[j]) {   // three-input max: one instruction fewer per cell
-                float t;
-                asm("max.f32 %0, %1, %2, %3;" : "=f"(t) : "f"(mx), "f"(fabsf(Ux[j])), "f"(fabsf(Uy[j])));
-                mx = fmaxf(t, fabsf(Uz[j]));
-            }
-            above[j] = m2[j] > T2lo;
-            if (!SPEC && p.dec_in && row_ok) above[j] = (p.dec_in[base >> 5] >> (4 * q + j)) & 1u;
-            amb[j] = SPEC && cell_ok[j] && above[j] && !(m2[j] > T2hi);
-            any_above = any_above || (row_ok && above[j]);
         }
-        float S[4], e1[4];   // S; 1 + 2 eps
-        float KS[4];         // fast arithmetic: (vp dt)^2 S
+        if (SPEC) {   // three-input max: one instruction fewer per cell
+            auto add_max = [&](int j) {
+                float t2;
+                asm("max.f32 %0, %1, %2, %3;" : "=f"(t2) : "f"(mx), "f"(fabsf(Ux[j])), "f"(fabsf(Uy[j])));
+                mx = fmaxf(t2, fabsf(Uz[j]));
+            };
+            if (!y_edge) {   // rows past the tile are left out at the end
+                add_max(0); add_max(1); add_max(2); add_max(3);
+            } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) e1[j] = __fadd_rn(1.0f, f4(Ev, j));
-        if (AR == kArithRef) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                S[j] = 1.0f;
-                if (cell_ok[j] && above[j])
-                    S[j] = xr::scalar_s(Ux[j], Uy[j], Uz[j], m2[j], f4(Ev, j), f4(Rv, j));
+                for (int j = 0; j < 4; ++j)
+                    if ((okb >> j) & 1u) add_max(j);
             }
-        } else if (__any_sync(0xffffffffu, any_above)) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {   // cells (0,1) and (2,3) as pairs
-                const int j0 = 2 * h, j1 = 2 * h + 1;
-                const float2 s = aniso_s2(make_float2(h2[j0], h2[j1]), make_float2(m2[j0], m2[j1]),
-                                          __fmul2_rn(make_float2(Uz[j0], Uz[j1]),
-                                                     make_float2(Uz[j0], Uz[j1])),
-                                          make_float2(f4(Ev, j0), f4(Ev, j1)),
-                                          make_float2(f4(Rv, j0), f4(Rv, j1)));
-                KS[j0] = __fmul_rn(k_of_vp(f4(Vv, j0), dt), above[j0] ? s.x : 1.0f);
-                KS[j1] = __fmul_rn(k_of_vp(f4(Vv, j1), dt), above[j1] ? s.y : 1.0f);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) KS[j] = __fmul_rn(k_of_vp(f4(Vv, j), dt), 1.0f);
         }
-        float out[4], alt[4];
+        // Scalar operator, GPU_kernel.cu:93-111 / CPU_function.c:339-370.
+        // kS: S in the reference arithmetic, (vp dt)^2 S in the fast one; k1:
+        // the same with S = 1.  Most warps lie wholly below the threshold
+        // (S = 1) or wholly above it; the others decide cell by cell, and
+        // list the cells whose decision waits for the exact max.
+        float kS[4], k1[4], e1[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (AR == kArithRef) {
-                out[j] = xr::interior_update(u0[j], f4(u1v, j), Uxx[j], Uyy[j], Uzz[j], e1[j],
-                                             S[j], f4(Vv, j), dt2);
-                alt[j] = xr::interior_update(u0[j], f4(u1v, j), Uxx[j], Uyy[j], Uzz[j], e1[j],
-                                             1.0f, f4(Vv, j), dt2);   // S = 1, deferred cells
-            } else {
-                const float Lp = fmaf(e1[j], __fadd_rn(Uxx[j], Uyy[j]), Uzz[j]);
-                const float lin = fmaf(2.0f, u0[j], -f4(u1v, j));
-                out[j] = fmaf(KS[j], Lp, lin);
-                alt[j] = fmaf(__fmul_rn(k_of_vp(f4(Vv, j), dt), 1.0f), Lp, lin);
-            }
+            k1[j] = AR == kArithRef ? 1.0f : k_of_vp(f4(Vv, j), dt);
+            e1[j] = __fadd_rn(1.0f, f4(Ev, j));
+            kS[j] = k1[j];
         }
-        if (__any_sync(0xffffffffu, pml_quad)) {
-            float n13[4], n21[4], n33[4], n3[4];
+        unsigned pmlb = 0;   // bits of the quad's PML cells
+        if (PML) pmlb = (fx >= 0 || fz >= 0 ? 15u : fyb) & okb;
+        unsigned above = 0;
+        const bool bits = !SPEC && (p.dec_in || p.dec_out);   // decisions replayed or kept
+        if (bits || !__all_sync(0xffffffffu, !row_ok || max4(m2) <= T2lo)) {
+            if (AR == kArithRef) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                int f, li;
-                cell_face(fx, lix, fy[j], liy[j], fz, liz, f, li);
-                const bool is_pml = pml_quad && cell_ok[j] && f >= 0;
-                const float4 lt = tab[is_pml ? (f >> 1) * pml + li : 0];
-                if (AR == kArithRef) {
-                    n13[j] = n33[j] = n3[j] = 0.0f;
-                    n21[j] = f4(w21, j);
-                    if (is_pml) {
-                        const bool isx = f < 2, isz = f >= 4;
-                        xr::PmlLayer Lr;
-                        Lr.a1h = lt.x; Lr.a1l = lt.y;
-                        Lr.a2 = __fmaf_rn(2.0f, lt.z, -1.0f);
-                        Lr.a3 = __fsub_rn(1.0f, lt.z);
-                        Lr.dd = lt.w;
-                        const float Unn = isx ? Uxx[j] : (isz ? Uzz[j] : Uyy[j]);
-                        const float Un = isx ? Ux[j] : (isz ? Uz[j] : Uy[j]);
-                        const float tang = isz ? __fadd_rn(Uxx[j], Uyy[j])
-                                               : __fadd_rn(Uzz[j], __fmul_rn(e1[j], isx ? Uyy[j] : Uxx[j]));
-                        const float vdt = __fmul_rn(f4(Vv, j), dt);
-                        const xr::PmlOut o = xr::pml_update(isz, (f & 1) != 0, S[j], e1[j], vdt,
-                                                            Unn, Un, tang, dt, Lr, f4(w11, j),
-                                                            f4(w12, j), f4(w21, j), f4(w31, j),
-                                                            f4(w32, j), f4(p1, j), f4(p2, j));
-                        out[j] = o.u3;
-                        n13[j] = o.w13; n21[j] = o.w21; n33[j] = o.w33; n3[j] = o.p3;
-                        if (SPEC && amb[j]) {   // the S = 1 update, kept for the fix-up
-                            const xr::PmlOut o1 = xr::pml_update(isz, (f & 1) != 0, 1.0f, e1[j],
-                                                                 vdt, Unn, Un, tang, dt, Lr,
-                                                                 f4(w11, j), f4(w12, j),
-                                                                 f4(w21, j), f4(w31, j),
-                                                                 f4(w32, j), f4(p1, j), f4(p2, j));
-                            alt[j] = o1.u3;
-                            p.apml[base + j] = make_float4(o1.w13, o1.w21, o1.w33, o1.p3);
-                        }
-                    }
+                for (int j = 0; j < 4; ++j)
+                    if (m2[j] > T2lo) above |= 1u << j;
+                if (!SPEC && p.dec_in && row_ok) above = (p.dec_in[base >> 5] >> (4 * q)) & 15u;
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if ((above & okb) >> j & 1u)
+                        kS[j] = xr::scalar_s(Ux[j], Uy[j], Uz[j], m2[j], f4(Ev, j), f4(Rv, j));
+            } else {
+                float S[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {   // cells (0,1) and (2,3) as pairs
+                    const int j0 = 2 * h, j1 = 2 * h + 1;
+                    const float2 v = aniso_s2(f2(h2[j0], h2[j1]), f2(m2[j0], m2[j1]),
+                                              __fmul2_rn(f2(Uz[j0], Uz[j1]), f2(Uz[j0], Uz[j1])),
+                                              f2(f4(Ev, j0), f4(Ev, j1)),
+                                              f2(f4(Rv, j0), f4(Rv, j1)));
+                    S[j0] = v.x;
+                    S[j1] = v.y;
+                }
+                if (!bits && __all_sync(0xffffffffu, !row_ok || min4(m2) > T2hi)) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) kS[j] = __fmul_rn(k1[j], S[j]);
                 } else {
-                    const float4 lc = fast_layer(lt);
-                    const float v = pml_cell(f < 0 ? 0 : f, lc, KS[j], e1[j], Ux[j], Uy[j], Uz[j],
-                                             Uxx[j], Uyy[j], Uzz[j], dt, f4(w11, j), f4(w12, j),
-                                             f4(w21, j), f4(w31, j), f4(w32, j), f4(p1, j),
-                                             f4(p2, j), n13[j], n21[j], n33[j], n3[j]);
-                    if (SPEC && is_pml && amb[j]) {
-                        // the S = 1 update of a deferred cell and its split-field
-                        // outputs, kept for the fix-up
-                        float a13, a21, a33, a3;
-                        alt[j] = pml_cell(f, lc, __fmul_rn(k_of_vp(f4(Vv, j), dt), 1.0f), e1[j],
-                                          Ux[j], Uy[j], Uz[j], Uxx[j], Uyy[j], Uzz[j], dt,
-                                          f4(w11, j), f4(w12, j), f4(w21, j), f4(w31, j),
-                                          f4(w32, j), f4(p1, j), f4(p2, j), a13, a21, a33, a3);
-                        p.apml[base + j] = make_float4(a13, a21, a33, a3);
-                    }
-                    out[j] = is_pml ? v : out[j];
-                    n13[j] = is_pml ? n13[j] : 0.0f;
-                    n33[j] = is_pml ? n33[j] : 0.0f;
-                    n3[j] = is_pml ? n3[j] : 0.0f;
-                    n21[j] = is_pml ? n21[j] : f4(w21, j);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (m2[j] > T2lo) above |= 1u << j;
+                    if (!SPEC && p.dec_in && row_ok) above = (p.dec_in[base >> 5] >> (4 * q)) & 15u;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        kS[j] = (above >> j) & 1u ? __fmul_rn(k1[j], S[j]) : k1[j];
                 }
             }
-            if (pml_quad && mem_ok) {
-                *reinterpret_cast<float4 *>(p.w1n + base) = make_float4(n13[0], n13[1], n13[2], n13[3]);
-                *reinterpret_cast<float4 *>(p.w3n + base) = make_float4(n33[0], n33[1], n33[2], n33[3]);
-                *reinterpret_cast<float4 *>(p.pn + base) = make_float4(n3[0], n3[1], n3[2], n3[3]);
-                *reinterpret_cast<float4 *>(p.w21n + base) = make_float4(n21[0], n21[1], n21[2], n21[3]);
-            }
-        }
-        // source injection (GPU_kernel.cu:727, CPU_function.c:334): u3 += source * wavelet
-        bool has_src[4] = {false, false, false, false};
-        for (int e = 0; e < ncsrc; ++e) {
-            const SrcEntry s = csrc[e];
-            if (s.z == z && s.x == x) {
-                const int js = s.y - yq;
-                const float add = __fmul_rn(s.v, p.wavelet);
+            if (SPEC) {
+                unsigned nib = 0;
 #pragma unroll
-                for (int jj = 0; jj < 4; ++jj)
-                    if (jj == js) {
-                        out[jj] = __fadd_rn(out[jj], add);
-                        alt[jj] = __fadd_rn(alt[jj], add);
-                        has_src[jj] = true;
+                for (int j = 0; j < 4; ++j)
+                    if (!(m2[j] > T2hi)) nib |= 1u << j;
+                nib &= above & okb;
+                if (__any_sync(0xffffffffu, nib)) {
+                    unsigned pos = defer_places(&misc_u[1], nib);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (!((nib >> j) & 1u)) continue;
+                        if (pos < seg.cap) {
+                            const size_t e = seg.base + pos;
+                            p.dkey[e] = make_uint2(base + j, __float_as_uint(m2[j]));
+                            float4 v;
+                            if ((pmlb >> j) & 1u) {
+                                const int f = fx >= 0 ? fx : ((fyb >> j) & 1u ? 2 : 4);
+                                v = pml_inputs<AR>(f, e1[j], Ux[j], Uy[j], Uz[j], Uxx[j], Uyy[j],
+                                                   Uzz[j]);
+                            } else {
+                                v.x = interior_cell<AR>(u0[j], f4(u1v, j), Uxx[j], Uyy[j], Uzz[j],
+                                                        e1[j], k1[j], f4(Vv, j), dt2);
+                            }
+                            p.dval[e] = v;
+                        }
+                        ++pos;
                     }
+                }
             }
         }
-        if (AR == kArithRef) {
+        float out[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            out[j] = interior_cell<AR>(u0[j], f4(u1v, j), Uxx[j], Uyy[j], Uzz[j], e1[j], kS[j],
+                                       f4(Vv, j), dt2);
+        if (PML) {
+            if (xy_face || (row_ok && fz >= 0)) {
+                PmlOwn o;
+                o.w11 = own[4 * nthr]; o.w12 = own[5 * nthr];
+                o.w31 = own[6 * nthr]; o.w32 = own[7 * nthr];
+                o.p1 = own[8 * nthr];  o.p2 = own[9 * nthr];
+                o.w21 = own[10 * nthr];
+                PmlNew n;
+                const int liz = z < pml ? pml - z : z - nz + pml;
+                if (AR == kArithRef)
+                    pml_quad_ref(p, tab, kS, e1, Vv, Ux, Uy, Uz, Uxx, Uyy, Uzz, o, pmlb, fx, lix,
+                                 yq, fz, liz, out, n);
+                else
+                    pml_quad_fast(p, tab, ytab + 4 * q, kS, e1, Ux, Uy, Uz, Uxx, Uyy, Uzz, o, pmlb,
+                                  fyb, fx, lix, fz, liz, out, n);
+                if (mem_ok) {
+                    *reinterpret_cast<float4 *>(p.w1n + base) = make_float4(n.w13[0].x, n.w13[0].y, n.w13[1].x, n.w13[1].y);
+                    *reinterpret_cast<float4 *>(p.w3n + base) = make_float4(n.w33[0].x, n.w33[0].y, n.w33[1].x, n.w33[1].y);
+                    *reinterpret_cast<float4 *>(p.pn + base) = make_float4(n.p3[0].x, n.p3[0].y, n.p3[1].x, n.p3[1].y);
+                    *reinterpret_cast<float4 *>(p.w21n + base) = make_float4(n.w21[0].x, n.w21[0].y, n.w21[1].x, n.w21[1].y);
+                }
+            }
+        }
+        if (t + 1 < nzc) {
+            const bool z_face = face_of_z(z + 1) >= 0;
+            if (xy_face_warp || z_face) prefetch_pml(base + plane, z_face);
+        }
+        if (AR == kArithRef) {   // source injection (CPU_function.c:334): u3 += source * wavelet
+            unsigned srcb = 0;
+            for (int e = 0; e < ncsrc; ++e) {
+                const SrcEntry s = csrc[e];
+                if (s.z == z && s.x == x) {
+                    const float add = __fmul_rn(s.v, p.wavelet);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (s.y - yq == j) {
+                            out[j] = __fadd_rn(out[j], add);
+                            srcb |= 1u << j;
+                        }
+                }
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (!has_src[j]) {
-                    out[j] = __fadd_rn(out[j], zw);
-                    alt[j] = __fadd_rn(alt[j], zw);
-                }
+                if (!((srcb >> j) & 1u)) out[j] = __fadd_rn(out[j], zw);
         }
+        if (y_edge) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) out[j] = cell_ok[j] ? out[j] : u0[j];   // never updated
-        if (mem_ok) {
+            for (int j = 0; j < 4; ++j) out[j] = (okb >> j) & 1u ? out[j] : u0[j];   // never updated
+        }
+        if (mem_ok)
             *reinterpret_cast<float4 *>(p.u_out + base) = make_float4(out[0], out[1], out[2], out[3]);
-            // receiver plane (3dPureqPModeling_single_shot.cu:333-337)
-            if (p.record && z == p.sz && x >= pml && x < nx - pml) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int y = yq + j;
-                    if (cell_ok[j] && y >= pml && y < ny - pml)
-                        p.record[(long long)(x - pml) * hy + (y - pml)] = out[j];
-                }
-            }
-        }
-        // the step's decisions, when asked for (same word layout as the
-        // deferred-cell mask below)
+        // the step's decisions, when asked for: one bit per cell, 32 y cells a
+        // word (the 8 lanes of a row combine their 4 bits)
         if (!SPEC && p.dec_out) {
-            const unsigned nib = (unsigned)(cell_ok[0] && above[0]) |
-                                 ((unsigned)(cell_ok[1] && above[1]) << 1) |
-                                 ((unsigned)(cell_ok[2] && above[2]) << 2) |
-                                 ((unsigned)(cell_ok[3] && above[3]) << 3);
-            unsigned w = nib << (4 * q);
+            unsigned w = (above & okb) << (4 * q);
             w |= __shfl_xor_sync(0xffffffffu, w, 1);
             w |= __shfl_xor_sync(0xffffffffu, w, 2);
             w |= __shfl_xor_sync(0xffffffffu, w, 4);
             if (q == 0 && row_ok) p.dec_out[base >> 5] = w;
         }
-        // deferred cells: the row's bitmask word (the 8 lanes of a row combine
-        // their 4 bits; written every step, so stale bits never survive), and
-        // for a quad with any deferred cell its m2 and S = 1 values
-        if (SPEC) {
-            const unsigned nib = (unsigned)amb[0] | ((unsigned)amb[1] << 1) |
-                                 ((unsigned)amb[2] << 2) | ((unsigned)amb[3] << 3);
-            if (nib) {
-                *reinterpret_cast<float4 *>(p.am2 + base) = make_float4(m2[0], m2[1], m2[2], m2[3]);
-                *reinterpret_cast<float4 *>(p.av + base) = make_float4(alt[0], alt[1], alt[2], alt[3]);
+        pipe_release(P, tm, t);
+    };
+    for (int t = 0; t < nzc; taps_next(T, P, t), ++t, base += plane) {
+        ok = __all_sync(0xffffffffu, pipe_wait(P, t));   // warps stay converged for the collectives below
+        if (!ok) break;
+        if (xy_face_warp || face_of_z(z0 + t) >= 0) plane_step(t, std::true_type());
+        else plane_step(t, std::false_type());
+    }
+    cp_async_wait();
+    // What happens on one plane only stays out of the loop; each thread works
+    // on the cells it has just written.  Source injection (GPU_kernel.cu:727):
+    // u3 += source * wavelet.
+    if (AR == kArithFast && ok)
+        for (int e = 0; e < ncsrc; ++e) {
+            const SrcEntry s = csrc[e];
+            if (s.x == x && (unsigned)(s.y - yq) < 4u) {
+                float *u = p.u_out + ((long long)s.z * p.plane + (long long)x * p.ldy + s.y);
+                *u = __fadd_rn(*u, __fmul_rn(s.v, p.wavelet));
             }
-            unsigned w = nib << (4 * q);
-            w |= __shfl_xor_sync(0xffffffffu, w, 1);
-            w |= __shfl_xor_sync(0xffffffffu, w, 2);
-            w |= __shfl_xor_sync(0xffffffffu, w, 4);
-            if (q == 0 && row_ok) p.amask[base >> 5] = w;
         }
-        pipe_release(P, t);
+    // receiver plane (3dPureqPModeling_single_shot.cu:333-337)
+    if (p.record && ok && p.sz >= z0 && p.sz < z1 && mem_ok && x >= pml && x < nx - pml) {
+        const float4 u = *reinterpret_cast<const float4 *>(
+            p.u_out + ((long long)p.sz * p.plane + (long long)x * p.ldy + yq));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int y = yq + j;
+            if (((okb >> j) & 1u) && y >= pml && y < ny - pml)
+                p.record[(long long)(x - pml) * (ny - 2 * pml) + (y - pml)] = f4(u, j);
+        }
     }
-    if (!ok) {
-        atomicOr(p.err, kErrWaitTimeout);
-        if (tid == 0) pipe_drain(P, next_issue);
-    }
+    ok = pipe_finish(P, ok, p.err);
     if (SPEC) {
+        if (!row_ok) mx = 0.0f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         if (lane == 0 && mx > 0.0f &&
             mx > *reinterpret_cast<const volatile float *>(p.gmax + p.step))
             atomicMax(reinterpret_cast<unsigned *>(p.gmax + p.step), __float_as_uint(mx));
+        if (tid == 0) {
+            *seg.count = misc_u[1];
+            if (misc_u[1] > seg.cap) *const_cast<int *>(p.gate) = 1;   // re-run the step
+        }
     }
-    if (REUSE) {
-        ok = __syncthreads_and(ok) != 0;
-        if (tid == 0 && ok) pipe_inval(P);
-    }
+    if (REUSE && tid == 0 && ok) pipe_inval(P);
     return ok;
 }
 
 template <bool SPEC, bool HALF, int AR>
-__global__ void __launch_bounds__(kThreads, 2)
-    qp3d_step_kernel(const __grid_constant__ CUtensorMap tm_u, const PlaneParams p)
+__global__ void __launch_bounds__(kStepThreads, 2)
+    qp3d_step_kernel(const __grid_constant__ TileMaps tm, const PlaneParams p)
 {
-    if (!SPEC && p.gate && *p.gate == 0) return;
     extern __shared__ __align__(128) unsigned char smem[];
+    pdl_trigger();
     const int y0 = blockIdx.x * kTileY, x0 = kRadius + blockIdx.y * p.tile_x;
     const int z0 = kRadius + blockIdx.z * p.chunk_z;
     const int z1 = min(z0 + p.chunk_z, p.nz - kRadius);
-    if (z0 >= z1) return;
-    step_tile<SPEC, false, HALF, AR>(&tm_u, p, p.k, p.tile_x, y0, x0, z0, z1,
-                                     blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0, smem);
-}
-
-// Resolution and compaction of a speculative step, over the deferred-cell
-// bitmask (four words per thread).  Every block derives from the true max M
-// whether it fell in the predicted window and the threshold T2 of M (thread 0,
-// while the others load their words); block 0 also sets the re-run flag and
-// shifts the history of the prediction's relative errors.  *p.alt_count ends as the number of deferred
-// cells of the step; when M is inside the window, the deferred cells below
-// the threshold are listed in p.alist and counted in *p.fix_count.
-__device__ __forceinline__ void compact_body(const PlaneParams &p, unsigned block, int *redo,
-                                             float *spec_err)
-{
-    __shared__ unsigned s_warp[32], s_def[32];
-    __shared__ unsigned s_base;
-    const float M = p.gmax[p.step];   // complete: the step kernel has finished
-    const bool inside = (M >= p.win[0]) && (M <= p.win[1]);
-    __shared__ float s_T2;
-    if (threadIdx.x == 0) s_T2 = threshold_m2(M);
-    if (block == 0 && threadIdx.x == 0) {
-        *redo = inside ? 0 : 1;   // the fix-up sets it too when the list overflows
-        const float pred = p.win[2];
-#pragma unroll
-        for (int i = kSpecHist - 1; i > 0; --i) spec_err[i] = spec_err[i - 1];
-        spec_err[0] = pred > 0.0f ? fabsf(__fdiv_rn(M, pred) - 1.0f) : 1.0f;
-    }
-    const unsigned nwords = (unsigned)defer_mask_words(p.plane * p.nz);   // a multiple of 4
-    const unsigned w0 = (block * blockDim.x + threadIdx.x) * 4u;
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint4 wv = make_uint4(0u, 0u, 0u, 0u);
-    if (w0 < nwords) wv = *reinterpret_cast<const uint4 *>(p.amask + w0);
-    __syncthreads();
-    const float T2 = s_T2;
-    const unsigned ws[4] = {wv.x, wv.y, wv.z, wv.w};
-    unsigned fix[4] = {0u, 0u, 0u, 0u};
-    unsigned c = 0, dcnt = 0;
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        const unsigned w = ws[h];
-        dcnt += __popc(w);
-        if (w && inside) {
-            const float4 *m = reinterpret_cast<const float4 *>(p.am2 + (size_t)(w0 + h) * 32);
-#pragma unroll
-            for (int q4 = 0; q4 < 8; ++q4) {
-                const unsigned nib = (w >> (4 * q4)) & 15u;
-                if (!nib) continue;
-                const float4 v = m[q4];
-                const unsigned below = (unsigned)!(v.x > T2) | ((unsigned)!(v.y > T2) << 1) |
-                                       ((unsigned)!(v.z > T2) << 2) | ((unsigned)!(v.w > T2) << 3);
-                fix[h] |= (nib & below) << (4 * q4);
-            }
-        }
-        c += __popc(fix[h]);
-    }
-    unsigned incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (unsigned)o) incl += v;
-        dcnt += __shfl_xor_sync(0xffffffffu, dcnt, o);
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    if (lane == 0) s_def[warp] = dcnt;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned t = 0, d = 0;
-        for (unsigned i = 0; i < (blockDim.x >> 5); ++i) {
-            const unsigned v = s_warp[i];
-            s_warp[i] = t;
-            t += v;
-            d += s_def[i];
-        }
-        if (d) atomicAdd(p.alt_count, d);
-        s_base = t ? atomicAdd(p.fix_count, t) : 0u;
-    }
-    __syncthreads();
-    unsigned pos = s_base + s_warp[warp] + incl - c;
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        unsigned bits = fix[h];
-        while (bits) {
-            const int bit = __ffs(bits) - 1;
-            bits &= bits - 1;
-            if (pos < p.alist_cap) p.alist[pos] = (w0 + h) * 32u + (unsigned)bit;
-            ++pos;
-        }
-    }
-}
-
-__global__ void qp3d_compact_kernel(const PlaneParams p, int *redo, float *spec_err)
-{
-    compact_body(p, blockIdx.x, redo, spec_err);
-}
-
-// Fix-up of a speculative step: every listed cell (deferred and below the
-// true threshold) gets the S = 1 results the step kernel stored for it
-// (u(k+1), and at PML cells the split-field state).  Only called when the max
-// fell in the window and the list did not overflow.
-__device__ __forceinline__ void fixup_cells(const PlaneParams &p, unsigned n, unsigned first,
-                                            unsigned stride)
-{
-    const int nx = p.nx, ny = p.ny, nz = p.nz, pml = p.pml, hy = ny - 2 * pml;
-    const unsigned plane = (unsigned)p.plane, ldy = (unsigned)p.ldy;
-    for (unsigned i = first; i < n; i += stride) {
-        const unsigned idx = p.alist[i];
-        const int z = (int)(idx / plane);
-        const unsigned rem = idx - (unsigned)z * plane;
-        const int x = (int)(rem / ldy), y = (int)(rem - (unsigned)x * ldy);
-        const bool in_pml = x < pml || x >= nx - pml || y < pml || y >= ny - pml || z < pml ||
-                            z >= nz - pml;
-        const float out = p.av[idx];   // the step kernel's S = 1 value, source included
-        if (in_pml) {                  // and a PML cell's split-field outputs
-            const float4 s = p.apml[idx];
-            p.w1n[idx] = s.x;
-            p.w21n[idx] = s.y;
-            p.w3n[idx] = s.z;
-            p.pn[idx] = s.w;
-        }
-        p.u_out[idx] = out;
-        if (p.record && z == p.sz && x >= pml && x < nx - pml && y >= pml && y < ny - pml)
-            p.record[(long long)(x - pml) * hy + (y - pml)] = out;
-    }
-}
-
-// The fix-up of a speculative step, or its exact re-run when the max fell
-// outside the predicted window (*p.gate, set by the compaction) or the list
-// overflowed: one persistent grid of one CTA per SM.  The re-run takes the
-// step's tile columns in turn, so a step that needs none costs one short
-// wave instead of a full grid of CTAs that each read the gate and exit.
-template <bool HALF, int AR>
-__global__ void __launch_bounds__(kThreads, 1)
-    qp3d_fix_or_rerun_kernel(const __grid_constant__ CUtensorMap tm_u, const PlaneParams p)
-{
-    const unsigned n = *p.fix_count;
-    const bool rerun = *p.gate != 0 || n > p.alist_cap;
-    if (!rerun) {
-        fixup_cells(p, n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    if (z0 >= z1) {
+        pdl_wait();
         return;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *const_cast<int *>(p.gate) = 1;   // overflow: count it
-    extern __shared__ __align__(128) unsigned char smem[];
+    const unsigned id = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    const DeferSeg seg = {(size_t)id * p.dcap, p.dcap, p.dcount + id};
+    step_tile<SPEC, false, HALF, AR>(&tm, p, p.k, p.tile_x, y0, x0, z0, z1, id == 0, seg, smem);
+}
+
+// ---------------------------------------------------------------------------
+// Resolution of a speculative step, once its step kernel has finished and the
+// true max M of the step is known.  M outside the predicted window, or a
+// segment that ran over: the step is re-run exactly.  Otherwise every listed
+// cell that turns out to be below the threshold of M gets the S = 1 results
+// the step kernel stored for it.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool step_missed(const PlaneParams &p)
+{
+    const float M = p.gmax[p.step];
+    return !((M >= p.win[0]) && (M <= p.win[1])) || *p.gate != 0;
+}
+
+// The re-run flag of the step and the history of the prediction's relative
+// errors (one warp of the grid; lanes 0 and 1), and, for the shots of a single
+// launch (p.win_next), the window and the thresholds of the next step.
+// Threads that read the flag meanwhile come to the same step_missed either
+// way.
+__device__ __forceinline__ void step_account(const PlaneParams &p, float *spec_err)
+{
+    const int lane = threadIdx.x & 31;
+    const float M = p.gmax[p.step], pred = p.win[2];
+    const bool missed = step_missed(p);
+    float err[kSpecHist];
+#pragma unroll
+    for (int i = kSpecHist - 1; i > 0; --i) err[i] = spec_err[i - 1];
+    err[0] = pred > 0.0f ? fabsf(__fdiv_rn(M, pred) - 1.0f) : 1.0f;
+    __syncwarp(3u);
+    if (lane == 0) {
+        if (missed) *const_cast<int *>(p.gate) = 1;
+#pragma unroll
+        for (int i = 0; i < kSpecHist; ++i) spec_err[i] = err[i];
+    }
+    if (!p.win_next) return;
+    float w[3];
+    spec_window(p, p.step + 1, err, w);
+    p.win_next[3 + lane] = threshold_m2(w[lane]);
+    p.win_next[lane] = w[lane];
+    if (lane == 0) p.win_next[2] = w[2];
+}
+
+// S = 1 results of entry e, if its cell is below the threshold
+// (double)mode > 0.01 * (double)max  <=>  mode > Tf (see threshold_m2).
+template <bool HALF, int AR>
+__device__ __forceinline__ void fix_cell(const PlaneParams &p, float Tf, size_t e)
+{
+    const uint2 key = p.dkey[e];
+    const float4 v = p.dval[e];
+    if (__fsqrt_rn(__uint_as_float(key.y)) > Tf) return;
+    const int nx = p.nx, ny = p.ny, nz = p.nz, pml = p.pml;
+    const unsigned plane = (unsigned)p.plane, ldy = (unsigned)p.ldy, idx = key.x;
+    const int z = (int)(idx / plane);
+    const unsigned rem = idx - (unsigned)z * plane;
+    const int x = (int)(rem / ldy), y = (int)(rem - (unsigned)x * ldy);
+    const int fx = x < pml ? 0 : (x >= nx - pml ? 1 : -1);
+    const int fy = y < pml ? 2 : (y >= ny - pml ? 3 : -1);
+    const int fz = z < pml ? 4 : (z >= nz - pml ? 5 : -1);
+    float out = v.x;
+    if (fx >= 0 || fy >= 0 || fz >= 0) {
+        int f, li;
+        cell_face(fx, x < pml ? pml - x : x - nx + pml, fy, y < pml ? pml - y : y - ny + pml, fz,
+                  z < pml ? pml - z : z - nz + pml, f, li);
+        float vp, e1;
+        if (HALF) {
+            vp = __half2float(p.h_vp[idx]);
+            e1 = __fadd_rn(1.0f, __fmul_rn(2.0f, __half2float(p.h_eps[idx])));
+        } else {
+            vp = p.prm_v[idx];
+            e1 = __fadd_rn(1.0f, p.prm_e[idx]);
+        }
+        const xr::PmlOut o = pml_cell<AR>(
+            f, p.layers[(f >> 1) * pml + li], AR == kArithRef ? 1.0f : k_of_vp(vp, p.dt), e1, vp,
+            v, p.dt, p.w1o[idx], p.w1c[idx], p.w21o[idx], p.w3o[idx], p.w3c[idx], p.po[idx],
+            p.pc[idx]);
+        p.w1n[idx] = o.w13;
+        p.w21n[idx] = o.w21;
+        p.w3n[idx] = o.w33;
+        p.pn[idx] = o.p3;
+        out = o.u3;
+    }
+    bool has_src = false;
+    for (int i = 0; i < p.nsrc; ++i) {
+        const SrcEntry s = p.src[i];
+        if (s.z == z && s.x == x && s.y == y) {
+            out = __fadd_rn(out, __fmul_rn(s.v, p.wavelet));
+            has_src = true;
+        }
+    }
+    if (AR == kArithRef && !has_src) out = __fadd_rn(out, __fmul_rn(0.0f, p.wavelet));
+    p.u_out[idx] = out;
+    if (p.record && z == p.sz && x >= pml && x < nx - pml && y >= pml && y < ny - pml)
+        p.record[(long long)(x - pml) * (ny - 2 * pml) + (y - pml)] = out;
+}
+
+// A block's share of the segments, kThreads at a time: lens of them are
+// scanned to offsets, so that the threads share the cells evenly however the
+// lengths differ.  len(i) is segment i's length (0: none to fix), fix(i, j)
+// handles its entry j.
+template <class Len, class Fix>
+__device__ __forceinline__ void for_segment_cells(int nseg, Len len, Fix fix)
+{
+    __shared__ unsigned s_off[kThreads + 1], s_w[kThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    for (int first = 0; first * (int)gridDim.x + (int)blockIdx.x < nseg; first += blockDim.x) {
+        const long long i = blockIdx.x + (long long)(first + tid) * gridDim.x;
+        const unsigned c = i < nseg ? len((int)i) : 0u;
+        unsigned incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) s_w[warp] = incl;
+        __syncthreads();
+        unsigned add = 0, total = 0;
+        for (int w = 0; w < nw; ++w) {
+            if (w < warp) add += s_w[w];
+            total += s_w[w];
+        }
+        s_off[tid + 1] = add + incl;
+        if (tid == 0) s_off[0] = 0;
+        __syncthreads();
+        for (unsigned e = tid; e < total; e += blockDim.x) {
+            int lo = 0, hi = blockDim.x;   // s_off[lo] <= e < s_off[hi]
+            while (hi - lo > 1) {
+                const int m = (lo + hi) >> 1;
+                if (s_off[m] <= e) lo = m;
+                else hi = m;
+            }
+            fix((int)(blockIdx.x + (long long)(first + lo) * gridDim.x), e - s_off[lo]);
+        }
+        __syncthreads();
+    }
+}
+
+__device__ __forceinline__ float threshold_of(float gmax)
+{
+    return __double2float_rd(1.0e-02 * (double)gmax);
+}
+
+// Resolution of a single shot's speculative step: a persistent grid of two
+// CTAs per SM, held to the registers that leave room for a CTA of the next
+// step beside them.  The re-run takes the step's tile columns in turn, so a step
+// that needs none costs one short wave instead of a full grid of CTAs that
+// each read the flag and exit.
+template <bool HALF, int AR>
+__global__ void __launch_bounds__(kStepThreads, 2)
+    qp3d_fix_or_rerun_kernel(const __grid_constant__ TileMaps tm, const PlaneParams p,
+                             float *spec_err)
+{
+    pdl_trigger();
+    pdl_wait();
+    const bool rerun = step_missed(p);
     const int nyt = (p.ny - kRadius - 1) / kTileY + 1;
     const int nxt = (p.nx - 2 * kRadius + p.tile_x - 1) / p.tile_x;
     const int nch = (p.nz - 2 * kRadius + p.chunk_z - 1) / p.chunk_z;
     const int ntiles = nyt * nxt * nch;
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < 2) step_account(p, spec_err);
+    const float Tf = threshold_of(p.gmax[p.step]);
+    for_segment_cells(
+        ntiles,
+        [&](int i) {
+            const unsigned n = p.dcount[i];
+            if (n) atomicAdd(p.alt_count, n);
+            return rerun ? 0u : n;
+        },
+        [&](int i, unsigned j) { fix_cell<HALF, AR>(p, Tf, (size_t)i * p.dcap + j); });
+    if (!rerun) return;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const DeferSeg none = {0, 0, nullptr};
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int by = t % nyt, bx = (t / nyt) % nxt, bz = t / (nyt * nxt);
         const int z0 = kRadius + bz * p.chunk_z;
         const int z1 = min(z0 + p.chunk_z, p.nz - kRadius);
         if (z0 >= z1) continue;
-        if (!step_tile<false, true, HALF, AR>(&tm_u, p, p.k, p.tile_x, by * kTileY,
-                                              kRadius + bx * p.tile_x, z0, z1, false, smem))
+        if (!step_tile<false, true, HALF, AR>(&tm, p, p.k, p.tile_x, by * kTileY,
+                                              kRadius + bx * p.tile_x, z0, z1, false, none, smem))
             return;
     }
 }
@@ -1674,17 +1820,17 @@ __global__ void qp3d_to_half_dense_kernel(const float *a, __half *h, int ny, lon
 //                               k + 1.  The step is therefore the same
 //                               sequence of launches for every k and can be
 //                               captured once in a CUDA graph.
-//   qp3d_batch_plane_kernel     persistent CTAs (as many as are resident)
-//                               take work items -- one tile column of one
-//                               shot -- from an atomic queue and run the
-//                               gradmax or step tile body on it; uneven shot
-//                               sizes mix in one launch.
-//   qp3d_batch_compact_kernel,  the speculative resolution, compaction
-//   qp3d_batch_fixup_kernel     and fix-up, blockIdx.y = shot.
+//   qp3d_batch_plane_kernel     one CTA per work item -- one tile column of
+//                               one shot -- runs the gradmax or step tile
+//                               body on it; uneven shot sizes mix in one
+//                               launch.
+//   qp3d_batch_resolve_kernel   the resolution of a speculative step.
 // ---------------------------------------------------------------------------
 __global__ void qp3d_batch_prepare_kernel(const BatchShot *shots, int nshots, PlaneParams *pp,
                                           int *ctr, int *queues, int spec)
 {
+    pdl_trigger();
+    pdl_wait();
     const int k = *ctr;
     for (int s = threadIdx.x; s < nshots; s += blockDim.x) {
         const BatchShot &b = shots[s];
@@ -1716,18 +1862,23 @@ __global__ void qp3d_batch_prepare_kernel(const BatchShot *shots, int nshots, Pl
             p.wavelet = b.wavelet[k];
             p.spec = spec;
             p.gate = spec ? b.redo + k : nullptr;
-            p.win = b.win + 3 * (long long)k;
+            p.win = b.win + kWinFloats * (long long)k;
             p.spec_err = b.spec_err;
             p.delta_min = b.delta_min;
             p.spec_bias = b.spec_bias;
-            p.amask = b.amask;
-            p.am2 = b.am2;
-            p.av = b.av;
-            p.apml = b.apml;
+            p.dkey = b.dkey;
+            p.dval = b.dval;
             p.alt_count = b.alt_count + k;
-            p.alist = b.alist;
-            p.alist_cap = b.alist_cap;
-            p.fix_count = b.fix_count + k;
+            if (spec) {
+                float w[3];
+                spec_window(p, k, p.spec_err, w);
+                p.win[0] = w[0];
+                p.win[1] = w[1];
+                p.win[2] = w[2];
+                p.win[3] = threshold_m2(w[0]);
+                p.win[4] = threshold_m2(w[1]);
+                p.win_ready = 1;
+            }
         }
         pp[s] = p;
     }
@@ -1745,21 +1896,89 @@ size_t batch_smem_bytes(int tile_x, int pml, int nsrc)
     return kParamBytes + plane_smem_bytes(tile_x, pml, nsrc);
 }
 
-// KIND 0: gradmax, 1: exact step (skipped for shots whose gate is 0),
-// 2: speculative step.  Bounded for one CTA of kThreads per SM: the per-shot
-// parameters live in shared memory rather than in the constant bank, and held
-// to the two-CTA budget of 128 registers the step body spills (measured: 15 %
-// fewer shots/s).  The shape tuner then picks the tile height, which sets how
-// many CTAs share an SM (three of 128 threads at 16 rows).
+// One work item: KIND 0 gradmax, 1 exact step, 2 speculative step.  sp: a copy
+// of the shot's parameters in shared memory.
+template <int KIND, bool REUSE, int AR>
+__device__ __forceinline__ bool batch_item(const BatchArgs &b, int it, unsigned char *smem)
+{
+    PlaneParams *sp = reinterpret_cast<PlaneParams *>(smem);
+    unsigned char *body = smem + kParamBytes;
+    const WorkItem w = b.work[it];
+    {
+        const unsigned *src = reinterpret_cast<const unsigned *>(b.pp + w.shot);
+        unsigned *dst = reinterpret_cast<unsigned *>(sp);
+        for (int i = threadIdx.x; i < (int)(sizeof(PlaneParams) / 4); i += blockDim.x)
+            dst[i] = src[i];
+    }
+    const TileMaps *tm = b.tm + 3 * w.shot;
+    if (threadIdx.x == 0)   // maps written by the host before the launch
+        for (int i = 0; i < 3; ++i) {
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&tm[i].z)
+                         : "memory");
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&tm[i].c)
+                         : "memory");
+        }
+    __syncthreads();
+    const PlaneParams &p = *sp;
+    tm += p.ucur;
+    if (KIND == 0) {
+        float mx;
+        const bool ok = gradmax_tile<REUSE, AR>(tm, p, b.k, w.tile_x, w.y0, w.x0, w.z0, w.z1, body, mx);
+        gradmax_publish(p, mx);
+        return ok;
+    }
+    const bool first = w.y0 == 0 && w.x0 == kRadius && w.z0 == kRadius;
+    const DeferSeg seg = {w.dbase, w.dcap, b.dcount + it};
+    return step_tile<KIND == 2, REUSE, false, AR>(tm, p, b.k, w.tile_x, w.y0, w.x0, w.z0, w.z1,
+                                                  first, seg, body);
+}
+
+// All items of a step, one per CTA, longest columns first.
 template <int KIND, int AR>
-__global__ void __launch_bounds__(kThreads, 1) qp3d_batch_plane_kernel(const __grid_constant__ BatchArgs b)
+__global__ void __launch_bounds__(kStepThreads, 2)
+    qp3d_batch_plane_kernel(const __grid_constant__ BatchArgs b)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    pdl_trigger();
+    pdl_wait();
+    if (b.pp[b.work[blockIdx.x].shot].active) batch_item<KIND, false, AR>(b, blockIdx.x, smem);
+}
+
+// After a speculative step of all shots: the resolution of every shot, then
+// the exact step of those that missed, by persistent CTAs that take the items
+// from a queue (most steps have none).
+template <int AR>
+__global__ void __launch_bounds__(kStepThreads, 2)
+    qp3d_batch_resolve_kernel(const __grid_constant__ BatchArgs b)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     // item slot double-buffered by iteration: thread 0 can run one iteration
     // ahead of the others only on the skip path, which has no second barrier
-    __shared__ int s_item[2], s_run[2];
-    PlaneParams *sp = reinterpret_cast<PlaneParams *>(smem);
-    unsigned char *body = smem + kParamBytes;
+    __shared__ int s_item[2], s_run[2], s_missed;
+    pdl_trigger();
+    pdl_wait();
+    if (threadIdx.x == 0) s_missed = 0;
+    __syncthreads();
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < 2)
+        for (int s = 0; s < b.nshots; ++s)
+            if (b.pp[s].active) step_account(b.pp[s], const_cast<float *>(b.pp[s].spec_err));
+    for (int s = threadIdx.x; s < b.nshots; s += blockDim.x)
+        if (b.pp[s].active && step_missed(b.pp[s])) s_missed = 1;
+    for_segment_cells(
+        b.nwork,
+        [&](int i) {
+            const PlaneParams &g = b.pp[b.work[i].shot];
+            if (!g.active) return 0u;
+            const unsigned n = b.dcount[i];
+            if (n) atomicAdd(g.alt_count, n);
+            return n && !step_missed(g) ? n : 0u;
+        },
+        [&](int i, unsigned j) {
+            const PlaneParams &g = b.pp[b.work[i].shot];
+            fix_cell<false, AR>(g, threshold_of(g.gmax[g.step]), b.work[i].dbase + j);
+        });
+    __syncthreads();
+    if (!s_missed) return;
     for (int iter = 0;; ++iter) {
         const int slot = iter & 1;
         if (threadIdx.x == 0) {
@@ -1767,8 +1986,7 @@ __global__ void __launch_bounds__(kThreads, 1) qp3d_batch_plane_kernel(const __g
             int run = 0;
             if (it < b.nwork) {
                 const PlaneParams &g = b.pp[b.work[it].shot];
-                run = g.active != 0;
-                if (KIND == 1) run = run && !(g.gate && *g.gate == 0);
+                run = g.active && step_missed(g);
             }
             s_item[slot] = it;
             s_run[slot] = run;
@@ -1776,54 +1994,8 @@ __global__ void __launch_bounds__(kThreads, 1) qp3d_batch_plane_kernel(const __g
         __syncthreads();
         const int it = s_item[slot];
         if (it >= b.nwork) return;
-        if (!s_run[slot]) continue;
-        const WorkItem w = b.work[it];
-        {
-            const unsigned *src = reinterpret_cast<const unsigned *>(b.pp + w.shot);
-            unsigned *dst = reinterpret_cast<unsigned *>(sp);
-            for (int i = threadIdx.x; i < (int)(sizeof(PlaneParams) / 4); i += blockDim.x)
-                dst[i] = src[i];
-        }
-        const CUtensorMap *tm = b.tm + 3 * w.shot;
-        if (threadIdx.x == 0)   // maps written by the host before the launch
-            for (int i = 0; i < 3; ++i)
-                asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tm + i)
-                             : "memory");
-        __syncthreads();
-        const PlaneParams &p = *sp;
-        tm += p.ucur;
-        bool ok;
-        if (KIND == 0) {
-            ok = gradmax_tile<true, AR>(tm, p, b.k, w.tile_x, w.y0, w.x0, w.z0, w.z1, body);
-        } else {
-            const bool first = w.y0 == 0 && w.x0 == kRadius && w.z0 == kRadius;
-            ok = step_tile<KIND == 2, true, false, AR>(tm, p, b.k, w.tile_x, w.y0, w.x0, w.z0,
-                                                       w.z1, first, body);
-        }
-        if (!ok) return;
+        if (s_run[slot] && !batch_item<1, true, AR>(b, it, smem)) return;
     }
-}
-
-__global__ void qp3d_batch_compact_kernel(const __grid_constant__ BatchArgs b)
-{
-    const PlaneParams &p = b.pp[blockIdx.y];
-    if (!p.active || !p.spec) return;
-    if ((long long)blockIdx.x * blockDim.x * 4 >= defer_mask_words(p.plane * p.nz)) return;
-    compact_body(p, blockIdx.x, const_cast<int *>(p.gate), const_cast<float *>(p.spec_err));
-}
-
-// Fix-up of the shots whose max fell in their window; a shot whose list
-// overflowed is marked for the exact pass instead.
-__global__ void qp3d_batch_fixup_kernel(const __grid_constant__ BatchArgs b)
-{
-    const PlaneParams &p = b.pp[blockIdx.y];
-    if (!p.active || !p.spec || *p.gate) return;
-    const unsigned n = *p.fix_count;
-    if (n > p.alist_cap) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) *const_cast<int *>(p.gate) = 1;
-        return;
-    }
-    fixup_cells(p, n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1864,16 +2036,6 @@ __device__ __forceinline__ void row_window(const float *f, long long i, int y, i
         w[4 * b] = v.x; w[4 * b + 1] = v.y; w[4 * b + 2] = v.z; w[4 * b + 3] = v.w;
     }
 }
-
-// 16 bytes global -> shared through L2 (cp.async.cg), completed by
-// adj_pf_wait in the same thread
-__device__ __forceinline__ void adj_pf(float4 *dst, const float *src)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void adj_pf_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void adj_pf_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Pass A, four consecutive y cells (a quad) per thread, block and warp
 // shapes as pass B.  The derivatives of u^k take the operation order of
@@ -2095,8 +2257,7 @@ __global__ void __launch_bounds__(256) qp3d_adj_b_kernel(const AdjParams a)
     __shared__ __align__(16) float4 pnu[256];
     const bool vec_nu = y + 3 < a.ny;
     if (vec_nu) {
-        adj_pf(&pnu[threadIdx.x], a.Nu + i);
-        adj_pf_commit();
+        cp_async16(&pnu[threadIdx.x], a.Nu + i);
     }
     const bool inside = !a.live && xw - kRadius >= a.pml && xw + 4 + kRadius <= a.nx - a.pml &&
                         yw - kRadius >= a.pml && yw + 32 + kRadius <= a.ny - a.pml &&
@@ -2167,7 +2328,7 @@ __global__ void __launch_bounds__(256) qp3d_adj_b_kernel(const AdjParams a)
     }
     float *nu = a.Nu + i;
     if (vec_nu) {
-        adj_pf_wait();
+        cp_async_wait();
         float4 v = pnu[threadIdx.x];
         v.x += acc[0]; v.y += acc[1]; v.z += acc[2]; v.w += acc[3];
         *reinterpret_cast<float4 *>(nu) = v;
@@ -2224,6 +2385,24 @@ __global__ void qp3d_from_bf16_kernel(const __nv_bfloat16 *h, float *a, long lon
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
+// A kernel of a time step, as a programmatic dependent of the one before it.
+template <typename... P, typename... A>
+static cudaError_t launch_pdl(void (*fn)(P...), dim3 grid, int threads, size_t smem,
+                              cudaStream_t stream, const A &...args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, fn, args...);
+}
+
 template <typename F>
 static cudaError_t set_smem(F *fn, int bytes)
 {
@@ -2239,151 +2418,116 @@ cudaError_t configure_kernels()
         (e = set_smem(qp3d_batch_plane_kernel<2, kArithFast>, bytes)) ||
         (e = set_smem(qp3d_batch_plane_kernel<0, kArithRef>, bytes)) ||
         (e = set_smem(qp3d_batch_plane_kernel<1, kArithRef>, bytes)) ||
-        (e = set_smem(qp3d_batch_plane_kernel<2, kArithRef>, bytes)))
+        (e = set_smem(qp3d_batch_plane_kernel<2, kArithRef>, bytes)) ||
+        (e = set_smem(qp3d_batch_resolve_kernel<kArithFast>, bytes)) ||
+        (e = set_smem(qp3d_batch_resolve_kernel<kArithRef>, bytes)))
         return e;
 #define QP3D_STEP_SMEM(AR)                                                                   \
     if ((e = set_smem(qp3d_step_kernel<true, false, AR>, bytes)) ||                         \
         (e = set_smem(qp3d_step_kernel<false, false, AR>, bytes)) ||                        \
         (e = set_smem(qp3d_step_kernel<true, true, AR>, bytes)) ||                          \
         (e = set_smem(qp3d_step_kernel<false, true, AR>, bytes)) ||                         \
-        (e = set_smem(qp3d_gradmax_kernel<false, AR>, bytes)) ||                            \
+        (e = set_smem(qp3d_gradmax_kernel<AR>, bytes)) ||                                   \
         (e = set_smem(qp3d_fix_or_rerun_kernel<false, AR>, bytes)) ||                              \
         (e = set_smem(qp3d_fix_or_rerun_kernel<true, AR>, bytes)))                                 \
         return e;
     QP3D_STEP_SMEM(kArithFast)
     QP3D_STEP_SMEM(kArithRef)
 #undef QP3D_STEP_SMEM
-    return set_smem(qp3d_gradmax_kernel<true, kArithFast>, bytes);
+    return cudaSuccess;
 }
 
-// whole warps: rows past tile_x are idle, so every warp collective sees 32 lanes
-static inline int plane_threads(int tile_x) { return (kQuadsY * tile_x + 31) & ~31; }
-
-cudaError_t launch_gradmax(const CUtensorMap &tm_u, const PlaneParams &p, dim3 grid, size_t smem,
-                           cudaStream_t stream, int variant)
+cudaError_t launch_gradmax(const TileMaps &tm, const PlaneParams &p, dim3 grid,
+                           cudaStream_t stream)
 {
     const int t = plane_threads(p.tile_x);
-    if (p.arith == kArithRef)
-        qp3d_gradmax_kernel<false, kArithRef><<<grid, t, smem, stream>>>(tm_u, p);
-    else if (variant == 0)
-        qp3d_gradmax_kernel<false, kArithFast><<<grid, t, smem, stream>>>(tm_u, p);
-    else
-        qp3d_gradmax_kernel<true, kArithFast><<<grid, t, smem, stream>>>(tm_u, p);
-    return cudaGetLastError();
+    const size_t smem = gradmax_smem_bytes(p.tile_x);
+    return launch_pdl(p.arith == kArithRef ? qp3d_gradmax_kernel<kArithRef>
+                                           : qp3d_gradmax_kernel<kArithFast>,
+                      grid, t, smem, stream, tm, p);
 }
 
 template <int AR>
-static void launch_step_t(const CUtensorMap &tm_u, const PlaneParams &p, dim3 grid, int t,
-                          size_t smem, cudaStream_t stream)
+static cudaError_t launch_step_t(const TileMaps &tm, const PlaneParams &p, dim3 grid, int t,
+                                 size_t smem, cudaStream_t stream)
 {
-    if (p.half_params) {
-        if (p.spec) qp3d_step_kernel<true, true, AR><<<grid, t, smem, stream>>>(tm_u, p);
-        else qp3d_step_kernel<false, true, AR><<<grid, t, smem, stream>>>(tm_u, p);
-    } else {
-        if (p.spec) qp3d_step_kernel<true, false, AR><<<grid, t, smem, stream>>>(tm_u, p);
-        else qp3d_step_kernel<false, false, AR><<<grid, t, smem, stream>>>(tm_u, p);
-    }
+    auto *fn = p.half_params ? (p.spec ? qp3d_step_kernel<true, true, AR>
+                                       : qp3d_step_kernel<false, true, AR>)
+                             : (p.spec ? qp3d_step_kernel<true, false, AR>
+                                       : qp3d_step_kernel<false, false, AR>);
+    return launch_pdl(fn, grid, t, smem, stream, tm, p);
 }
 
-cudaError_t launch_step(const CUtensorMap &tm_u, const PlaneParams &p, dim3 grid, size_t smem,
+cudaError_t launch_step(const TileMaps &tm, const PlaneParams &p, dim3 grid, size_t smem,
                         cudaStream_t stream)
 {
     const int t = plane_threads(p.tile_x);
-    if (p.arith == kArithRef) launch_step_t<kArithRef>(tm_u, p, grid, t, smem, stream);
-    else launch_step_t<kArithFast>(tm_u, p, grid, t, smem, stream);
-    return cudaGetLastError();
+    return p.arith == kArithRef ? launch_step_t<kArithRef>(tm, p, grid, t, smem, stream)
+                                : launch_step_t<kArithFast>(tm, p, grid, t, smem, stream);
 }
 
-cudaError_t configure_gradmax_partial()
+cudaError_t configure_gradmax_single()
 {
-    cudaError_t e;
-    if ((e = set_smem(qp3d_gradmax_partial_kernel<kArithFast>, 200 * 1024))) return e;
-    return set_smem(qp3d_gradmax_partial_kernel<kArithRef>, 200 * 1024);
+    return set_smem(qp3d_gradmax_single_kernel, 200 * 1024);
 }
 
-cudaError_t launch_gradmax_partial(const CUtensorMap &tm_u, const PlaneParams &p, dim3 grid,
-                                   size_t smem, cudaStream_t stream, float *partial,
-                                   unsigned nblocks, float *out)
+cudaError_t launch_gradmax_single(const TileMaps &tm, const PlaneParams &p, dim3 grid,
+                                  cudaStream_t stream, GradmaxScratch *sc, float *out,
+                                  unsigned *host_flags)
 {
-    const int t = plane_threads(p.tile_x);
-    if (p.arith == kArithRef)
-        qp3d_gradmax_partial_kernel<kArithRef><<<grid, t, smem, stream>>>(tm_u, p, partial);
-    else
-        qp3d_gradmax_partial_kernel<kArithFast><<<grid, t, smem, stream>>>(tm_u, p, partial);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    qp3d_reduce_max_kernel<<<1, 1024, 0, stream>>>(partial, nblocks, p.err, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_compact(const PlaneParams &p, int *redo, float *spec_err, cudaStream_t stream)
-{
-    const long long words = defer_mask_words(p.plane * p.nz);
-    qp3d_compact_kernel<<<(unsigned)((words / 4 + 255) / 256), 256, 0, stream>>>(p, redo,
-                                                                                 spec_err);
+    qp3d_gradmax_single_kernel<<<grid, plane_threads(p.tile_x), gradmax_smem_bytes(p.tile_x),
+                                 stream>>>(tm, p, sc, out, host_flags);
     return cudaGetLastError();
 }
 
 template <int AR>
-static void launch_fix_or_rerun_t(const CUtensorMap &tm_u, const PlaneParams &p, int grid, int t,
-                                  size_t smem, cudaStream_t stream)
+static cudaError_t launch_fix_or_rerun_t(const TileMaps &tm, const PlaneParams &p,
+                                         float *spec_err, int grid, int t, size_t smem,
+                                         cudaStream_t stream)
 {
-    if (p.half_params) qp3d_fix_or_rerun_kernel<true, AR><<<grid, t, smem, stream>>>(tm_u, p);
-    else qp3d_fix_or_rerun_kernel<false, AR><<<grid, t, smem, stream>>>(tm_u, p);
+    return launch_pdl(p.half_params ? qp3d_fix_or_rerun_kernel<true, AR>
+                                    : qp3d_fix_or_rerun_kernel<false, AR>,
+                      dim3(grid), t, smem, stream, tm, p, spec_err);
 }
 
-cudaError_t launch_fix_or_rerun(const CUtensorMap &tm_u, const PlaneParams &p, int nsm,
-                                size_t smem, cudaStream_t stream)
+cudaError_t launch_fix_or_rerun(const TileMaps &tm, const PlaneParams &p, float *spec_err,
+                                int nsm, size_t smem, cudaStream_t stream)
 {
     const int t = plane_threads(p.tile_x);
-    if (p.arith == kArithRef) launch_fix_or_rerun_t<kArithRef>(tm_u, p, nsm, t, smem, stream);
-    else launch_fix_or_rerun_t<kArithFast>(tm_u, p, nsm, t, smem, stream);
-    return cudaGetLastError();
+    return p.arith == kArithRef
+               ? launch_fix_or_rerun_t<kArithRef>(tm, p, spec_err, 2 * nsm, t, smem, stream)
+               : launch_fix_or_rerun_t<kArithFast>(tm, p, spec_err, 2 * nsm, t, smem, stream);
 }
-
-int batch_plane_threads(int tile_x) { return plane_threads(tile_x); }
 
 cudaError_t launch_batch_prepare(const BatchShot *shots, int nshots, PlaneParams *pp, int *ctr,
                                  int *queues, int spec, cudaStream_t stream)
 {
-    qp3d_batch_prepare_kernel<<<1, 128, 0, stream>>>(shots, nshots, pp, ctr, queues, spec);
-    return cudaGetLastError();
+    return launch_pdl(qp3d_batch_prepare_kernel, dim3(1), 128, 0, stream, shots, nshots, pp, ctr,
+                      queues, spec);
 }
 
-static const void *batch_plane_fn(int kind, int arith)
+template <int AR>
+static cudaError_t launch_batch_plane_t(int kind, const BatchArgs &b, int threads, size_t smem,
+                                        cudaStream_t stream)
 {
-    if (arith == kArithRef)
-        return kind == 0 ? (const void *)qp3d_batch_plane_kernel<0, kArithRef>
-             : kind == 1 ? (const void *)qp3d_batch_plane_kernel<1, kArithRef>
-                         : (const void *)qp3d_batch_plane_kernel<2, kArithRef>;
-    return kind == 0 ? (const void *)qp3d_batch_plane_kernel<0, kArithFast>
-         : kind == 1 ? (const void *)qp3d_batch_plane_kernel<1, kArithFast>
-                     : (const void *)qp3d_batch_plane_kernel<2, kArithFast>;
+    auto *fn = kind == 0 ? qp3d_batch_plane_kernel<0, AR>
+             : kind == 1 ? qp3d_batch_plane_kernel<1, AR> : qp3d_batch_plane_kernel<2, AR>;
+    return launch_pdl(fn, dim3(b.nwork), threads, smem, stream, b);
 }
 
-cudaError_t batch_ctas_per_sm(int kind, int arith, int threads, size_t smem, int *n)
-{
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, batch_plane_fn(kind, arith), threads,
-                                                         smem);
-}
-
-cudaError_t launch_batch_plane(int kind, const BatchArgs &b, int grid, int threads, size_t smem,
+cudaError_t launch_batch_plane(int kind, const BatchArgs &b, int threads, size_t smem,
                                cudaStream_t stream)
 {
-    void *args[] = {const_cast<BatchArgs *>(&b)};
-    return cudaLaunchKernel(batch_plane_fn(kind, b.arith), dim3(grid), dim3(threads), args, smem,
-                            stream);
+    return b.arith == kArithRef ? launch_batch_plane_t<kArithRef>(kind, b, threads, smem, stream)
+                                : launch_batch_plane_t<kArithFast>(kind, b, threads, smem, stream);
 }
 
-cudaError_t launch_batch_fixup(const BatchArgs &b, int nshots, int blocks_per_shot,
-                               long long max_words, cudaStream_t stream)
+cudaError_t launch_batch_resolve(const BatchArgs &b, int grid, int threads, size_t smem,
+                                 cudaStream_t stream)
 {
-    qp3d_batch_compact_kernel<<<dim3((unsigned)((max_words / 4 + 255) / 256), nshots), 256, 0,
-                                stream>>>(b);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    qp3d_batch_fixup_kernel<<<dim3(blocks_per_shot, nshots), 256, 0, stream>>>(b);
-    return cudaGetLastError();
+    return launch_pdl(b.arith == kArithRef ? qp3d_batch_resolve_kernel<kArithRef>
+                                           : qp3d_batch_resolve_kernel<kArithFast>,
+                      dim3(grid), threads, smem, stream, b);
 }
 
 cudaError_t launch_band_sources(float *u_new, const float *u_cur, const SrcEntry *src, int n,

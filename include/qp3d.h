@@ -208,8 +208,8 @@ int qp3d_shot_time(qp3d_ctx *ctx, int nsteps, float *ms_total, float *ms_step,
 int qp3d_shot_launches_per_step(const qp3d_ctx *ctx);
 long long qp3d_ctx_launch_count(const qp3d_ctx *ctx);
 
-/* Launch tuning.  Keys: "gradmax_variant" (0: shared-memory z taps,
- * 1: register queue), "tile_x" (rows per tile, 0 = automatic),
+/* Launch tuning.  Keys: "gradmax_variant" (0 or 1: one form of the kernel
+ * serves both), "tile_x" (rows per tile, 0 = automatic),
  * "chunks" (z chunks, 0 = automatic), "threshold_mode" (0: gradmax pre-pass
  * every step, 1: speculative threshold), "spec_delta_ppm" (smallest
  * half-width of the predicted max window; default 1% for single shots, 2% in
