@@ -52,7 +52,9 @@ namespace qp3d {
 struct AdjState {
     long long vol = 0;
     int nt = 0, C = 0, nck = 0, bf16 = 1, keep = 0;
-    float *L[9] = {}, *N[9] = {}, *Cf[6] = {}, *g[3] = {};
+    // adjoint of u: this step's, the step after's, the step before's; the seven
+    // PML states; coefficient fields; gradient sums
+    float *U[3] = {}, *L[7] = {}, *N[7] = {}, *Cf[6] = {}, *g[3] = {};
     float *seg = nullptr;          // C volumes: u^k of the segment (keep: C = nt)
     void *ck = nullptr;            // nck checkpoints x 9 volumes
     float *resid = nullptr;        // nt * hx * hy: d_obs, then the residual
@@ -64,6 +66,7 @@ struct AdjState {
 void adjoint_free(AdjState *s)
 {
     if (!s) return;
+    for (auto *p : s->U) cudaFree(p);
     for (auto *p : s->L) cudaFree(p);
     for (auto *p : s->N) cudaFree(p);
     for (auto *p : s->Cf) cudaFree(p);
@@ -99,10 +102,9 @@ void live_state(qp3d_ctx *ctx, int k, float *v[9])
 int alloc_state(qp3d_ctx *ctx, AdjState *s, int C, int nck, int bf16, int keep, size_t rec)
 {
     const size_t vb = (size_t)s->vol * sizeof(float);
-    for (int i = 0; i < 9; ++i) {
-        CK(cudaMalloc(&s->L[i], vb));
-        CK(cudaMalloc(&s->N[i], vb));
-    }
+    for (auto *&p : s->U) CK(cudaMalloc(&p, vb));
+    for (auto *&p : s->L) CK(cudaMalloc(&p, vb));
+    for (auto *&p : s->N) CK(cudaMalloc(&p, vb));
     for (auto *&p : s->Cf) CK(cudaMalloc(&p, vb));
     for (auto *&p : s->g) CK(cudaMalloc(&p, vb));
     CK(cudaMalloc(&s->seg, vb * C));
@@ -208,7 +210,7 @@ extern "C" int qp3d_adjoint(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model 
         float *const *u;
         bool on;
         ~OwnGuard() { if (on) (void)qp3d_internal_restore_wavefields(c, u); }
-    } own_guard{ctx, own, keep != 0};
+    } own_guard{ctx, own, true};
     if (keep) CK(cudaMemsetAsync(S->seg, 0, vb, ctx->stream));   // u^0
     for (int k = 0; k < nt; ++k) {
         if (keep) {
@@ -240,6 +242,7 @@ extern "C" int qp3d_adjoint(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model 
     CK(cudaMemcpyAsync(&J, S->misfit, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     // every entry the adjoint kernels never write must be zero in both
     // buffers of each pair (see qp3d_adj_a_kernel)
+    for (auto *p : S->U) CK(cudaMemsetAsync(p, 0, vb, ctx->stream));
     for (auto *p : S->L) CK(cudaMemsetAsync(p, 0, vb, ctx->stream));
     for (auto *p : S->N) CK(cudaMemsetAsync(p, 0, vb, ctx->stream));
     for (auto *p : S->Cf) CK(cudaMemsetAsync(p, 0, vb, ctx->stream));
@@ -252,13 +255,18 @@ extern "C" int qp3d_adjoint(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model 
     a.hx = ctx->hx; a.hy = ctx->hy; a.plane = ctx->plane; a.k = ctx->coefs; a.dt = g->dt;
     a.VP = ctx->VP; a.E2 = ctx->E2; a.R8 = ctx->R8; a.layers = ctx->layers;
     a.live = ctx->adj_live;
+    a.err = ctx->errword;
+    a.wait_ns = ctx->wait_ns;
+    plan_adjoint(a, ctx->nsm);
     for (int c = (keep ? 1 : nck) - 1; c >= 0; --c) {
         const int k0 = c * C, k1 = std::min(nt, k0 + C);
         if (!keep) {   // restore the checkpoint, recompute keeping u^k
             ctx->dec_mode = 2;
             if ((rc = qp3d_internal_restore_step(ctx, k0))) return rc;
+            for (int j = 0; j < 3; ++j) ctx->U[j] = own[j];
             float *v[9];
             live_state(ctx, k0, v);
+            v[0] = S->seg;
             for (int j = 0; j < 9; ++j) {
                 if (S->bf16 && j >= 2)
                     CKL(launch_from_bf16(
@@ -268,10 +276,14 @@ extern "C" int qp3d_adjoint(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model 
                     CK(cudaMemcpyAsync(v[j], ck_slot(c, j), vb, cudaMemcpyDeviceToDevice,
                                        ctx->stream));
             }
-            for (int k = k0; k < k1; ++k) {
-                CK(cudaMemcpyAsync(S->seg + (size_t)(k - k0) * vol, ctx->U[ctx->cur], vb,
-                                   cudaMemcpyDeviceToDevice, ctx->stream));
-                if ((rc = qp3d_internal_enqueue_step(ctx))) return rc;
+            // the steps write u(k+1) into its slot; the adjoint of the last
+            // step needs no u(k1)
+            for (int k = k0; k + 1 < k1; ++k) {
+                float *const slot = S->seg + (size_t)(k - k0) * vol;
+                if ((rc = qp3d_internal_bind_wavefields(
+                         ctx, k == k0 ? v[1] : slot - vol, slot, slot + vol)) ||
+                    (rc = qp3d_internal_enqueue_step(ctx)))
+                    return rc;
             }
         }
         CKL(launch_threshold(ctx->gmax + k0, S->T2, k1 - k0, ctx->stream));
@@ -280,19 +292,30 @@ extern "C" int qp3d_adjoint(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model 
             a.dec = keep ? nullptr : S->dec + (size_t)k * (size_t)(vol / 32);
             a.u = S->seg + (size_t)(k - k0) * vol;
             a.resid = S->resid + (size_t)k * ctx->hx * ctx->hy;
-            const float **Lc[9] = {&a.Lu, &a.Lup, &a.Lw1, &a.Lw1o, &a.Lp, &a.Lpo, &a.Lw21,
-                                   &a.Lw3, &a.Lw3o};
-            float **Nc[9] = {&a.Nu, &a.Nup, &a.Nw1, &a.Nw1o, &a.Np, &a.Npo, &a.Nw21, &a.Nw3,
-                             &a.Nw3o};
-            for (int j = 0; j < 9; ++j) {
+            a.resid_prev = k + 1 < nt ? a.resid + (size_t)ctx->hx * ctx->hy : nullptr;
+            a.Lu = S->U[0];
+            a.Lprev = S->U[1];
+            a.Nu = S->U[2];
+            const float **Lc[7] = {&a.Lw1, &a.Lw1o, &a.Lp, &a.Lpo, &a.Lw21, &a.Lw3, &a.Lw3o};
+            float **Nc[7] = {&a.Nw1, &a.Nw1o, &a.Np, &a.Npo, &a.Nw21, &a.Nw3, &a.Nw3o};
+            for (int j = 0; j < 7; ++j) {
                 *Lc[j] = S->L[j];
                 *Nc[j] = S->N[j];
             }
             for (int j = 0; j < 6; ++j) a.C[j] = S->Cf[j];
             a.gK = S->g[0]; a.gE = S->g[1]; a.gD = S->g[2];
-            CKL(launch_adjoint_step(a, ctx->stream));
+            TileMaps tm;
+            const CUresult cr = encode_tile_maps(ctx->encode, a.u, a.nx, a.ny, a.nz, a.ldy,
+                                                 a.tile_x, &tm);
+            if (cr != CUDA_SUCCESS)
+                return ctx_fail(ctx, QP3D_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)cr);
+            CKL(launch_adjoint_step(tm, a, ctx->stream));
             ++ctx->launches;   // two passes
-            for (int j = 0; j < 9; ++j) std::swap(S->L[j], S->N[j]);
+            for (int j = 0; j < 7; ++j) std::swap(S->L[j], S->N[j]);
+            float *const next = S->U[2];   // u's adjoint moves on one step
+            S->U[2] = S->U[1];
+            S->U[1] = S->U[0];
+            S->U[0] = next;
         }
     }
     // ---- gradient: interior cells, added to the caller's FP64 arrays

@@ -392,7 +392,7 @@ constexpr int kSpecFirstStep = 3;
 
 static bool use_spec(const qp3d_ctx *ctx, int k)
 {
-    return ctx->threshold_mode == 1 && ctx->dec_mode == 0 && k >= kSpecFirstStep;
+    return ctx->threshold_mode == 1 && ctx->dec_mode != 2 && k >= kSpecFirstStep;
 }
 
 // Enqueue one time step.  ev_* are optional events bracketing the main step
@@ -466,7 +466,7 @@ static int enqueue_step(qp3d_ctx *ctx, cudaEvent_t ev_g0, cudaEvent_t ev_g1, cud
         if (ev_g1) CK(cudaEventRecord(ev_g1, ctx->stream));
     } else {
         if (ev_g0) CK(cudaEventRecord(ev_g0, ctx->stream));
-        CKL(launch_gradmax(ctx->tm[a], p, grid, ctx->stream));
+        if (ctx->dec_mode != 2) CKL(launch_gradmax(ctx->tm[a], p, grid, ctx->stream));
         if (ev_g1) CK(cudaEventRecord(ev_g1, ctx->stream));
         if (ev_s0) CK(cudaEventRecord(ev_s0, ctx->stream));
         CKL(launch_step(ctx->tm[a], p, grid, ctx->smem, ctx->stream));
@@ -490,8 +490,8 @@ static int enqueue_step(qp3d_ctx *ctx, cudaEvent_t ev_g0, cudaEvent_t ev_g1, cud
 }
 
 // For qp3d_adjoint.cu: one step of the loaded shot, and a jump back to the
-// start of step `step` (rotation as from a reset; the per-step bookkeeping
-// of the steps to come is cleared; the caller restores the state volumes).
+// start of step `step` (rotation as from a reset; the caller restores the
+// state volumes and replays the steps' decisions, so their maxima stay).
 int qp3d_internal_enqueue_step(qp3d_ctx *ctx)
 {
     if (ctx->step >= ctx->g.nt) return ctx_fail(ctx, QP3D_ERR_STATE, "step past nt");
@@ -526,11 +526,6 @@ int qp3d_internal_restore_wavefields(qp3d_ctx *ctx, float *const U[3])
 int qp3d_internal_restore_step(qp3d_ctx *ctx, int step)
 {
     if (step < 0 || step >= ctx->g.nt) return ctx_fail(ctx, QP3D_ERR_ARG, "bad step %d", step);
-    const size_t n = (size_t)(ctx->g.nt - step);
-    CK(cudaMemsetAsync(ctx->gmax + step, 0, n * sizeof(float), ctx->stream));
-    CK(cudaMemsetAsync(ctx->win + kWinFloats * (size_t)step, 0, kWinFloats * n * sizeof(float), ctx->stream));
-    CK(cudaMemsetAsync(ctx->redo + step, 0, n * sizeof(int), ctx->stream));
-    CK(cudaMemsetAsync(ctx->alt_count + step, 0, n * sizeof(unsigned), ctx->stream));
     ctx->step = step;
     ctx->win_step = -1;
     ctx->cur = (3 - step % 3) % 3;

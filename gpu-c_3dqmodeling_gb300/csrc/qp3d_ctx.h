@@ -106,8 +106,7 @@ struct qp3d_ctx {
     unsigned long long wait_ns = 0;
     int hold_plane = 0;
     // threshold decisions of each step (qp3d_adjoint): 1 = record them into
-    // dec_base + step * dec_words, 2 = replay them; steps then run exactly
-    // (gradmax pre-pass), not speculatively
+    // dec_base + step * dec_words, 2 = replay them (no maximum is needed then)
     int dec_mode = 0;
     unsigned *dec_base = nullptr;
     long long dec_words = 0;

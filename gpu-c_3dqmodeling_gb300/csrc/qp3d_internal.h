@@ -111,9 +111,10 @@ struct PlaneParams {
     int nsrc;
     unsigned *err;
     // threshold decisions of the step, one bit per cell, 32 y cells a word
-    // (word = pitched index / 32; exact steps only): written to dec_out, or
-    // read from dec_in instead of being taken (the gradient's recomputation
-    // replays the forward's)
+    // (word = pitched index / 32; FP32 parameters only): written to dec_out
+    // (a speculative step's resolution clears the bits of the cells it fixes),
+    // or read from dec_in instead of being taken (exact steps: the gradient's
+    // recomputation replays the forward's)
     unsigned *dec_out;
     const unsigned *dec_in;
     unsigned long long wait_ns;   // limit of every bounded device wait (0: 2 s)
@@ -194,7 +195,9 @@ struct BatchArgs {
 // One backward step of the adjoint (qp3d_adjoint.cu): the adjoint state of
 // s^{k+1} (L*) to that of s^k (N*), with the scalar operator of step k frozen
 // from u^k and the step's threshold.  C: coefficient fields of the
-// transposed derivatives (x, y, z first; xx, yy, zz second).
+// transposed derivatives (x, y, z first; xx, yy, zz second).  The adjoint of
+// u_prev is not kept: at a cell of the interior it is minus the adjoint of u
+// of the step after, elsewhere zero.
 struct AdjParams {
     int nx, ny, nz, ldy, pml, sz, hx, hy;
     long long plane;
@@ -206,14 +209,24 @@ struct AdjParams {
     const float *T2;                       // threshold m2 of step k
     const unsigned *dec;                   // or its decisions, one bit per cell (null: T2)
     const float *resid;                    // record residual of step k (hx * hy)
-    const float *Lu, *Lup, *Lw1, *Lw1o, *Lp, *Lpo, *Lw21, *Lw3, *Lw3o;
-    float *Nu, *Nup, *Nw1, *Nw1o, *Np, *Npo, *Nw21, *Nw3, *Nw3o;
+    const float *resid_prev;               // and of step k + 1 (null: k is the last)
+    const float *Lprev;                    // Lu of step k + 1 (zero for the last step)
+    const float *Lu, *Lw1, *Lw1o, *Lp, *Lpo, *Lw21, *Lw3, *Lw3o;
+    float *Nu, *Nw1, *Nw1o, *Np, *Npo, *Nw21, *Nw3, *Nw3o;
     float *C[6];
     float *gK, *gE, *gD;                   // gradient sums over the steps
     int live;                              // 1: S's dependence on grad u included
+    int tile_x, chunk_z;                   // pass A's tiles
+    unsigned *err;
+    unsigned long long wait_ns;
 };
 
-cudaError_t launch_adjoint_step(const AdjParams &a, cudaStream_t stream);
+// Tile height of pass A: with its 15 streams two CTAs of 24 rows fit an SM,
+// 12 warps with up to 168 registers a thread.
+constexpr int kAdjTileX = 24;
+void plan_adjoint(AdjParams &a, int nsm);
+// tm: u^k's maps for tiles of a.tile_x rows
+cudaError_t launch_adjoint_step(const TileMaps &tm, const AdjParams &a, cudaStream_t stream);
 cudaError_t launch_threshold(const float *gmax, float *T2, int n, cudaStream_t stream);
 cudaError_t launch_residual(const float *rec, const float *dobs, float *r, long long n,
                             double *misfit, cudaStream_t stream);

@@ -591,11 +591,8 @@ __device__ bool pipe_finish(const Pipe &P, bool ok, unsigned *err)
     return false;
 }
 
-// hooks: the launch's wait limit (0: 2 s) and the plane-withholding test hook
-// apply (grid launches; the hook to the first CTA only)
 __device__ __forceinline__ void pipe_setup(Pipe &P, unsigned char *smem, const SmemLayout &L,
-                                           const PlaneParams &p, bool hooks, int tile_x, int y0,
-                                           int x0, int z0, int nzc)
+                                           int tile_x, int y0, int x0, int z0, int nzc)
 {
     P.zr = reinterpret_cast<float *>(smem);
     P.cr = reinterpret_cast<float *>(smem + L.c_off);
@@ -613,11 +610,14 @@ __device__ __forceinline__ void pipe_setup(Pipe &P, unsigned char *smem, const S
     P.ncw = blockDim.x >> 5;   // every warp of the CTA releases every iteration
     P.wait_ns = 2000000000ull;
     P.hold = -1;
-    if (hooks) {
-        if (p.wait_ns) P.wait_ns = p.wait_ns;
-        if (p.hold_plane > 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0)
-            P.hold = p.hold_plane - 1;
-    }
+}
+
+// The launch's wait limit (0: 2 s) and the plane-withholding test hook (the
+// first CTA of a grid launch only).
+__device__ __forceinline__ void pipe_hooks(Pipe &P, unsigned long long wait_ns, int hold_plane)
+{
+    if (wait_ns) P.wait_ns = wait_ns;
+    if (hold_plane > 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) P.hold = hold_plane - 1;
 }
 
 // Before a CTA reuses its barriers for another tile (thread 0, after a CTA
@@ -666,7 +666,8 @@ __device__ __forceinline__ bool gradmax_tile(const TileMaps *tm, const PlanePara
     const int nzc = z1 - z0;
     const SmemLayout L = smem_layout(tile_x, 0, 0, 0);
     Pipe P;
-    pipe_setup(P, smem, L, p, !REUSE, tile_x, y0, x0, z0, nzc);
+    pipe_setup(P, smem, L, tile_x, y0, x0, z0, nzc);
+    if (!REUSE) pipe_hooks(P, p.wait_ns, p.hold_plane);
     if (tid == 0) {
         pipe_init(P);
         pipe_start(P, tm);
@@ -1130,7 +1131,9 @@ __device__ __forceinline__ void pml_quad_fast(
 // the end, return value uniform over the CTA; false = a wait timed out).
 // AR: kArithRef (the reference CPU operators' roundings, qp3d_exact.h) or
 // kArithFast (folded coefficients, fused multiply-adds, one reciprocal in S).
-template <bool SPEC, bool REUSE, bool HALF = false, int AR = kArithFast>
+// DEC: the step's threshold decisions are kept or replayed (p.dec_out,
+// p.dec_in) where asked for.
+template <bool SPEC, bool REUSE, bool HALF, int AR, bool DEC>
 __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams &p,
                                           const Coefs &k, int tile_x, int y0, int x0, int z0,
                                           int z1, bool win_writer, const DeferSeg &seg,
@@ -1147,7 +1150,8 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
     const int q = tid & (kQuadsY - 1), r = tid / kQuadsY;
     const int nzc = z1 - z0;
     Pipe P;
-    pipe_setup(P, smem, L, p, !REUSE, tile_x, y0, x0, z0, nzc);
+    pipe_setup(P, smem, L, tile_x, y0, x0, z0, nzc);
+    if (!REUSE) pipe_hooks(P, p.wait_ns, p.hold_plane);
     const int nx = p.nx, ny = p.ny, nz = p.nz, pml = p.pml;
     const int x = x0 + r, yq = y0 + 4 * q;
     const bool row_ok = (r < tile_x) && (x < nx - kRadius);
@@ -1339,13 +1343,13 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
         unsigned pmlb = 0;   // bits of the quad's PML cells
         if (PML) pmlb = (fx >= 0 || fz >= 0 ? 15u : fyb) & okb;
         unsigned above = 0;
-        const bool bits = !SPEC && (p.dec_in || p.dec_out);   // decisions replayed or kept
+        const bool bits = DEC && (p.dec_in || p.dec_out);   // decisions replayed or kept
         if (bits || !__all_sync(0xffffffffu, !row_ok || max4(m2) <= T2lo)) {
             if (AR == kArithRef) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     if (m2[j] > T2lo) above |= 1u << j;
-                if (!SPEC && p.dec_in && row_ok) above = (p.dec_in[base >> 5] >> (4 * q)) & 15u;
+                if (DEC && !SPEC && p.dec_in && row_ok) above = (p.dec_in[base >> 5] >> (4 * q)) & 15u;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     if ((above & okb) >> j & 1u)
@@ -1369,7 +1373,7 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         if (m2[j] > T2lo) above |= 1u << j;
-                    if (!SPEC && p.dec_in && row_ok) above = (p.dec_in[base >> 5] >> (4 * q)) & 15u;
+                    if (DEC && !SPEC && p.dec_in && row_ok) above = (p.dec_in[base >> 5] >> (4 * q)) & 15u;
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         kS[j] = (above >> j) & 1u ? __fmul_rn(k1[j], S[j]) : k1[j];
@@ -1463,7 +1467,7 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
             *reinterpret_cast<float4 *>(p.u_out + base) = make_float4(out[0], out[1], out[2], out[3]);
         // the step's decisions, when asked for: one bit per cell, 32 y cells a
         // word (the 8 lanes of a row combine their 4 bits)
-        if (!SPEC && p.dec_out) {
+        if (DEC && p.dec_out) {
             unsigned w = (above & okb) << (4 * q);
             w |= __shfl_xor_sync(0xffffffffu, w, 1);
             w |= __shfl_xor_sync(0xffffffffu, w, 2);
@@ -1518,7 +1522,7 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
     return ok;
 }
 
-template <bool SPEC, bool HALF, int AR>
+template <bool SPEC, bool HALF, int AR, bool DEC = !SPEC>
 __global__ void __launch_bounds__(kStepThreads, 2)
     qp3d_step_kernel(const __grid_constant__ TileMaps tm, const PlaneParams p)
 {
@@ -1533,7 +1537,8 @@ __global__ void __launch_bounds__(kStepThreads, 2)
     }
     const unsigned id = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     const DeferSeg seg = {(size_t)id * p.dcap, p.dcap, p.dcount + id};
-    step_tile<SPEC, false, HALF, AR>(&tm, p, p.k, p.tile_x, y0, x0, z0, z1, id == 0, seg, smem);
+    step_tile<SPEC, false, HALF, AR, DEC>(&tm, p, p.k, p.tile_x, y0, x0, z0, z1, id == 0, seg,
+                                          smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -1626,6 +1631,7 @@ __device__ __forceinline__ void fix_cell(const PlaneParams &p, float Tf, size_t 
     }
     if (AR == kArithRef && !has_src) out = __fadd_rn(out, __fmul_rn(0.0f, p.wavelet));
     p.u_out[idx] = out;
+    if (p.dec_out) atomicAnd(p.dec_out + (idx >> 5), ~(1u << (idx & 31)));
     if (p.record && z == p.sz && x >= pml && x < nx - pml && y >= pml && y < ny - pml)
         p.record[(long long)(x - pml) * (ny - 2 * pml) + (y - pml)] = out;
 }
@@ -1711,8 +1717,9 @@ __global__ void __launch_bounds__(kStepThreads, 2)
         const int z0 = kRadius + bz * p.chunk_z;
         const int z1 = min(z0 + p.chunk_z, p.nz - kRadius);
         if (z0 >= z1) continue;
-        if (!step_tile<false, true, HALF, AR>(&tm, p, p.k, p.tile_x, by * kTileY,
-                                              kRadius + bx * p.tile_x, z0, z1, false, none, smem))
+        if (!step_tile<false, true, HALF, AR, true>(&tm, p, p.k, p.tile_x, by * kTileY,
+                                                    kRadius + bx * p.tile_x, z0, z1, false, none,
+                                                    smem))
             return;
     }
 }
@@ -1929,8 +1936,8 @@ __device__ __forceinline__ bool batch_item(const BatchArgs &b, int it, unsigned 
     }
     const bool first = w.y0 == 0 && w.x0 == kRadius && w.z0 == kRadius;
     const DeferSeg seg = {w.dbase, w.dcap, b.dcount + it};
-    return step_tile<KIND == 2, REUSE, false, AR>(tm, p, b.k, w.tile_x, w.y0, w.x0, w.z0, w.z1,
-                                                  first, seg, body);
+    return step_tile<KIND == 2, REUSE, false, AR, false>(tm, p, b.k, w.tile_x, w.y0, w.x0, w.z0,
+                                                         w.z1, first, seg, body);
 }
 
 // All items of a step, one per CTA, longest columns first.
@@ -2037,186 +2044,301 @@ __device__ __forceinline__ void row_window(const float *f, long long i, int y, i
     }
 }
 
-// Pass A, four consecutive y cells (a quad) per thread, block and warp
-// shapes as pass B.  The derivatives of u^k take the operation order of
-// quad_derivs; the streamed volumes move as 16-byte loads and stores.  Every
-// entry a quad writes that its cells leave unchanged is written as zero,
-// which it already is (padding, PML state at interior cells, u_prev and
-// gradient at PML cells).
-#define QP3D_ST4(ptr, v) *reinterpret_cast<float4 *>((ptr) + i) = make_float4(v[0], v[1], v[2], v[3])
-__global__ void __launch_bounds__(256, 2) qp3d_adj_a_kernel(const AdjParams a)
+// Derivatives of u^k for pass A, two cells at a time.  The second derivatives
+// keep the centre weight in one coefficient.
+__device__ __forceinline__ void adj_derivs(const Taps &T, const Coefs &k, float Ux[4], float Uy[4],
+                                           float Uz[4], float Uxx[4], float Uyy[4], float Uzz[4])
 {
-    const int q = threadIdx.x & 7, r = threadIdx.x >> 3;
-    const int y = blockIdx.x * 32 + 4 * q, x = blockIdx.y * 32 + r, z = blockIdx.z;
-    if (y >= a.ny || x >= a.nx) return;
-    const long long i = (long long)z * a.plane + (long long)x * a.ldy + y;
-    const int nx = a.nx, ny = a.ny, nz = a.nz, pml = a.pml;
-    const Coefs &k = a.k;
-    const float4 lu = ldg4_or0(a.Lu, i, true), lup = ldg4_or0(a.Lup, i, true);
-    float l[4] = {lu.x, lu.y, lu.z, lu.w}, nu[4] = {lup.x, lup.y, lup.z, lup.w};
-    if (a.resid && z == a.sz && x >= pml && x < nx - pml) {
+    const float *pc = T.pc;
+    float Y[20];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (y + j >= pml && y + j < ny - pml)
-                l[j] += a.resid[(long long)(x - pml) * a.hy + (y + j - pml)];
+    for (int b = 0; b < 5; ++b) {
+        const float4 v = lds4(pc - 8 + 4 * b);
+        Y[4 * b] = v.x; Y[4 * b + 1] = v.y; Y[4 * b + 2] = v.z; Y[4 * b + 3] = v.w;
     }
-    const bool row_upd = x >= kRadius && x < nx - kRadius && z >= kRadius && z < nz - kRadius;
-    const int fx = x < pml ? 0 : (x >= nx - pml ? 1 : -1);
-    const int fz = z < pml ? 4 : (z >= nz - pml ? 5 : -1);
-    const int lix = x < pml ? pml - x : x - nx + pml, liz = z < pml ? pml - z : z - nz + pml;
-    bool upd[4];
-    int f[4], li[4];
-    bool any_int = false, any_pml = false;
+    const float2 uc[2] = {f2(Y[8], Y[9]), f2(Y[10], Y[11])};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int yj = y + j;
-        upd[j] = row_upd && yj >= kRadius && yj < ny - kRadius;
-        const int fy = yj < pml ? 2 : (yj >= ny - pml ? 3 : -1);
-        cell_face(fx, lix, fy, yj < pml ? pml - yj : yj - ny + pml, fz, liz, f[j], li[j]);
-        any_int = any_int || (upd[j] && f[j] < 0);
-        any_pml = any_pml || (upd[j] && f[j] >= 0);
-        if (!upd[j]) nu[j] += l[j];   // a never-updated cell keeps its value
-    }
-    float c3[4] = {0.f, 0.f, 0.f, 0.f}, c4[4] = {0.f, 0.f, 0.f, 0.f}, c5[4] = {0.f, 0.f, 0.f, 0.f};
-    float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};
-    if (any_int || any_pml) {
-        // derivatives of u^k (all taps in range for updated cells)
-        float Ux[4], Uy[4], Uz[4], Uxx[4], Uyy[4], Uzz[4], u0[4];
-        {
-            float w[20];
-            row_window(a.u, i, y, a.ldy, w);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                u0[j] = w[8 + j];
-                float g = 0.0f, l2 = __fmul_rn(k.ky, u0[j]);
-#pragma unroll
-                for (int m = 0; m < kRadius; ++m) {
-                    const float pa = w[8 + j + m + 1], pb = w[8 + j - m - 1];
-                    const float d = __fsub_rn(pa, pb);
-                    g = (m == 0) ? __fmul_rn(k.cy[0], d) : fmaf(k.cy[m], d, g);
-                    l2 = fmaf(k.c2y[m], __fadd_rn(pa, pb), l2);
-                }
-                Uy[j] = g;
-                Uyy[j] = l2;
-                Ux[j] = Uz[j] = 0.0f;
-                Uxx[j] = __fmul_rn(k.kx, u0[j]);
-                Uzz[j] = __fmul_rn(k.kz, u0[j]);
-            }
-        }
+    for (int h = 0; h < 2; ++h) {
+        const int j0 = 2 * h, j1 = j0 + 1;
+        float2 g = f2(0.f, 0.f), l = __fmul2_rn(k.ky2, uc[h]);
 #pragma unroll
         for (int m = 0; m < kRadius; ++m) {
-            const long long dx = (long long)(m + 1) * a.ldy, dz = (long long)(m + 1) * a.plane;
-            const float4 xp = ldg4_or0(a.u, i + dx, true), xm = ldg4_or0(a.u, i - dx, true);
-            const float4 zp = ldg4_or0(a.u, i + dz, true), zm = ldg4_or0(a.u, i - dz, true);
+            const float2 a = f2(Y[8 + j0 + m + 1], Y[8 + j1 + m + 1]);
+            const float2 b = f2(Y[8 + j0 - m - 1], Y[8 + j1 - m - 1]);
+            const float2 d = sub2(a, b);
+            g = m == 0 ? __fmul2_rn(k.cy2[0], d) : __ffma2_rn(k.cy2[m], d, g);
+            l = __ffma2_rn(k.c2y2[m], __fadd2_rn(a, b), l);
+        }
+        Uy[j0] = g.x; Uy[j1] = g.y;
+        Uyy[j0] = l.x; Uyy[j1] = l.y;
+    }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float ddx = __fsub_rn(f4(xp, j), f4(xm, j));
-                const float ddz = __fsub_rn(f4(zp, j), f4(zm, j));
-                Ux[j] = (m == 0) ? __fmul_rn(k.cx[0], ddx) : fmaf(k.cx[m], ddx, Ux[j]);
-                Uz[j] = (m == 0) ? __fmul_rn(k.cz[0], ddz) : fmaf(k.cz[m], ddz, Uz[j]);
-                Uxx[j] = fmaf(k.c2x[m], __fadd_rn(f4(xp, j), f4(xm, j)), Uxx[j]);
-                Uzz[j] = fmaf(k.c2z[m], __fadd_rn(f4(zp, j), f4(zm, j)), Uzz[j]);
+    for (int ax = 0; ax < 2; ++ax) {   // x, then z
+        const float2 kc = ax ? k.kz2 : k.kx2;
+        float2 g[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
+        float2 l[2] = {__fmul2_rn(kc, uc[0]), __fmul2_rn(kc, uc[1])};
+#pragma unroll
+        for (int m = 0; m < kRadius; ++m) {
+            const float4 a = ax ? ztap(T, kRadius + m + 1) : lds4(pc + (m + 1) * kBoxY);
+            const float4 b = ax ? ztap(T, kRadius - m - 1) : lds4(pc - (m + 1) * kBoxY);
+            const float2 c1 = ax ? k.cz2[m] : k.cx2[m], c2 = ax ? k.c2z2[m] : k.c2x2[m];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 d = sub2(half2of(a, h), half2of(b, h));
+                g[h] = m == 0 ? __fmul2_rn(c1, d) : __ffma2_rn(c1, d, g[h]);
+                l[h] = __ffma2_rn(c2, __fadd2_rn(half2of(a, h), half2of(b, h)), l[h]);
             }
         }
+        float *U = ax ? Uz : Ux, *UU = ax ? Uzz : Uxx;
+        U[0] = g[0].x; U[1] = g[0].y; U[2] = g[1].x; U[3] = g[1].y;
+        UU[0] = l[0].x; UU[1] = l[0].y; UU[2] = l[1].x; UU[3] = l[1].y;
+    }
+}
+
+// Pass A, marching along z as the step kernels do: u^k staged by TMA, the
+// cell's own values copied one plane ahead by cp.async, four consecutive y
+// cells (a quad) per thread, a loop body of its own for the warps with cells
+// of the shell.  Bound by HBM: 72 bytes a cell of the interior.  (One thread
+// per quad that gathered its 31 taps through L1 held 128 registers with
+// spills, and waited for three dependent groups of loads: 258 us on
+// 240x240x190, 50% of the DRAM peak; this form 199 us with the 80 bytes of
+// storing u_prev's adjoint and Cyy as well.)  Only updated cells are written: the
+// adjoint of the never-updated band reaches no other cell and no output.
+constexpr int kAdjStreams = 15;
+constexpr int kAdjThreads = kQuadsY * kAdjTileX;
+
+#define QP3D_ST4(ptr, v) *reinterpret_cast<float4 *>((ptr) + base) = make_float4(v[0], v[1], v[2], v[3])
+__global__ void __launch_bounds__(kAdjThreads, 2)
+    qp3d_adj_a_kernel(const __grid_constant__ TileMaps tm, const AdjParams a)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    pdl_trigger();
+    const int tile_x = a.tile_x;
+    const int y0 = blockIdx.x * kTileY, x0 = kRadius + blockIdx.y * tile_x;
+    const int z0 = kRadius + blockIdx.z * a.chunk_z, z1 = min(z0 + a.chunk_z, a.nz - kRadius);
+    if (z0 >= z1) {
+        pdl_wait();
+        return;
+    }
+    const int tid = threadIdx.x;
+    const int q = tid & (kQuadsY - 1), r = tid / kQuadsY;
+    const int nzc = z1 - z0, nx = a.nx, ny = a.ny, nz = a.nz, pml = a.pml;
+    const SmemLayout L = smem_layout(tile_x, pml, 0, kAdjStreams);
+    float4 *tab = reinterpret_cast<float4 *>(smem + L.tab_off);
+    Pipe P;
+    pipe_setup(P, smem, L, tile_x, y0, x0, z0, nzc);
+    pipe_hooks(P, a.wait_ns, 0);
+    const int x = x0 + r, yq = y0 + 4 * q;
+    const bool row_ok = r < tile_x && x < nx - kRadius;
+    unsigned okb = 0, fyb = 0;   // bits per cell: updated; of a y face
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int y = yq + j;
+        if (row_ok && y >= kRadius && y < ny - kRadius) okb |= 1u << j;
+        if (y < pml || y >= ny - pml) fyb |= 1u << j;
+    }
+    const bool mem_ok = okb != 0, y_inner = yq >= pml && yq + 3 < ny - pml;
+    const int fx = x < pml ? 0 : (x >= nx - pml ? 1 : -1);
+    const int lix = x < pml ? pml - x : x - nx + pml;
+    const bool xy_face = row_ok && (fx >= 0 || (fyb & okb));
+    const bool xy_face_warp = __any_sync(0xffffffffu, xy_face);
+    auto face_of_z = [&](int z) { return z < pml ? 4 : (z >= nz - pml ? 5 : -1); };
+    float4 *own = reinterpret_cast<float4 *>(smem + L.own_off) + tid;
+    const int nthr = blockDim.x;
+    unsigned base = (unsigned)((long long)z0 * a.plane + (long long)x * a.ldy + yq);
+    const unsigned plane = (unsigned)a.plane;
+    auto prefetch_params = [&](unsigned b) {
+        if (!mem_ok) return;
+        cp_async16(own + 2 * nthr, a.VP + b);
+        cp_async16(own + 3 * nthr, a.E2 + b);
+        cp_async16(own + 4 * nthr, a.R8 + b);
+    };
+    auto prefetch = [&](unsigned b, int z) {
+        if (!mem_ok) return;
+        cp_async16(own, a.Lu + b);
+        cp_async16(own + nthr, a.Lprev + b);
+        const bool z_face = face_of_z(z) >= 0;
+        if (!(fx >= 0 || z_face || (fyb & okb) == okb)) {   // a cell of the interior
+            cp_async16(own + 5 * nthr, a.gK + b);
+            cp_async16(own + 6 * nthr, a.gE + b);
+            cp_async16(own + 7 * nthr, a.gD + b);
+        }
+        if (xy_face || z_face) {
+            cp_async16(own + 8 * nthr, a.Lw1 + b);
+            cp_async16(own + 9 * nthr, a.Lw21 + b);
+            cp_async16(own + 10 * nthr, a.Lw3 + b);
+            cp_async16(own + 11 * nthr, a.Lp + b);
+            cp_async16(own + 12 * nthr, a.Lw1o + b);
+            cp_async16(own + 13 * nthr, a.Lpo + b);
+            cp_async16(own + 14 * nthr, a.Lw3o + b);
+        }
+    };
+    prefetch_params(base);
+    if (tid == 0) pipe_init(P);
+    for (int i = tid; i < 3 * pml; i += blockDim.x) tab[i] = fast_layer(a.layers[i]);
+    pdl_wait();
+    if (tid == 0) pipe_start(P, &tm);
+    prefetch(base, z0);
+    const float T2 = *a.T2;
+    __syncthreads();
+    const Coefs &k = a.k;
+    Taps T = taps_start(P, r, q);
+    bool ok = true;
+    auto plane_adj = [&](int t, auto shell) {
+        constexpr bool PML = decltype(shell)::value;
+        const int z = z0 + t;
+        const int fz = PML ? face_of_z(z) : -1;
+        cp_async_wait();
+        const float4 lu = own[0], lq = own[nthr], Vv = own[2 * nthr], Ev = own[3 * nthr],
+                     Rv = own[4 * nthr], vK = own[5 * nthr], vE = own[6 * nthr],
+                     vD = own[7 * nthr];
+        float4 vw1, vw21, vw3, vp, vw1o, vpo, vw3o;
+        const bool pml_quad = PML && (xy_face || (row_ok && fz >= 0));
+        if (pml_quad) {
+            vw1 = own[8 * nthr]; vw21 = own[9 * nthr]; vw3 = own[10 * nthr]; vp = own[11 * nthr];
+            vw1o = own[12 * nthr]; vpo = own[13 * nthr]; vw3o = own[14 * nthr];
+        }
+        if (t + 1 < nzc) {
+            prefetch(base + plane, z + 1);
+            prefetch_params(base + plane);
+        }
+        ok = __all_sync(0xffffffffu, pipe_wait(P, t));
+        if (!ok) return;
+        float Ux[4], Uy[4], Uz[4], Uxx[4], Uyy[4], Uzz[4];
+        adj_derivs(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz);
+        // the adjoint of u, and that of the step after: the residual is added
+        // at the receivers
+        float l[4] = {lu.x, lu.y, lu.z, lu.w}, lp[4] = {lq.x, lq.y, lq.z, lq.w};
+        if (z == a.sz && row_ok && x >= pml && x < nx - pml) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (yq + j >= pml && yq + j < ny - pml) {
+                    const long long i = (long long)(x - pml) * a.hy + (yq + j - pml);
+                    l[j] += a.resid[i];
+                    if (a.resid_prev) lp[j] += a.resid_prev[i];
+                }
+        }
+        float nu[4] = {0.f, 0.f, 0.f, 0.f};
         // frozen scalar operator and its eps / delta derivatives
-        const float4 Vv = ldg4_or0(a.VP, i, true), Ev = ldg4_or0(a.E2, i, true),
-                     Rv = ldg4_or0(a.R8, i, true);
         const float4 Kv = make_float4(k_of_vp(Vv.x, a.dt), k_of_vp(Vv.y, a.dt),
                                       k_of_vp(Vv.z, a.dt), k_of_vp(Vv.w, a.dt));
-        const float T2 = *a.T2;
         // wa: with the live operator, dS/da times 2 / m2, so that the
         // derivatives of S in Ux, Uy, Uz are wa (Ux (1 - a), Uy (1 - a), -Uz a)
         // (a = h2 / m2 = nx^2 + ny^2, h2 = Ux^2 + Uy^2, m2 = h2 + Uz^2; no
         // power of m2 above the first, which could leave the float range)
-        float KS[4], e2[4], S[4], dSe[4], dSd[4], wa[4], av[4];
+        float KS[4], e2[4], S[4], dSe[4], dSd[4], wa[4], av[4], m2[4], h2[4];
+        unsigned on = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float E2 = f4(Ev, j), R8 = f4(Rv, j);
-            e2[j] = 1.0f + E2;
-            const float h2 = fmaf(Uy[j], Uy[j], Ux[j] * Ux[j]), m2 = fmaf(Uz[j], Uz[j], h2);
+            h2[j] = fmaf(Uy[j], Uy[j], Ux[j] * Ux[j]);
+            m2[j] = fmaf(Uz[j], Uz[j], h2[j]);
+            if (m2[j] > T2) on |= 1u << j;
             S[j] = 1.0f;
             dSe[j] = dSd[j] = wa[j] = av[j] = 0.0f;
-            const bool on = a.dec ? ((a.dec[i >> 5] >> ((unsigned)(i & 31) + j)) & 1u) != 0
-                                  : (m2 > T2);
-            if (on) {
-                const float aa = __fdividef(h2, m2), bb = 1.0f - aa, D = fmaf(E2, aa, 1.0f);
+            e2[j] = 1.0f + f4(Ev, j);
+        }
+        if (a.dec && row_ok) on = (a.dec[base >> 5] >> (4 * q)) & 15u;
+        if (__any_sync(0xffffffffu, on & okb)) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float E2 = f4(Ev, j), R8 = f4(Rv, j);
+                const float aa = __fdividef(h2[j], m2[j]), bb = 1.0f - aa, D = fmaf(E2, aa, 1.0f);
                 const float iD = __fdividef(1.0f, D);
                 const float ab8 = 8.0f * aa * bb * iD * iD;
                 const float qq = 0.125f * R8 * ab8;
                 const float rr = sqrtf(fmaxf(1.0f - qq, 0.0f));
-                S[j] = 0.5f + 0.5f * rr;
                 const float dSdq = rr > 0.0f ? __fdividef(-0.25f, rr) : 0.0f;
-                dSe[j] = dSdq * ab8 * (1.0f - 0.5f * aa * R8 * iD);
-                dSd[j] = -dSdq * ab8;
-                if (a.live) {   // dq/da = R8 ((1 - 2a) D - 2 E2 a (1 - a)) / D^3
-                    const float dqda = R8 * ((1.0f - 2.0f * aa) * D - 2.0f * E2 * aa * bb) * iD * iD * iD;
-                    wa[j] = __fdividef(2.0f * dSdq * dqda, m2);
-                    av[j] = aa;
+                // dq/da = R8 ((1 - 2a) D - 2 E2 a (1 - a)) / D^3
+                const float dqda = R8 * ((1.0f - 2.0f * aa) * D - 2.0f * E2 * aa * bb) * iD * iD * iD;
+                if (on >> j & 1u) {
+                    S[j] = 0.5f + 0.5f * rr;
+                    dSe[j] = dSdq * ab8 * (1.0f - 0.5f * aa * R8 * iD);
+                    dSd[j] = -dSdq * ab8;
+                    if (a.live) {
+                        wa[j] = __fdividef(2.0f * dSdq * dqda, m2[j]);
+                        av[j] = aa;
+                    }
                 }
             }
-            KS[j] = f4(Kv, j) * S[j];
         }
-        if (any_int) {   // interior leapfrog and the gradient sums
-            const float4 vK = ldg4_or0(a.gK, i, true), vE = ldg4_or0(a.gE, i, true),
-                         vD = ldg4_or0(a.gD, i, true);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) KS[j] = f4(Kv, j) * S[j];
+        float c0[4], c1[4], c2[4], c3[4], c4[4], c5[4];
+        const unsigned pmlb = PML ? (fx >= 0 || fz >= 0 ? 15u : fyb) & okb : 0u;
+        const unsigned intb = okb & ~pmlb;
+        if (PML) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) c0[j] = c1[j] = c2[j] = c3[j] = c4[j] = c5[j] = 0.0f;
+        }
+        if (!PML || intb) {   // interior leapfrog and the gradient sums
             float gK[4] = {vK.x, vK.y, vK.z, vK.w}, gE[4] = {vE.x, vE.y, vE.z, vE.w},
-                  gD[4] = {vD.x, vD.y, vD.z, vD.w}, nup[4] = {0.f, 0.f, 0.f, 0.f};
+                  gD[4] = {vD.x, vD.y, vD.z, vD.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                if (!(upd[j] && f[j] < 0)) continue;
-                nu[j] += 2.0f * l[j];
-                nup[j] = -l[j];
-                c3[j] = KS[j] * e2[j] * l[j];
-                c4[j] = c3[j];
-                c5[j] = KS[j] * l[j];
+                const bool in = (intb >> j) & 1u;
+                // u_prev's adjoint is -l of the step after (0 in the shell)
+                const float n2 = -lp[j] + 2.0f * l[j];
+                const float cc = KS[j] * e2[j] * l[j];
                 const float Lh = Uxx[j] + Uyy[j], Lap = fmaf(e2[j], Lh, Uzz[j]);
                 const float Kc = f4(Kv, j);
-                gK[j] += l[j] * S[j] * Lap;
-                gE[j] += l[j] * Kc * (2.0f * S[j] * Lh + dSe[j] * Lap);
-                gD[j] += l[j] * Kc * dSd[j] * Lap;
+                const float aK = gK[j] + l[j] * S[j] * Lap;
+                const float aE = gE[j] + l[j] * Kc * (2.0f * S[j] * Lh + dSe[j] * Lap);
+                const float aD = gD[j] + l[j] * Kc * dSd[j] * Lap;
                 // live operator: S's dependence on grad u, through the
                 // transposed first derivatives (zero where S = 1)
                 const float w = l[j] * Kc * Lap * wa[j], bv = 1.0f - av[j];
-                c0[j] = w * Ux[j] * bv;
-                c1[j] = w * Uy[j] * bv;
-                c2[j] = -w * Uz[j] * av[j];
+                if (in) {
+                    nu[j] = n2;
+                    c3[j] = c4[j] = cc;
+                    c5[j] = KS[j] * l[j];
+                    gK[j] = aK; gE[j] = aE; gD[j] = aD;
+                    c0[j] = w * Ux[j] * bv;
+                    c1[j] = w * Uy[j] * bv;
+                    c2[j] = -w * Uz[j] * av[j];
+                } else if (!PML) {
+                    gK[j] = gE[j] = gD[j] = 0.0f;
+                    c0[j] = c1[j] = c2[j] = c3[j] = c4[j] = c5[j] = 0.0f;
+                }
             }
-            QP3D_ST4(a.gK, gK); QP3D_ST4(a.gE, gE); QP3D_ST4(a.gD, gD); QP3D_ST4(a.Nup, nup);
+            if (mem_ok) {
+                QP3D_ST4(a.gK, gK); QP3D_ST4(a.gE, gE); QP3D_ST4(a.gD, gD);
+            }
         }
-        if (any_pml) {   // transposed split-field recursions
-            const float4 vw1 = ldg4_or0(a.Lw1, i, true), vw21 = ldg4_or0(a.Lw21, i, true),
-                         vw3 = ldg4_or0(a.Lw3, i, true), vp = ldg4_or0(a.Lp, i, true),
-                         vw1o = ldg4_or0(a.Lw1o, i, true), vpo = ldg4_or0(a.Lpo, i, true),
-                         vw3o = ldg4_or0(a.Lw3o, i, true);
+        if (PML && pml_quad) {   // transposed split-field recursions
             float nw1[4], nw1o[4], np_[4], npo[4], nw21[4], nw3[4], nw3o[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 nw1[j] = nw1o[j] = np_[j] = npo[j] = nw21[j] = nw3[j] = nw3o[j] = 0.0f;
-                if (!(upd[j] && f[j] >= 0)) continue;
-                const float4 lc = fast_layer(a.layers[(f[j] >> 1) * pml + li[j]]);
-                const bool isz = f[j] >= 4;
+                if (!((pmlb >> j) & 1u)) continue;
+                int f, li;
+                const int y = yq + j;
+                const int fy = y < pml ? 2 : (y >= ny - pml ? 3 : -1);
+                cell_face(fx, lix, fy, y < pml ? pml - y : y - ny + pml, fz,
+                          z < pml ? pml - z : z - nz + pml, f, li);
+                const float4 lc = tab[(f >> 1) * pml + li];
+                const bool isz = f >= 4;
                 const float A = isz ? KS[j] : e2[j] * KS[j], Bt = isz ? e2[j] * KS[j] : KS[j];
-                const float sgn = (f[j] & 1) ? -1.0f : 1.0f;
+                const float sgn = (f & 1) ? -1.0f : 1.0f;
                 const float W1 = f4(vw1, j) + l[j], W21 = f4(vw21, j) + l[j], W3 = f4(vw3, j) + l[j];
-                const float P = fmaf(a.dt, W21, f4(vp, j));
+                const float Pp = fmaf(a.dt, W21, f4(vp, j));
                 nw1[j] = fmaf(-lc.x, W1, f4(vw1o, j));
                 nw1o[j] = lc.y * W1;
-                np_[j] = fmaf(-lc.x, P, f4(vpo, j));
-                npo[j] = lc.y * P;
+                np_[j] = fmaf(-lc.x, Pp, f4(vpo, j));
+                npo[j] = lc.y * Pp;
                 nw21[j] = lc.z * W21;
                 nw3[j] = fmaf(2.0f, W3, f4(vw3o, j));
                 nw3o[j] = -W3;
-                const float cn = A * W1, cf = sgn * A * lc.w * P, ct = Bt * W3;
-                if (f[j] < 2) { c3[j] = cn; c0[j] = cf; c4[j] = ct * e2[j]; c5[j] = ct; }
-                else if (f[j] < 4) { c4[j] = cn; c1[j] = cf; c3[j] = ct * e2[j]; c5[j] = ct; }
+                const float cn = A * W1, cf = sgn * A * lc.w * Pp, ct = Bt * W3;
+                if (f < 2) { c3[j] = cn; c0[j] = cf; c4[j] = ct * e2[j]; c5[j] = ct; }
+                else if (f < 4) { c4[j] = cn; c1[j] = cf; c3[j] = ct * e2[j]; c5[j] = ct; }
                 else { c5[j] = cn; c2[j] = cf; c3[j] = ct; c4[j] = ct; }
                 if (a.live && wa[j] != 0.0f) {
                     // the S-proportional terms of w1', p' and w3' (their
                     // weights cn, cf, ct over S) times dS/d(grad u)
-                    const float Unn = f[j] < 2 ? Uxx[j] : (isz ? Uzz[j] : Uyy[j]);
-                    const float Un = f[j] < 2 ? Ux[j] : (isz ? Uz[j] : Uy[j]);
+                    const float Unn = f < 2 ? Uxx[j] : (isz ? Uzz[j] : Uyy[j]);
+                    const float Un = f < 2 ? Ux[j] : (isz ? Uz[j] : Uy[j]);
                     const float tang = isz ? Uxx[j] + Uyy[j]
-                                           : fmaf(e2[j], f[j] < 2 ? Uyy[j] : Uxx[j], Uzz[j]);
+                                           : fmaf(e2[j], f < 2 ? Uyy[j] : Uxx[j], Uzz[j]);
                     const float w = __fdividef(cn * Unn + cf * Un + ct * tang, S[j]) * wa[j];
                     const float bv = 1.0f - av[j];
                     c0[j] += w * Ux[j] * bv;
@@ -2224,119 +2346,121 @@ __global__ void __launch_bounds__(256, 2) qp3d_adj_a_kernel(const AdjParams a)
                     c2[j] -= w * Uz[j] * av[j];
                 }
             }
-            QP3D_ST4(a.Nw1, nw1); QP3D_ST4(a.Nw1o, nw1o); QP3D_ST4(a.Np, np_);
-            QP3D_ST4(a.Npo, npo); QP3D_ST4(a.Nw21, nw21); QP3D_ST4(a.Nw3, nw3);
-            QP3D_ST4(a.Nw3o, nw3o);
+            if (mem_ok) {
+                QP3D_ST4(a.Nw1, nw1); QP3D_ST4(a.Nw1o, nw1o); QP3D_ST4(a.Np, np_);
+                QP3D_ST4(a.Npo, npo); QP3D_ST4(a.Nw21, nw21); QP3D_ST4(a.Nw3, nw3);
+                QP3D_ST4(a.Nw3o, nw3o);
+            }
         }
-        if (any_pml || a.live) {
-            QP3D_ST4(a.C[0], c0); QP3D_ST4(a.C[1], c1); QP3D_ST4(a.C[2], c2);
+        if (mem_ok) {
+            if (pml_quad || a.live) {
+                QP3D_ST4(a.C[0], c0); QP3D_ST4(a.C[1], c1); QP3D_ST4(a.C[2], c2);
+            }
+            QP3D_ST4(a.C[3], c3); QP3D_ST4(a.C[5], c5);
+            // Cyy equals Cxx at cells of the interior: pass B takes it from there
+            // for quads that hold nothing else
+            if (!y_inner || (PML && pml_quad)) QP3D_ST4(a.C[4], c4);
+            QP3D_ST4(a.Nu, nu);
         }
-        QP3D_ST4(a.C[3], c3); QP3D_ST4(a.C[4], c4); QP3D_ST4(a.C[5], c5);
+        pipe_release(P, &tm, t);
+    };
+    for (int t = 0; t < nzc && ok; taps_next(T, P, t), ++t, base += plane) {
+        if (xy_face_warp || face_of_z(z0 + t) >= 0) plane_adj(t, std::true_type());
+        else plane_adj(t, std::false_type());
     }
-    QP3D_ST4(a.Nu, nu);
+    cp_async_wait();
+    pipe_finish(P, ok, a.err);
+}
 #undef QP3D_ST4
+
+// Pass B: Nu += the transposed stencils of the six coefficient fields, over
+// the updated cells (their taps lie inside the volume; along y the rows are
+// padded to whole quads, and taps before a row's start or past its end read
+// zero).  Bound by the bytes through L1.
+//
+__device__ __forceinline__ void fma4(float acc[4], float c, const float4 &a, const float4 &b, bool minus)
+{
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        acc[j] = fmaf(c, minus ? f4(a, j) - f4(b, j) : f4(a, j) + f4(b, j), acc[j]);
 }
 
-// Pass B: Nu += the transposed stencils of the six coefficient fields, four
-// consecutive y cells (a quad) per thread with 16-byte loads; a block is 8
-// quads (32 y) x 32 rows, a warp 8 quads x 4 rows.  Taps outside the volume
-// read zero (the coefficient fields are zero in the row padding).  Outside
-// the PML shell the first-derivative fields Cx, Cy, Cz are zero and Cyy
-// equals Cxx (qp3d_adj_a_kernel), so a warp whose whole footprint (its cells
-// and 5 around them) lies inside reads two fields.
+// A thread takes one quad.  With the frozen operator, a warp whose whole
+// footprint (its cells and 5 around them) lies outside the shell, where Cx, Cy,
+// Cz are zero and Cyy equals Cxx (qp3d_adj_a_kernel), reads two fields.
+// Two rows by two planes of quads per thread, which needs 34 16-byte loads a
+// quad instead of 53, left 16 warps an SM and took 111 us instead of 105 on
+// 240x240x190: the pass waits for latency rather than for the bytes.
 __global__ void __launch_bounds__(256) qp3d_adj_b_kernel(const AdjParams a)
 {
+    pdl_trigger();
+    pdl_wait();
     const int q = threadIdx.x & 7, r = threadIdx.x >> 3;
-    const int y = blockIdx.x * 32 + 4 * q, x = blockIdx.y * 32 + r, z = blockIdx.z;
-    if (y >= a.ny || x >= a.nx) return;
+    const int y = blockIdx.x * 32 + 4 * q, x = blockIdx.y * 32 + r;
+    const int z = kRadius + blockIdx.z;
+    if (y + 3 < kRadius || y >= a.ny - kRadius || x < kRadius || x >= a.nx - kRadius) return;
     const int xw = blockIdx.y * 32 + ((threadIdx.x >> 5) << 2), yw = blockIdx.x * 32;
     const long long i = (long long)z * a.plane + (long long)x * a.ldy + y;
     const Coefs &k = a.k;
     // the quad's Nu, read-modified-written at the end, moves to shared memory
     // while the taps are gathered (7% of the pass on a 240x240x190 grid)
     __shared__ __align__(16) float4 pnu[256];
-    const bool vec_nu = y + 3 < a.ny;
-    if (vec_nu) {
-        cp_async16(&pnu[threadIdx.x], a.Nu + i);
-    }
+    cp_async16(&pnu[threadIdx.x], a.Nu + i);
     const bool inside = !a.live && xw - kRadius >= a.pml && xw + 4 + kRadius <= a.nx - a.pml &&
                         yw - kRadius >= a.pml && yw + 32 + kRadius <= a.ny - a.pml &&
                         z - kRadius >= a.pml && z + kRadius < a.nz - a.pml;
     float acc[4];
-    if (inside) {
-        const float *H = a.C[3], *V = a.C[5];
-        float w[20];
-        row_window(H, i, y, a.ldy, w);
-        const float4 v0 = ldg4_or0(V, i, true);
+    const float *Cx = a.C[0], *Cy = a.C[1], *Cz = a.C[2], *Cxx = a.C[3], *Cyy = a.C[4],
+                *Czz = a.C[5];
+    float w[20];
+    // Cyy, of quads wholly in the interior kept in Cxx only
+    const bool row_in = x >= a.pml && x < a.nx - a.pml && z >= a.pml && z < a.nz - a.pml;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] = k.kx * w[8 + j] + k.ky * w[8 + j] + k.kz * f4(v0, j);
+    for (int b = 0; b < 5; ++b) {
+        const int yb = y - 8 + 4 * b;
+        const bool in = row_in && yb >= a.pml && yb + 3 < a.ny - a.pml;
+        const float4 v = ldg4_or0(in ? Cxx : Cyy, i - 8 + 4 * b, yb >= 0 && yb < a.ldy);
+        w[4 * b] = v.x; w[4 * b + 1] = v.y; w[4 * b + 2] = v.z; w[4 * b + 3] = v.w;
+    }
+    const float4 xx0 = ldg4_or0(Cxx, i, true), zz0 = ldg4_or0(Czz, i, true);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j] = k.kx * f4(xx0, j) + k.ky * w[8 + j] + k.kz * f4(zz0, j);
+    if (inside) {
 #pragma unroll
         for (int m = 0; m < kRadius; ++m) {
             const int d = m + 1;
             const long long dx = (long long)d * a.ldy, dz = (long long)d * a.plane;
-            const float4 hp = ldg4_or0(H, i + dx, true), hm = ldg4_or0(H, i - dx, true);
-            const float4 vp = ldg4_or0(V, i + dz, true), vm = ldg4_or0(V, i - dz, true);
+            fma4(acc, k.c2x[m], ldg4_or0(Cxx, i + dx, true), ldg4_or0(Cxx, i - dx, true), false);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                acc[j] = fmaf(k.c2x[m], f4(hp, j) + f4(hm, j), acc[j]);
-                acc[j] = fmaf(k.c2y[m], w[8 + j + d] + w[8 + j - d], acc[j]);
-                acc[j] = fmaf(k.c2z[m], f4(vp, j) + f4(vm, j), acc[j]);
-            }
+            for (int j = 0; j < 4; ++j) acc[j] = fmaf(k.c2y[m], w[8 + j + d] + w[8 + j - d], acc[j]);
+            fma4(acc, k.c2z[m], ldg4_or0(Czz, i + dz, true), ldg4_or0(Czz, i - dz, true), false);
         }
     } else {
-        const float *Cx = a.C[0], *Cy = a.C[1], *Cz = a.C[2], *Cxx = a.C[3], *Cyy = a.C[4],
-                    *Czz = a.C[5];
-        {
-            float wyy[20];
-            row_window(Cyy, i, y, a.ldy, wyy);
-            const float4 xx0 = ldg4_or0(Cxx, i, true), zz0 = ldg4_or0(Czz, i, true);
+#pragma unroll
+        for (int m = 0; m < kRadius; ++m)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                acc[j] = k.kx * f4(xx0, j) + k.ky * wyy[8 + j] + k.kz * f4(zz0, j);
+                acc[j] = fmaf(k.c2y[m], w[8 + j + m + 1] + w[8 + j - m - 1], acc[j]);
+        row_window(Cy, i, y, a.ldy, w);
 #pragma unroll
-            for (int m = 0; m < kRadius; ++m)
+        for (int m = 0; m < kRadius; ++m)
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[j] = fmaf(k.c2y[m], wyy[8 + j + m + 1] + wyy[8 + j - m - 1], acc[j]);
-        }
-        {
-            float wy[20];
-            row_window(Cy, i, y, a.ldy, wy);
-#pragma unroll
-            for (int m = 0; m < kRadius; ++m)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[j] = fmaf(k.cy[m], wy[8 + j - m - 1] - wy[8 + j + m + 1], acc[j]);
-        }
+            for (int j = 0; j < 4; ++j)
+                acc[j] = fmaf(k.cy[m], w[8 + j - m - 1] - w[8 + j + m + 1], acc[j]);
 #pragma unroll
         for (int m = 0; m < kRadius; ++m) {
             const int d = m + 1;
             const long long dx = (long long)d * a.ldy, dz = (long long)d * a.plane;
-            const bool xp = x + d < a.nx, xm = x - d >= 0, zp = z + d < a.nz, zm = z - d >= 0;
-            const float4 xxp = ldg4_or0(Cxx, i + dx, xp), xxm = ldg4_or0(Cxx, i - dx, xm);
-            const float4 x1p = ldg4_or0(Cx, i + dx, xp), x1m = ldg4_or0(Cx, i - dx, xm);
-            const float4 zzp = ldg4_or0(Czz, i + dz, zp), zzm = ldg4_or0(Czz, i - dz, zm);
-            const float4 z1p = ldg4_or0(Cz, i + dz, zp), z1m = ldg4_or0(Cz, i - dz, zm);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                acc[j] = fmaf(k.c2x[m], f4(xxp, j) + f4(xxm, j), acc[j]);
-                acc[j] = fmaf(k.c2z[m], f4(zzp, j) + f4(zzm, j), acc[j]);
-                acc[j] = fmaf(k.cx[m], f4(x1m, j) - f4(x1p, j), acc[j]);
-                acc[j] = fmaf(k.cz[m], f4(z1m, j) - f4(z1p, j), acc[j]);
-            }
+            fma4(acc, k.c2x[m], ldg4_or0(Cxx, i + dx, true), ldg4_or0(Cxx, i - dx, true), false);
+            fma4(acc, k.c2z[m], ldg4_or0(Czz, i + dz, true), ldg4_or0(Czz, i - dz, true), false);
+            fma4(acc, k.cx[m], ldg4_or0(Cx, i - dx, true), ldg4_or0(Cx, i + dx, true), true);
+            fma4(acc, k.cz[m], ldg4_or0(Cz, i - dz, true), ldg4_or0(Cz, i + dz, true), true);
         }
     }
-    float *nu = a.Nu + i;
-    if (vec_nu) {
-        cp_async_wait();
-        float4 v = pnu[threadIdx.x];
-        v.x += acc[0]; v.y += acc[1]; v.z += acc[2]; v.w += acc[3];
-        *reinterpret_cast<float4 *>(nu) = v;
-    } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (y + j < a.ny) nu[j] += acc[j];
-    }
+    cp_async_wait();
+    float4 v = pnu[threadIdx.x];
+    v.x += acc[0]; v.y += acc[1]; v.z += acc[2]; v.w += acc[3];
+    *reinterpret_cast<float4 *>(a.Nu + i) = v;
 }
 
 __global__ void qp3d_threshold_kernel(const float *gmax, float *T2, int n)
@@ -2420,11 +2544,13 @@ cudaError_t configure_kernels()
         (e = set_smem(qp3d_batch_plane_kernel<1, kArithRef>, bytes)) ||
         (e = set_smem(qp3d_batch_plane_kernel<2, kArithRef>, bytes)) ||
         (e = set_smem(qp3d_batch_resolve_kernel<kArithFast>, bytes)) ||
+        (e = set_smem(qp3d_adj_a_kernel, bytes)) ||
         (e = set_smem(qp3d_batch_resolve_kernel<kArithRef>, bytes)))
         return e;
 #define QP3D_STEP_SMEM(AR)                                                                   \
     if ((e = set_smem(qp3d_step_kernel<true, false, AR>, bytes)) ||                         \
         (e = set_smem(qp3d_step_kernel<false, false, AR>, bytes)) ||                        \
+        (e = set_smem(qp3d_step_kernel<true, false, AR, true>, bytes)) ||                   \
         (e = set_smem(qp3d_step_kernel<true, true, AR>, bytes)) ||                          \
         (e = set_smem(qp3d_step_kernel<false, true, AR>, bytes)) ||                         \
         (e = set_smem(qp3d_gradmax_kernel<AR>, bytes)) ||                                   \
@@ -2452,9 +2578,10 @@ static cudaError_t launch_step_t(const TileMaps &tm, const PlaneParams &p, dim3 
                                  size_t smem, cudaStream_t stream)
 {
     auto *fn = p.half_params ? (p.spec ? qp3d_step_kernel<true, true, AR>
-                                       : qp3d_step_kernel<false, true, AR>)
-                             : (p.spec ? qp3d_step_kernel<true, false, AR>
-                                       : qp3d_step_kernel<false, false, AR>);
+                                       : qp3d_step_kernel<false, true, AR>)   // no decisions kept
+               : !p.spec     ? qp3d_step_kernel<false, false, AR>
+               : p.dec_out   ? qp3d_step_kernel<true, false, AR, true>
+                             : qp3d_step_kernel<true, false, AR>;
     return launch_pdl(fn, grid, t, smem, stream, tm, p);
 }
 
@@ -2571,15 +2698,28 @@ cudaError_t launch_crop(const float *u, float *out, int x0, int x1, int y0, int 
     return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_step(const AdjParams &a, cudaStream_t stream)
+void plan_adjoint(AdjParams &a, int nsm)
 {
-    // one thread per quad of 4 y cells; a block is 8 quads x 32 rows
-    const dim3 grid((a.ny + 31) / 32, (a.nx + 31) / 32, a.nz);
-    qp3d_adj_a_kernel<<<grid, 256, 0, stream>>>(a);
-    cudaError_t e = cudaGetLastError();
+    const int ncx = a.nx - 2 * kRadius, ncz = a.nz - 2 * kRadius;
+    const int ntx = (ncx + kAdjTileX - 1) / kAdjTileX;
+    a.tile_x = (ncx + ntx - 1) / ntx;
+    const long long tiles = (long long)ntx * ((a.ny - kRadius - 1) / kTileY + 1);
+    const size_t smem = smem_layout(a.tile_x, a.pml, 0, kAdjStreams).total;
+    const int n = plan_chunks(tiles, ncz, std::max(192, plane_threads(a.tile_x)), smem, nsm);
+    a.chunk_z = (ncz + n - 1) / n;
+}
+
+cudaError_t launch_adjoint_step(const TileMaps &tm, const AdjParams &a, cudaStream_t stream)
+{
+    const int nyt = (a.ny - kRadius - 1) / kTileY + 1;
+    const int nxt = (a.nx - 2 * kRadius + a.tile_x - 1) / a.tile_x;
+    const int nch = (a.nz - 2 * kRadius + a.chunk_z - 1) / a.chunk_z;
+    cudaError_t e = launch_pdl(qp3d_adj_a_kernel, dim3(nyt, nxt, nch), plane_threads(a.tile_x),
+                               smem_layout(a.tile_x, a.pml, 0, kAdjStreams).total, stream, tm, a);
     if (e != cudaSuccess) return e;
-    qp3d_adj_b_kernel<<<grid, 256, 0, stream>>>(a);
-    return cudaGetLastError();
+    const int ncz = a.nz - 2 * kRadius;
+    return launch_pdl(qp3d_adj_b_kernel, dim3(nyt, (a.nx + 31) / 32, ncz), 256, 0,
+                      stream, a);
 }
 
 cudaError_t launch_threshold(const float *gmax, float *T2, int n, cudaStream_t stream)
