@@ -38,6 +38,8 @@ extern "C" const char *qp3d_strerror(int code)
 
 extern "C" const char *qp3d_ctx_last_error(const qp3d_ctx *ctx) { return ctx ? ctx->err : ""; }
 
+constexpr int kStateVols = 14;   // U, W1, W3, P: three levels each, W21 two
+
 static void free_defer(qp3d_ctx *ctx)
 {
     if (ctx->dkey) cudaFree(ctx->dkey);
@@ -52,32 +54,25 @@ static void free_defer(qp3d_ctx *ctx)
 static void free_shot(qp3d_ctx *ctx)
 {
     cudaSetDevice(ctx->device);
-    float **bufs[] = {&ctx->U[0],  &ctx->U[1],  &ctx->U[2],  &ctx->VP,     &ctx->E2,
-                      &ctx->R8,    &ctx->W1[0], &ctx->W1[1], &ctx->W1[2], &ctx->W3[0],
-                      &ctx->W3[1], &ctx->W3[2], &ctx->P[0],  &ctx->P[1],  &ctx->P[2],
-                      &ctx->W21[0], &ctx->W21[1], &ctx->record, &ctx->gmax, &ctx->snap_dev,
-                      &ctx->win,   &ctx->spec_err};
-    for (float **b : bufs) {
+    void **bufs[] = {(void **)&ctx->state, &ctx->params, (void **)&ctx->book,
+                     (void **)&ctx->record, (void **)&ctx->snap_dev, (void **)&ctx->spec_err,
+                     (void **)&ctx->layers, (void **)&ctx->src_fused, (void **)&ctx->src_band,
+                     (void **)&ctx->src_all};
+    for (void **b : bufs) {
         if (*b) cudaFree(*b);
         *b = nullptr;
     }
-    if (ctx->redo) cudaFree(ctx->redo);
-    if (ctx->alt_count) cudaFree(ctx->alt_count);
+    float **parts[] = {&ctx->U[0],  &ctx->U[1],  &ctx->U[2],  &ctx->VP,     &ctx->E2,
+                       &ctx->R8,    &ctx->W1[0], &ctx->W1[1], &ctx->W1[2], &ctx->W3[0],
+                       &ctx->W3[1], &ctx->W3[2], &ctx->P[0],  &ctx->P[1],  &ctx->P[2],
+                       &ctx->W21[0], &ctx->W21[1], &ctx->gmax, &ctx->win};
+    for (float **b : parts) *b = nullptr;
     ctx->redo = nullptr;
     ctx->alt_count = nullptr;
+    ctx->h_vp = ctx->h_eps = ctx->h_del = nullptr;
+    ctx->cap_fused = ctx->cap_band = ctx->cap_all = 0;
     free_defer(ctx);
-    __half **halves[] = {&ctx->h_vp, &ctx->h_eps, &ctx->h_del};
-    for (__half **h : halves) {
-        if (*h) cudaFree(*h);
-        *h = nullptr;
-    }
-    if (ctx->layers) cudaFree(ctx->layers);
-    if (ctx->src_fused) cudaFree(ctx->src_fused);
-    if (ctx->src_band) cudaFree(ctx->src_band);
-    if (ctx->src_all) cudaFree(ctx->src_all);
     if (ctx->snap_host) cudaFreeHost(ctx->snap_host);
-    ctx->layers = nullptr;
-    ctx->src_fused = ctx->src_band = ctx->src_all = nullptr;
     ctx->snap_host = nullptr;
     ctx->snap_cap = 0;
     ctx->loaded = false;
@@ -211,12 +206,6 @@ static int ensure_defer(qp3d_ctx *ctx)
     return QP3D_OK;
 }
 
-static int alloc_vol(qp3d_ctx *ctx, float **p)
-{
-    CK(cudaMalloc(p, (size_t)ctx->vol * sizeof(float)));
-    return QP3D_OK;
-}
-
 // Copy a dense [nz][nx][ny] host volume into the pitched device layout.
 static int upload_vol(qp3d_ctx *ctx, float *dst, const float *src)
 {
@@ -264,31 +253,40 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
     }
 
     if (!same) {
+        const size_t vol = (size_t)ctx->vol, ntb = (size_t)std::max(g->nt, 1);
         float **vols[] = {&ctx->U[0],  &ctx->U[1],  &ctx->U[2],  &ctx->W1[0], &ctx->W1[1],
                           &ctx->W1[2], &ctx->W3[0], &ctx->W3[1], &ctx->W3[2], &ctx->P[0],
-                          &ctx->P[1],  &ctx->P[2],  &ctx->W21[0], &ctx->W21[1],
-                          &ctx->VP,     &ctx->E2,    &ctx->R8};
-        const int nvols = half ? 14 : 17;   // half storage: no FP32 parameter volumes
-        for (int v = 0; v < nvols; ++v)
-            if ((rc = alloc_vol(ctx, vols[v]))) {
-                free_shot(ctx);
-                return rc;
-            }
-        if (half) {
-            __half **hs[] = {&ctx->h_vp, &ctx->h_eps, &ctx->h_del};
-            for (__half **h : hs) CK(cudaMalloc(h, (size_t)ctx->vol * sizeof(__half)));
+                          &ctx->P[1],  &ctx->P[2],  &ctx->W21[0], &ctx->W21[1]};
+        auto alloc = [&](auto **p, size_t n) -> int {
+            CK(cudaMalloc(p, n));
+            return QP3D_OK;
+        };
+        ctx->book_floats = (kWinFloats + 3) * ntb;
+        if ((rc = alloc(&ctx->state, kStateVols * vol * sizeof(float))) ||
+            (rc = alloc(&ctx->params, 3 * vol * (half ? sizeof(__half) : sizeof(float)))) ||
+            (rc = alloc(&ctx->book, ctx->book_floats * sizeof(float))) ||
+            (rc = alloc(&ctx->record, ntb * ctx->hx * ctx->hy * sizeof(float))) ||
+            (rc = alloc(&ctx->layers, sizeof(float4) * 3 * std::max(g->pml, 1))) ||
+            (rc = alloc(&ctx->spec_err, kSpecHist * sizeof(float)))) {
+            free_shot(ctx);
+            return rc;
         }
+        for (int v = 0; v < kStateVols; ++v) *vols[v] = ctx->state + v * vol;
+        if (half) {
+            ctx->h_vp = static_cast<__half *>(ctx->params);
+            ctx->h_eps = ctx->h_vp + vol;
+            ctx->h_del = ctx->h_eps + vol;
+        } else {
+            ctx->VP = static_cast<float *>(ctx->params);
+            ctx->E2 = ctx->VP + vol;
+            ctx->R8 = ctx->E2 + vol;
+        }
+        ctx->win = ctx->book;
+        ctx->gmax = ctx->win + kWinFloats * ntb;
+        ctx->redo = reinterpret_cast<int *>(ctx->gmax + ntb);
+        ctx->alt_count = reinterpret_cast<unsigned *>(ctx->redo + ntb);
         ctx->half_loaded = half;
-        size_t nrec = (size_t)std::max(g->nt, 1) * ctx->hx * ctx->hy;
-        CK(cudaMalloc(&ctx->record, nrec * sizeof(float)));
-        CK(cudaMalloc(&ctx->gmax, (size_t)std::max(g->nt, 1) * sizeof(float)));
-        CK(cudaMalloc(&ctx->layers, sizeof(float4) * 3 * std::max(g->pml, 1)));
         if (!ctx->errword) CK(cudaMalloc(&ctx->errword, sizeof(unsigned)));
-        size_t ntb = (size_t)std::max(g->nt, 1);
-        CK(cudaMalloc(&ctx->win, kWinFloats * ntb * sizeof(float)));
-        CK(cudaMalloc(&ctx->redo, ntb * sizeof(int)));
-        CK(cudaMalloc(&ctx->alt_count, ntb * sizeof(unsigned)));
-        CK(cudaMalloc(&ctx->spec_err, kSpecHist * sizeof(float)));
     }
     // vp, eps, delta go to the device in one piece each (the wavefield buffers
     // serve as staging; the reset below zeroes them) and are laid out pitched
@@ -311,13 +309,13 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
     // coefficient tables
     derive_coefs(m->c, m->c2, g->dx, g->dy, g->dz, &ctx->coefs);
     if (g->pml > 0) {
-        std::vector<float4> tab(3 * g->pml);
+        std::vector<float4> &tab = ctx->layers_host;   // the copy may still read it on return
+        tab.resize(3 * g->pml);
         derive_layers(m->dlr, m->ddlr, g->pml, g->dt, tab.data());
         derive_layers(m->dfb, m->ddfb, g->pml, g->dt, tab.data() + g->pml);
         derive_layers(m->dtb, m->ddtb, g->pml, g->dt, tab.data() + 2 * g->pml);
         CK(cudaMemcpyAsync(ctx->layers, tab.data(), sizeof(float4) * tab.size(),
                            cudaMemcpyHostToDevice, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
     }
     ctx->wavelet.assign(m->wavelet, m->wavelet + g->nt);
     // sparse source: every non-zero sample (CPU_function.c:326-338 adds all)
@@ -328,23 +326,30 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
                             e.y < g->ny - kRadius && e.z >= kRadius && e.z < g->nz - kRadius;
         (inside ? fused : band).push_back(e);
     }
-    if (ctx->src_fused) cudaFree(ctx->src_fused);
-    if (ctx->src_band) cudaFree(ctx->src_band);
-    if (ctx->src_all) cudaFree(ctx->src_all);
-    ctx->src_fused = ctx->src_band = ctx->src_all = nullptr;
     ctx->fuse_sources = fused.size() <= (size_t)kMaxFusedSources;
     ctx->n_fused = (int)fused.size();
     ctx->n_band = (int)band.size();
     ctx->n_all = (int)all.size();
-    auto up = [&](std::vector<SrcEntry> &v, SrcEntry **d) -> int {
+    // only the lists that the steps read; their buffers are kept for the next shot
+    auto up = [&](const std::vector<SrcEntry> &v, SrcEntry **d, size_t *cap) -> int {
         if (v.empty()) return QP3D_OK;
-        CK(cudaMalloc(d, v.size() * sizeof(SrcEntry)));
+        if (v.size() > *cap) {
+            if (*d) cudaFree(*d);
+            *d = nullptr;
+            *cap = 0;
+            CK(cudaMalloc(d, v.size() * sizeof(SrcEntry)));
+            *cap = v.size();
+        }
         CK(cudaMemcpy(*d, v.data(), v.size() * sizeof(SrcEntry), cudaMemcpyHostToDevice));
         return QP3D_OK;
     };
-    if ((rc = up(fused, &ctx->src_fused)) || (rc = up(band, &ctx->src_band)) ||
-        (rc = up(all, &ctx->src_all)))
+    if (ctx->fuse_sources) {
+        if ((rc = up(fused, &ctx->src_fused, &ctx->cap_fused)) ||
+            (rc = up(band, &ctx->src_band, &ctx->cap_band)))
+            return rc;
+    } else if ((rc = up(all, &ctx->src_all, &ctx->cap_all))) {
         return rc;
+    }
     // the receiver plane is written by the step kernel when every record cell
     // lies inside the updated box
     ctx->rec_fused = g->pml >= kRadius && g->sz >= kRadius && g->sz < g->nz - kRadius &&
@@ -362,19 +367,11 @@ extern "C" int qp3d_shot_reset(qp3d_ctx *ctx)
     if (!ctx) return QP3D_ERR_ARG;
     if (!ctx->loaded) return ctx_fail(ctx, QP3D_ERR_STATE, "no shot loaded");
     CK(cudaSetDevice(ctx->device));
-    size_t vb = (size_t)ctx->vol * sizeof(float);
-    float *zero[] = {ctx->U[0],  ctx->U[1],  ctx->U[2],  ctx->W1[0], ctx->W1[1], ctx->W1[2],
-                     ctx->W3[0], ctx->W3[1], ctx->W3[2], ctx->P[0],  ctx->P[1],  ctx->P[2],
-                     ctx->W21[0], ctx->W21[1]};
-    for (float *p : zero) CK(cudaMemsetAsync(p, 0, vb, ctx->stream));
-    size_t ntb = (size_t)std::max(ctx->g.nt, 1);
-    CK(cudaMemsetAsync(ctx->win, 0, kWinFloats * ntb * sizeof(float), ctx->stream));
-    CK(cudaMemsetAsync(ctx->redo, 0, ntb * sizeof(int), ctx->stream));
-    CK(cudaMemsetAsync(ctx->alt_count, 0, ntb * sizeof(unsigned), ctx->stream));
+    CK(cudaMemsetAsync(ctx->state, 0, kStateVols * (size_t)ctx->vol * sizeof(float), ctx->stream));
+    CK(cudaMemsetAsync(ctx->book, 0, ctx->book_floats * sizeof(float), ctx->stream));
     // error history: no prediction yet (1.0 opens the widest window once)
     static const float first[kSpecHist] = {1.0f};
     CK(cudaMemcpyAsync(ctx->spec_err, first, sizeof(first), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemsetAsync(ctx->gmax, 0, sizeof(float) * std::max(ctx->g.nt, 1), ctx->stream));
     CK(cudaMemsetAsync(ctx->record, 0,
                        sizeof(float) * (size_t)std::max(ctx->g.nt, 1) * ctx->hx * ctx->hy,
                        ctx->stream));

@@ -36,6 +36,12 @@ struct qp3d_ctx {
     int tile_x = 0, nxt = 0, nyt = 0, nchunks = 0, chunk_z = 0;
     size_t smem = 0;
     bool rec_fused = true;
+    // one allocation each: the wavefields and split fields (zeroed together),
+    // the FP32 or half parameters, the per-step bookkeeping
+    float *state = nullptr;
+    void *params = nullptr;
+    float *book = nullptr;
+    size_t book_floats = 0;
     float *U[3] = {nullptr, nullptr, nullptr};
     float *VP = nullptr, *E2 = nullptr, *R8 = nullptr;   // vp, 2 eps, 8 (eps - delta)
     __half *h_vp = nullptr, *h_eps = nullptr, *h_del = nullptr;   // param_fp16 storage
@@ -59,6 +65,8 @@ struct qp3d_ctx {
     float4 *layers = nullptr;
     qp3d::SrcEntry *src_fused = nullptr, *src_band = nullptr, *src_all = nullptr;
     int n_fused = 0, n_band = 0, n_all = 0;
+    size_t cap_fused = 0, cap_band = 0, cap_all = 0;   // entries allocated
+    std::vector<float4> layers_host;
     bool fuse_sources = true;
     unsigned *errword = nullptr;
     qp3d::TileMaps tm[3];

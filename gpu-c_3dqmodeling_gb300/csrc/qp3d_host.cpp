@@ -10,6 +10,7 @@
 #include "qp3d_internal.h"
 #include "qp3d_exact.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -22,21 +23,40 @@ namespace qp3d {
 
 // The reference adds the whole source volume every step
 // (CPU_function.c:326-338); its non-zero samples are the sparse source.
-// Planes are split over up to 16 threads and the lists joined in plane
-// order, so the order is that of one sequential scan.
-void scan_source_volume(const float *s, int nx, int ny, int nz, std::vector<SrcEntry> &out)
+// Planes are split over threads and the lists joined in plane order, so the
+// order is that of one sequential scan.  A thread costs 50 us to start and
+// scans 4 M samples in about 1 ms, so a small volume takes none (with 16
+// threads for every volume a shot of 26x22x18 cells spent half of its load
+// here, 0.8 ms).  Rows are passed over 16 samples at a time: a sample is
+// non-zero when any bit but its sign is set.
+void scan_source_volume(const float *s, int nx, int ny, int nz, std::vector<SrcEntry> &out,
+                        int max_threads)
 {
     out.clear();
     const unsigned hw = std::thread::hardware_concurrency();
-    const int nth = (int)std::max(1u, std::min(16u, hw ? hw : 1u));
+    const long long n = (long long)nx * ny * nz;
+    const int nth = (int)std::max(1ll, std::min({(long long)max_threads, (long long)(hw ? hw : 1u),
+                                                 (n + (1 << 22) - 1) >> 22}));
     std::vector<std::vector<SrcEntry>> part(nth);
     auto work = [&](int t) {
         const int z0 = (int)((long long)nz * t / nth), z1 = (int)((long long)nz * (t + 1) / nth);
         for (int z = z0; z < z1; ++z)
             for (int x = 0; x < nx; ++x) {
                 const float *row = s + ((size_t)z * nx + x) * ny;
-                for (int y = 0; y < ny; ++y)
-                    if (row[y] != 0.0f) part[t].push_back(SrcEntry{x, y, z, row[y]});
+                for (int y = 0; y < ny;) {
+                    if (y + 16 <= ny) {
+                        uint32_t b[16], any = 0;
+                        memcpy(b, row + y, sizeof(b));
+                        for (int i = 0; i < 16; ++i) any |= b[i] << 1;
+                        if (!any) {
+                            y += 16;
+                            continue;
+                        }
+                    }
+                    const int e = std::min(ny, y + 16);
+                    for (; y < e; ++y)
+                        if (row[y] != 0.0f) part[t].push_back(SrcEntry{x, y, z, row[y]});
+                }
             }
     };
     std::vector<std::thread> th;
