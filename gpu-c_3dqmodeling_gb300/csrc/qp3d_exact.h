@@ -148,6 +148,58 @@ QP3D_HD void two_sum(float a, float b, float &s, float &e)
     e = add(sub(a, sub(s, bb)), sub(b, bb));
 }
 
+// ---------------------------------------------------------------------------
+// p / h for a constant h with y = RN(1/h), five operations instead of an IEEE
+// division: q0 = RN(p y) is within 1.5 ulp of the quotient; one correction by
+// the exact remainder leaves q1 = RN(p/h + e) with |e| below 2^-22 ulp, hence
+// within one ulp; by Markstein's theorem (a quotient within one ulp, corrected
+// by its exact remainder times the correctly rounded reciprocal, rounds
+// correctly) the second correction gives RN(p/h).  With kDivLo <= |p| <= kDivHi
+// and a divisor in [kDivHLo, kDivHHi] the quotient is a normal number and a
+// remainder, a multiple of 2^-47 times p's power of two, is exact; p = 0 gives
+// a zero (of either sign).
+// ---------------------------------------------------------------------------
+constexpr float kDivLo = 1.9721523e-31f, kDivHi = 8589934592.0f;     // 2^-102, 2^33
+constexpr float kDivHLo = 9.3132257e-10f, kDivHHi = 8388608.0f;      // 2^-30, 2^23
+QP3D_HD float div_const(float p, float h, float y)
+{
+    const float q0 = mul(p, y);
+    const float q1 = fma_(fma_(-q0, h, p), y, q0);
+    return fma_(fma_(-q1, h, p), y, q1);
+}
+
+// The same for any dividend up to kDivHi, subnormal quotients included: the
+// quotient of p 2^64 is taken as above (24 bits, q), and scaled back, which
+// rounds it to the subnormal grid (t).  That second rounding can differ from
+// the rounding of the exact quotient only when q lies halfway between two grid
+// values; the exact quotient's side of q, the sign of its remainder, then
+// decides.
+QP3D_HD float div_const_scaled(float p, float h, float y)
+{
+    const float up = 18446744073709551616.0f, down = 5.4210109e-20f;   // 2^64, 2^-64
+    const float half = 1.2924697e-26f, grid = 1.4012985e-45f;          // 2^-86, 2^-149
+    const float ps = mul(p, up);
+    const float q = div_const(ps, h, y);
+    const float r = fma_(-q, h, ps), t = mul(q, down);
+    const float e = fma_(-t, up, q);   // q - t 2^64
+    const bool tie = (e == half && r > 0.0f) || (e == -half && r < 0.0f);
+    return tie ? add(t, e > 0.0f ? grid : -grid) : t;
+}
+
+// The taps' dividends stay in div_const's range when every wavefield value they are
+// made of is 0 or has a magnitude in [kWinLo, kWinHi] and every FD weight is 0
+// or in [kWeightLo, kWeightHi]: a difference of such values is 0 or at least
+// an ulp of the smallest, 2^-90, a product 2^-102, and at most 2^(29 + 2 + 2).
+constexpr float kWinLo = 6.7762636e-21f, kWinHi = 536870912.0f;      // 2^-67, 2^29
+constexpr float kWeightLo = 2.4414062e-4f, kWeightHi = 4.0f;         // 2^-12, 2^2
+QP3D_HD bool weight_in_range(float c)
+{
+    const float a = c < 0.0f ? -c : c;
+    return a == 0.0f || (a >= kWeightLo && a <= kWeightHi);
+}
+QP3D_HD bool divisor_in_range(float h) { return h >= kDivHLo && h <= kDivHHi; }
+
+
 // float-float value hi + lo
 struct FF {
     float hi, lo;

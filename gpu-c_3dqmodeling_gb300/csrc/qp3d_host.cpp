@@ -112,7 +112,14 @@ void derive_coefs(const float *c, const float *c2, float dx, float dy, float dz,
     for (int a = 0; a < 3; a++) {
         k->rh[a] = h[a];
         k->rh2[a] = h2[a];
+        k->ry[a] = 1.0f / h[a];
+        k->ry2[a] = 1.0f / h2[a];
     }
+    k->div_ok = 1;
+    for (int m = 0; m < kRadius; m++)
+        if (!xr::weight_in_range(c[31 + m]) || !xr::weight_in_range(c2[31 + m])) k->div_ok = 0;
+    for (int a = 0; a < 3; a++)
+        if (!xr::divisor_in_range(h[a]) || !xr::divisor_in_range(h2[a])) k->div_ok = 0;
 }
 
 // Per-layer PML recursion coefficients (GPU_kernel.cu:569-572,

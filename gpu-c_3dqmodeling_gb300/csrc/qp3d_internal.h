@@ -28,10 +28,18 @@ constexpr int kTileY = 32;        // y cells per tile = 8 quads of 4 cells
 constexpr int kQuadsY = kTileY / 4;
 constexpr int kHaloY = 8;         // y halo rounded up to 16 bytes
 constexpr int kBoxY = kTileY + 2 * kHaloY;   // 48 floats per staged halo row
-// Load groups in flight or in use: the current plane's and two ahead.  One
-// ahead leaves the load's latency open whenever the warps of a CTA drift.
-constexpr int kGroups = 2;
-constexpr int kRingZ = 2 * kRadius + kGroups;   // own-cell planes staged
+// Load groups in flight or in use: the current plane's and those ahead.  The
+// step kernels take microseconds a plane, so one ahead covers a load (a third
+// group with 28-row tiles in the same memory made no difference); the gradmax
+// kernels are done with a plane sooner than its load takes.
+constexpr int kGroups = 2, kGradmaxGroups = 3;
+// Tile height of the allocation-free maximum.  The kernel is bound by shared-
+// memory bandwidth (25 16-byte loads a quad) and its latency; 24-row tiles
+// leave room for four CTAs an SM: 460x460x360 278 us a call with 32 rows, 264
+// with 24; 240x240x190 65 and 60.
+constexpr int kGradmaxTileX = 24;
+// own-cell planes staged
+__host__ __device__ constexpr int ring_z(int groups) { return 2 * kRadius + groups; }
 constexpr int kMaxTileX = 32;
 constexpr int kThreads = kQuadsY * kMaxTileX;        // 256
 constexpr int kStepTileX = 32;   // largest tile height of the step kernels
@@ -65,6 +73,10 @@ struct Coefs {
     // h and h*h rounded.
     float2 rc[kRadius], rc2[kRadius];                  // c[31+m], c2[31+m]
     float rh[3], rh2[3];                               // x, y, z
+    // their rounded reciprocals, and whether weights and divisors allow the
+    // division by them (xr::div_const)
+    float ry[3], ry2[3];
+    int div_ok;
 };
 
 // Arithmetic of the step: the reference CPU operators' roundings

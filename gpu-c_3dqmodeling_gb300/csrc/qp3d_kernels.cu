@@ -187,16 +187,17 @@ struct SmemLayout {
 };
 
 // streams: 16-byte slots per thread (0 for the gradmax kernels)
-__host__ __device__ inline SmemLayout smem_layout(int tile_x, int pml, int nsrc, int streams)
+__host__ __device__ inline SmemLayout smem_layout(int tile_x, int pml, int nsrc, int streams,
+                                                  int groups = kGroups)
 {
     SmemLayout L;
     L.zslot = tile_x * kTileY;
     L.cslot = ((tile_x + 2 * kRadius) * kBoxY + 31) & ~31;
-    L.c_off = (size_t)L.zslot * 4 * kRingZ;
-    L.own_off = L.c_off + (size_t)L.cslot * 4 * kGroups;
+    L.c_off = (size_t)L.zslot * 4 * ring_z(groups);
+    L.own_off = L.c_off + (size_t)L.cslot * 4 * groups;
     L.bar_off = L.own_off + (size_t)plane_threads(tile_x) * 16 * streams;
-    L.cnt_off = L.bar_off + 8 * kGroups;
-    L.tab_off = (L.cnt_off + 4 * (kGroups + 1) + 15) & ~(size_t)15;
+    L.cnt_off = L.bar_off + 8 * groups;
+    L.tab_off = (L.cnt_off + 4 * (groups + 1) + 15) & ~(size_t)15;
     L.ytab_off = L.tab_off + (streams ? 16 * 3 * (size_t)(pml > 0 ? pml : 1) : 0);
     L.src_off = L.ytab_off + (streams ? 16 * kTileY : 0);
     L.misc_off = L.src_off + (streams ? sizeof(SrcEntry) * (size_t)(nsrc > 0 ? nsrc : 1) : 0);
@@ -214,7 +215,10 @@ size_t plane_smem_bytes(int tile_x, int pml, int nsrc)
     return smem_layout(tile_x, pml, nsrc, step_streams(pml)).total;
 }
 
-size_t gradmax_smem_bytes(int tile_x) { return smem_layout(tile_x, 0, 0, 0).total; }
+size_t gradmax_smem_bytes(int tile_x)
+{
+    return smem_layout(tile_x, 0, 0, 0, kGradmaxGroups).total;
+}
 
 // The number of z chunks of a plane kernel's grid: tiles columns of ncz planes,
 // smem bytes a CTA.  A CTA's march over its planes is a serial chain (2-3 us a
@@ -390,12 +394,48 @@ __device__ __forceinline__ float2 div2(float2 p, float h)
     return make_float2(__fdiv_rn(p.x, h), __fdiv_rn(p.y, h));
 }
 
-// one tap of both derivatives for a pair of cells: a = u[+m], b = u[-m]
-__device__ __forceinline__ void tap2(float2 a, float2 b, float2 u0, float2 c, float2 c2, float h,
-                                     float h2, float2 &g, float2 &l)
+// How the taps divide: IEEE division, or xr::div_const or
+// xr::div_const_scaled in packed form.  IEEE divisions, with their slow path
+// for the subnormal values ahead of a wavefront, were 9300 of the instructions
+// a warp spent on a plane (998 us a step on 140^3; 223 with products in their
+// place).
+enum TapDiv { kDivIeee, kDivConst, kDivScaled };
+
+__device__ __forceinline__ float2 div_const2(float2 p, float h, float y)
 {
-    g = __fadd2_rn(g, div2(__fmul2_rn(c, sub2(a, b)), h));
-    l = __fadd2_rn(l, div2(__fmul2_rn(c2, lap_tap2(a, b, u0)), h2));
+    const float2 nh = make_float2(-h, -h), y2 = make_float2(y, y);
+    const float2 q0 = __fmul2_rn(p, y2);
+    const float2 q1 = __ffma2_rn(__ffma2_rn(q0, nh, p), y2, q0);
+    return __ffma2_rn(__ffma2_rn(q1, nh, p), y2, q1);
+}
+
+template <int DIV>
+__device__ __forceinline__ float2 tap_div2(float2 p, float h, float y)
+{
+    if (DIV == kDivIeee) return div2(p, h);
+    if (DIV == kDivConst) return div_const2(p, h, y);
+    const float up = 18446744073709551616.0f, down = 5.4210109e-20f;   // 2^64, 2^-64
+    const float half = 1.2924697e-26f, grid = 1.4012985e-45f;          // 2^-86, 2^-149
+    const float2 ps = __fmul2_rn(p, make_float2(up, up));
+    const float2 q = div_const2(ps, h, y);
+    const float2 r = __ffma2_rn(q, make_float2(-h, -h), ps);
+    float2 t = __fmul2_rn(q, make_float2(down, down));
+    const float2 e = __ffma2_rn(t, make_float2(-up, -up), q);
+    if (fabsf(e.x) == half && (e.x > 0.0f ? r.x > 0.0f : r.x < 0.0f))
+        t.x = __fadd_rn(t.x, copysignf(grid, e.x));
+    if (fabsf(e.y) == half && (e.y > 0.0f ? r.y > 0.0f : r.y < 0.0f))
+        t.y = __fadd_rn(t.y, copysignf(grid, e.y));
+    return t;
+}
+
+// one tap (m) of both derivatives along an axis for a pair of cells: a = u[+m],
+// b = u[-m]
+template <int DIV>
+__device__ __forceinline__ void tap2(float2 a, float2 b, float2 u0, const Coefs &k, int m, int ax,
+                                     float2 &g, float2 &l)
+{
+    g = __fadd2_rn(g, tap_div2<DIV>(__fmul2_rn(k.rc[m], sub2(a, b)), k.rh[ax], k.ry[ax]));
+    l = __fadd2_rn(l, tap_div2<DIV>(__fmul2_rn(k.rc2[m], lap_tap2(a, b, u0)), k.rh2[ax], k.ry2[ax]));
 }
 
 __device__ __forceinline__ void quad_derivs_ref(const Taps &T, const Coefs &k, float Ux[4],
@@ -420,8 +460,8 @@ __device__ __forceinline__ void quad_derivs_ref(const Taps &T, const Coefs &k, f
         float2 g = zero, l = zero;
 #pragma unroll
         for (int m = 0; m < kRadius; ++m)
-            tap2(f2(Y[8 + j0 + m + 1], Y[8 + j1 + m + 1]), f2(Y[8 + j0 - m - 1], Y[8 + j1 - m - 1]),
-                 c0[h], k.rc[m], k.rc2[m], k.rh[1], k.rh2[1], g, l);
+            tap2<kDivConst>(f2(Y[8 + j0 + m + 1], Y[8 + j1 + m + 1]),
+                       f2(Y[8 + j0 - m - 1], Y[8 + j1 - m - 1]), c0[h], k, m, 1, g, l);
         Uy[j0] = g.x; Uy[j1] = g.y;
         Uyy[j0] = l.x; Uyy[j1] = l.y;
     }
@@ -433,7 +473,7 @@ __device__ __forceinline__ void quad_derivs_ref(const Taps &T, const Coefs &k, f
         const float2 a2[2] = {f2(a.x, a.y), f2(a.z, a.w)}, b2[2] = {f2(b.x, b.y), f2(b.z, b.w)};
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-            tap2(a2[h], b2[h], c0[h], k.rc[m], k.rc2[m], k.rh[0], k.rh2[0], gx[h], lx[h]);
+            tap2<kDivConst>(a2[h], b2[h], c0[h], k, m, 0, gx[h], lx[h]);
     }
     Ux[0] = gx[0].x; Ux[1] = gx[0].y; Ux[2] = gx[1].x; Ux[3] = gx[1].y;
     Uxx[0] = lx[0].x; Uxx[1] = lx[0].y; Uxx[2] = lx[1].x; Uxx[3] = lx[1].y;
@@ -445,10 +485,83 @@ __device__ __forceinline__ void quad_derivs_ref(const Taps &T, const Coefs &k, f
         const float2 a2[2] = {f2(a.x, a.y), f2(a.z, a.w)}, b2[2] = {f2(b.x, b.y), f2(b.z, b.w)};
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-            tap2(a2[h], b2[h], c0[h], k.rc[m], k.rc2[m], k.rh[2], k.rh2[2], gz[h], lz[h]);
+            tap2<kDivConst>(a2[h], b2[h], c0[h], k, m, 2, gz[h], lz[h]);
     }
     Uz[0] = gz[0].x; Uz[1] = gz[0].y; Uz[2] = gz[1].x; Uz[3] = gz[1].y;
     Uzz[0] = lz[0].x; Uzz[1] = lz[0].y; Uzz[2] = lz[1].x; Uzz[3] = lz[1].y;
+}
+
+// The same with the other two divisions, as loops: they run for the warps
+// around the leading edge of a wavefield, and three unrolled forms would not
+// stay in the instruction cache.
+template <int DIV>
+__device__ __forceinline__ void quad_derivs_ref_loop(const Taps &T, const Coefs &k, float Ux[4],
+                                                     float Uy[4], float Uz[4], float Uxx[4],
+                                                     float Uyy[4], float Uzz[4], float u0[4])
+{
+    const float4 c = lds4(T.pc);
+    const float2 c0[2] = {f2(c.x, c.y), f2(c.z, c.w)};
+    u0[0] = c.x; u0[1] = c.y; u0[2] = c.z; u0[3] = c.w;
+    float2 g[3][2], l[3][2];
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        g[ax][0] = g[ax][1] = l[ax][0] = l[ax][1] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+        for (int m = 0; m < kRadius; ++m) {
+            float4 a, b;
+            if (ax == 0) {
+                a = lds4(T.pc + (m + 1) * kBoxY);
+                b = lds4(T.pc - (m + 1) * kBoxY);
+            } else if (ax == 1) {
+                const float *pa = T.pc + m + 1, *pb = T.pc - m - 1;
+                a = make_float4(pa[0], pa[1], pa[2], pa[3]);
+                b = make_float4(pb[0], pb[1], pb[2], pb[3]);
+            } else {
+                a = ztap(T, kRadius + m + 1);
+                b = ztap(T, kRadius - m - 1);
+            }
+            tap2<DIV>(f2(a.x, a.y), f2(b.x, b.y), c0[0], k, m, ax, g[ax][0], l[ax][0]);
+            tap2<DIV>(f2(a.z, a.w), f2(b.z, b.w), c0[1], k, m, ax, g[ax][1], l[ax][1]);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        Ux[2 * h] = g[0][h].x; Ux[2 * h + 1] = g[0][h].y;
+        Uy[2 * h] = g[1][h].x; Uy[2 * h + 1] = g[1][h].y;
+        Uz[2 * h] = g[2][h].x; Uz[2 * h + 1] = g[2][h].y;
+        Uxx[2 * h] = l[0][h].x; Uxx[2 * h + 1] = l[0][h].y;
+        Uyy[2 * h] = l[1][h].x; Uyy[2 * h + 1] = l[1][h].y;
+        Uzz[2 * h] = l[2][h].x; Uzz[2 * h + 1] = l[2][h].y;
+    }
+}
+
+// What four wavefield values ask of the division: 0 when each is 0 or in
+// [kWinLo, kWinHi], bit 0 for a smaller one, bit 1 for a larger one, an
+// infinity or a NaN (magnitudes compared as integers, the sign shifted out).
+__device__ __forceinline__ unsigned window_class(const float4 &v)
+{
+    const unsigned lo = 2u * __float_as_uint(xr::kWinLo), hi = 2u * __float_as_uint(xr::kWinHi);
+    const unsigned a = 2u * __float_as_uint(v.x), b = 2u * __float_as_uint(v.y),
+                   c = 2u * __float_as_uint(v.z), d = 2u * __float_as_uint(v.w);
+    // 0 - 1 is the largest unsigned value
+    return (unsigned)(min(min(a - 1u, b - 1u), min(c - 1u, d - 1u)) < lo - 1u) |
+           ((unsigned)(max(max(a, b), max(c, d)) > hi) << 1);
+}
+
+// The same of every x and y tap of a warp's four rows (rows r0..r0+3 of a tile
+// of tile_x; halo: the halo plane), shared among the lanes: 14 rows of the
+// tile's 32 columns, and the 8 columns either side of the warp's own rows.
+__device__ __forceinline__ unsigned halo_class(const float *halo, int r0, int tile_x)
+{
+    const int lane = threadIdx.x & 31, last = tile_x + 2 * kRadius - 1;
+    unsigned cls = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int e = min(lane + 32 * i, 111);
+        cls |= window_class(lds4(halo + min(r0 + (e >> 3), last) * kBoxY + kHaloY + 4 * (e & 7)));
+    }
+    const int row = min(r0 + kRadius + ((lane & 15) >> 2), last), c = lane & 3;
+    return cls | window_class(lds4(halo + row * kBoxY + (c < 2 ? 4 * c : kTileY + 4 * c)));
 }
 
 // First derivatives only, for the gradmax kernels.
@@ -501,18 +614,17 @@ __device__ __forceinline__ void quad_grad_ref(const Taps &T, const Coefs &k, flo
 // rows.  The x and y taps need the 5-row, 8-column halo, but of the current
 // plane only: 8 KB.  Iteration t (z = z0 + t) therefore waits for one group
 // of loads: own-cell plane t + 10 (iteration 0: planes 0..10; plane i holds
-// z = z0 - 5 + i, in slot i % kRingZ) and halo plane t (slot t % kGroups),
-// both completing on full[t % kGroups].  Keeping eleven halo planes instead,
-// 8 KB each, left room for one load ahead, whose latency every iteration then
-// waited for; this form keeps kGroups - 1 = 2 groups ahead in less memory.
+// z = z0 - 5 + i, in slot i % (10 + G)) and halo plane t (slot t % G), both
+// completing on full[t % G].  Eleven halo planes of 8 KB instead would leave
+// no room for the step kernels' per-cell streams.
 //
-// A warp that has finished iteration t adds one to cnt[t % kGroups]; the last
-// one to do so refills what the iteration freed with group t + kGroups (its
+// A warp that has finished iteration t adds one to cnt[t % G]; the last one to
+// do so refills what the iteration freed with group t + G (its
 // own-cell plane goes to the slot of plane t, its halo plane to that of halo
 // plane t).  No CTA barrier, no producer warp, and the load starts as soon as
 // its slots are free.
 // ---------------------------------------------------------------------------
-struct Pipe {
+template <int G> struct Pipe {
     float *zr, *cr;
     uint64_t *full;
     unsigned *cnt;
@@ -526,44 +638,48 @@ struct Pipe {
     int hold;        // test hook: own-cell plane never loaded (-1: none)
 };
 
-__device__ __forceinline__ void pipe_issue(const Pipe &P, const TileMaps *tm, int g)
+template <int G>
+__device__ __forceinline__ void pipe_issue(const Pipe<G> &P, const TileMaps *tm, int g)
 {
-    const int s = g % kGroups;
+    const int s = g % G;
     uint64_t *bar = &P.full[s];
     *P.issued = g + 1;
     mbar_arrive_expect_tx(bar, P.cbytes + P.zbytes * (g == 0 ? 2 * kRadius + 1 : 1));
     for (int i = g == 0 ? 0 : g + 2 * kRadius; i <= g + 2 * kRadius; ++i)
         if (i != P.hold)   // test hook: the wait for this group runs out
-            tma_load_3d(P.zr + (i % kRingZ) * P.zslot, &tm->z, P.y0, P.x0, P.z0 - kRadius + i, bar);
+            tma_load_3d(P.zr + (i % ring_z(G)) * P.zslot, &tm->z, P.y0, P.x0, P.z0 - kRadius + i, bar);
     tma_load_3d(P.cr + s * P.cslot, &tm->c, P.y0 - kHaloY, P.x0 - kRadius, P.z0 + g, bar);
 }
 
-__device__ __forceinline__ bool pipe_wait(const Pipe &P, int g)
+template <int G>
+__device__ __forceinline__ bool pipe_wait(const Pipe<G> &P, int g)
 {
-    return mbar_wait_bounded(&P.full[g % kGroups], (unsigned)((g / kGroups) & 1), P.wait_ns);
+    return mbar_wait_bounded(&P.full[g % G], (unsigned)((g / G) & 1), P.wait_ns);
 }
 
 // The end of a warp's iteration t (see above).
-__device__ __forceinline__ void pipe_release(const Pipe &P, const TileMaps *tm, int t)
+template <int G>
+__device__ __forceinline__ void pipe_release(const Pipe<G> &P, const TileMaps *tm, int t)
 {
     __syncwarp();
-    if ((threadIdx.x & 31) == 0 && t + kGroups < P.ngroups) {
+    if ((threadIdx.x & 31) == 0 && t + G < P.ngroups) {
         unsigned old;
-        unsigned *c = &P.cnt[t % kGroups];
+        unsigned *c = &P.cnt[t % G];
         asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
                      : "=r"(old) : "r"(smem_u32(c)) : "memory");
         if (old == (unsigned)P.ncw - 1) {
             *c = 0;   // next used after the group issued here has landed
             fence_proxy_async();
-            pipe_issue(P, tm, t + kGroups);
+            pipe_issue(P, tm, t + G);
         }
     }
 }
 
 // Thread 0, before a CTA barrier: barriers and counters, then the first groups.
-__device__ void pipe_init(const Pipe &P)
+template <int G>
+__device__ void pipe_init(const Pipe<G> &P)
 {
-    for (int s = 0; s < kGroups; ++s) {
+    for (int s = 0; s < G; ++s) {
         mbar_init(&P.full[s], 1);
         P.cnt[s] = 0;
     }
@@ -573,32 +689,35 @@ __device__ void pipe_init(const Pipe &P)
     fence_proxy_async();
 }
 
-__device__ void pipe_start(const Pipe &P, const TileMaps *tm)
+template <int G>
+__device__ void pipe_start(const Pipe<G> &P, const TileMaps *tm)
 {
-    for (int g = 0; g < kGroups && g < P.ngroups; ++g) pipe_issue(P, tm, g);
+    for (int g = 0; g < G && g < P.ngroups; ++g) pipe_issue(P, tm, g);
 }
 
 // The end of a column: true if no wait ran out (the same in every thread).
 // Otherwise the loads still in flight are waited for (bounded), so that none
 // lands in shared memory after the CTA has exited.
-__device__ bool pipe_finish(const Pipe &P, bool ok, unsigned *err)
+template <int G>
+__device__ bool pipe_finish(const Pipe<G> &P, bool ok, unsigned *err)
 {
     if (__syncthreads_and(ok)) return true;
     if (threadIdx.x == 0) {
         atomicOr(err, kErrWaitTimeout);
-        for (int g = max(0, *P.issued - kGroups); g < *P.issued; ++g) (void)pipe_wait(P, g);
+        for (int g = max(0, *P.issued - G); g < *P.issued; ++g) (void)pipe_wait(P, g);
     }
     return false;
 }
 
-__device__ __forceinline__ void pipe_setup(Pipe &P, unsigned char *smem, const SmemLayout &L,
+template <int G>
+__device__ __forceinline__ void pipe_setup(Pipe<G> &P, unsigned char *smem, const SmemLayout &L,
                                            int tile_x, int y0, int x0, int z0, int nzc)
 {
     P.zr = reinterpret_cast<float *>(smem);
     P.cr = reinterpret_cast<float *>(smem + L.c_off);
     P.full = reinterpret_cast<uint64_t *>(smem + L.bar_off);
     P.cnt = reinterpret_cast<unsigned *>(smem + L.cnt_off);
-    P.issued = reinterpret_cast<int *>(P.cnt + kGroups);
+    P.issued = reinterpret_cast<int *>(P.cnt + G);
     P.zslot = L.zslot;
     P.cslot = L.cslot;
     P.zbytes = (unsigned)(tile_x * kTileY * 4);
@@ -614,7 +733,8 @@ __device__ __forceinline__ void pipe_setup(Pipe &P, unsigned char *smem, const S
 
 // The launch's wait limit (0: 2 s) and the plane-withholding test hook (the
 // first CTA of a grid launch only).
-__device__ __forceinline__ void pipe_hooks(Pipe &P, unsigned long long wait_ns, int hold_plane)
+template <int G>
+__device__ __forceinline__ void pipe_hooks(Pipe<G> &P, unsigned long long wait_ns, int hold_plane)
 {
     if (wait_ns) P.wait_ns = wait_ns;
     if (hold_plane > 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) P.hold = hold_plane - 1;
@@ -622,32 +742,35 @@ __device__ __forceinline__ void pipe_hooks(Pipe &P, unsigned long long wait_ns, 
 
 // Before a CTA reuses its barriers for another tile (thread 0, after a CTA
 // barrier; every load of the previous tile has been waited for).
-__device__ void pipe_inval(const Pipe &P)
+template <int G>
+__device__ void pipe_inval(const Pipe<G> &P)
 {
-    for (int s = 0; s < kGroups; ++s)
+    for (int s = 0; s < G; ++s)
         asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&P.full[s])) : "memory");
 }
 
 // The ring positions of iteration t, kept incrementally.
-__device__ __forceinline__ Taps taps_start(const Pipe &P, int r, int q)
+template <int G>
+__device__ __forceinline__ Taps taps_start(const Pipe<G> &P, int r, int q)
 {
     Taps T;
     T.pc = P.cr + (r + kRadius) * kBoxY + kHaloY + 4 * q;
     T.za = P.zr + r * kTileY + 4 * q;
-    T.wrap = kRingZ;
+    T.wrap = ring_z(G);
     T.zslot = P.zslot;
-    T.zlen = kRingZ * P.zslot;
+    T.zlen = ring_z(G) * P.zslot;
     return T;
 }
 
-__device__ __forceinline__ void taps_next(Taps &T, const Pipe &P, int t)   // from t to t + 1
+template <int G>
+__device__ __forceinline__ void taps_next(Taps &T, const Pipe<G> &P, int t)   // from t to t + 1
 {
     T.za += T.zslot;
     if (--T.wrap == 0) {
         T.za -= T.zlen;
-        T.wrap = kRingZ;
+        T.wrap = ring_z(G);
     }
-    T.pc += t % kGroups == kGroups - 1 ? -(kGroups - 1) * P.cslot : P.cslot;
+    T.pc += t % G == G - 1 ? -(G - 1) * P.cslot : P.cslot;
 }
 
 // ---------------------------------------------------------------------------
@@ -664,8 +787,8 @@ __device__ __forceinline__ bool gradmax_tile(const TileMaps *tm, const PlanePara
     const int tid = threadIdx.x;
     const int q = tid & (kQuadsY - 1), r = tid / kQuadsY;
     const int nzc = z1 - z0;
-    const SmemLayout L = smem_layout(tile_x, 0, 0, 0);
-    Pipe P;
+    const SmemLayout L = smem_layout(tile_x, 0, 0, 0, kGradmaxGroups);
+    Pipe<kGradmaxGroups> P;
     pipe_setup(P, smem, L, tile_x, y0, x0, z0, nzc);
     if (!REUSE) pipe_hooks(P, p.wait_ns, p.hold_plane);
     if (tid == 0) {
@@ -730,7 +853,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 // launch finds zero.  The last CTA delivers the result (NaN when a wait ran
 // out) and the error flags, and leaves the scratch zero again.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kQuadsY * kGradmaxTileX, 4)
     qp3d_gradmax_single_kernel(const __grid_constant__ TileMaps tm, const PlaneParams p,
                                GradmaxScratch *sc, float *out, unsigned *host_flags)
 {
@@ -1149,7 +1272,7 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
     const int tid = threadIdx.x, lane = tid & 31;
     const int q = tid & (kQuadsY - 1), r = tid / kQuadsY;
     const int nzc = z1 - z0;
-    Pipe P;
+    Pipe<kGroups> P;
     pipe_setup(P, smem, L, tile_x, y0, x0, z0, nzc);
     if (!REUSE) pipe_hooks(P, p.wait_ns, p.hold_plane);
     const int nx = p.nx, ny = p.ny, nz = p.nz, pml = p.pml;
@@ -1278,13 +1401,14 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
     // The body exists twice, so that the warps of the interior carry nothing
     // of the shell's update: sharing one body, with the update under a branch,
     // cost them 160 of 650 instructions a plane.
+    // reference arithmetic: the classes (window_class) of the thread's quad in
+    // the planes staged last, two bits each, the newest lowest
+    unsigned zhist = 0;
+    float Ux[4], Uy[4], Uz[4], Uxx[4], Uyy[4], Uzz[4], u0[4];
     auto plane_step = [&](int t, auto shell) {
         constexpr bool PML = decltype(shell)::value;
         const int z = z0 + t;
         const int fz = PML ? face_of_z(z) : -1;
-        float Ux[4], Uy[4], Uz[4], Uxx[4], Uyy[4], Uzz[4], u0[4];
-        if (AR == kArithRef) quad_derivs_ref(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
-        else quad_derivs<true>(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
         // a thread without a cell reads whatever its slots hold: it stores nothing
         cp_async_wait();
         const float4 u1v = own[0];
@@ -1479,6 +1603,19 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
     for (int t = 0; t < nzc; taps_next(T, P, t), ++t, base += plane) {
         ok = __all_sync(0xffffffffu, pipe_wait(P, t));   // warps stay converged for the collectives below
         if (!ok) break;
+        if (AR == kArithRef) {
+            if (t == 0)
+                for (int i = 0; i < 2 * kRadius; ++i) zhist = (zhist << 2) | window_class(ztap(T, i));
+            zhist = (zhist << 2) | window_class(ztap(T, 2 * kRadius));
+            unsigned cls = halo_class(T.pc - ((r + kRadius) * kBoxY + kHaloY + 4 * q), r & ~3, tile_x);
+            if (row_ok) cls |= ((zhist & 0x155555u) ? 1u : 0u) | ((zhist & 0x2aaaaau) ? 2u : 0u);
+            cls = k.div_ok ? __reduce_or_sync(0xffffffffu, cls) : 2u;
+            if (cls == 0) quad_derivs_ref(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
+            else if (cls == 1) quad_derivs_ref_loop<kDivScaled>(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
+            else quad_derivs_ref_loop<kDivIeee>(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
+        } else {
+            quad_derivs<true>(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
+        }
         if (xy_face_warp || face_of_z(z0 + t) >= 0) plane_step(t, std::true_type());
         else plane_step(t, std::false_type());
     }
@@ -2125,7 +2262,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
     const int nzc = z1 - z0, nx = a.nx, ny = a.ny, nz = a.nz, pml = a.pml;
     const SmemLayout L = smem_layout(tile_x, pml, 0, kAdjStreams);
     float4 *tab = reinterpret_cast<float4 *>(smem + L.tab_off);
-    Pipe P;
+    Pipe<kGroups> P;
     pipe_setup(P, smem, L, tile_x, y0, x0, z0, nzc);
     pipe_hooks(P, a.wait_ns, 0);
     const int x = x0 + r, yq = y0 + 4 * q;

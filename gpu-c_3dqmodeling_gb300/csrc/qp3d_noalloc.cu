@@ -33,9 +33,9 @@ using namespace qp3d;
 
 namespace {
 
-// Largest number of CTAs.  With 32-cell x 32-row tiles this covers nx*ny up
-// to about 64 M cells per plane.
-constexpr unsigned kNoAllocMaxBlocks = 1u << 16;
+// Largest number of 32-cell x 32-row tiles per plane: nx*ny up to about 64 M
+// cells.
+constexpr unsigned kNoAllocMaxTiles = 1u << 16;
 
 static __device__ GradmaxScratch g_noalloc_scratch;
 
@@ -96,19 +96,19 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
 
     // launch plan (as the shot path plans it)
     const int ncx = nx - 2 * kRadius, ncz = nz - 2 * kRadius;
-    const int ntx = (ncx + kMaxTileX - 1) / kMaxTileX;
+    const int ntx = (ncx + kGradmaxTileX - 1) / kGradmaxTileX;
     const int tile_x = (ncx + ntx - 1) / ntx;
     const int nxt = (ncx + tile_x - 1) / tile_x;
     const int nyt = (ny - kRadius - 1) / kTileY + 1;
     const long long tiles = (long long)nxt * nyt;
-    if (tiles > kNoAllocMaxBlocks) {
+    const long long tiles32 = (long long)((ncx + 31) / 32) * nyt;
+    if (tiles32 > kNoAllocMaxTiles) {
         snprintf(msg, sizeof(msg),
                  "grid %dx%d needs %lld tiles per z chunk; qp3d_gradmax_noalloc holds at most %u",
-                 nx, ny, tiles, kNoAllocMaxBlocks);
+                 nx, ny, tiles32, kNoAllocMaxTiles);
         return report(err, errlen, QP3D_ERR_ARG, msg);
     }
     long long nch = plan_chunks(tiles, ncz, plane_threads(tile_x), gradmax_smem_bytes(tile_x), nsm);
-    nch = std::min(nch, (long long)(kNoAllocMaxBlocks / tiles));
     const int chunk_z = (int)((ncz + nch - 1) / nch);
     nch = (ncz + chunk_z - 1) / chunk_z;
     // the launch grid is (y tiles, x tiles, z chunks); CUDA limits its second
