@@ -1056,8 +1056,10 @@ __device__ __forceinline__ float4 step_layer(float4 t)
 
 // The split-field update of one PML cell of face code f, layer li; v: its
 // pml_inputs, ks as in step_tile.
+// (Not inlined, as scalar_s_call: four copies each in two loop bodies did not
+// stay in the instruction cache; 2-5 % of a step in the reference arithmetic.)
 template <int AR>
-__device__ __forceinline__ xr::PmlOut pml_cell(int f, float4 layer, float ks, float e1, float vp,
+__device__ __noinline__ xr::PmlOut pml_cell(int f, float4 layer, float ks, float e1, float vp,
                                                float4 v, float dt, float w11, float w12, float w21,
                                                float w31, float w32, float p1, float p2)
 {
@@ -1249,6 +1251,12 @@ __device__ __forceinline__ void pml_quad_fast(
     }
 }
 
+__device__ __noinline__ float scalar_s_call(float Ux, float Uy, float Uz, float m2, float e,
+                                            float r)
+{
+    return xr::scalar_s(Ux, Uy, Uz, m2, e, r);
+}
+
 // One tile column [z0, z1) of the step.  The grid kernel below runs one per
 // CTA; the batched kernel runs many per CTA (REUSE: barriers invalidated at
 // the end, return value uniform over the CTA; false = a wait timed out).
@@ -1341,7 +1349,7 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
     const unsigned plane = (unsigned)p.plane;
 
     // Before the previous kernel has finished (grid launches): barriers, the
-    // parameters and the layer coefficients, which no step changes.
+    // parameters, the layer coefficients and the sources, which no step changes.
     prefetch_params(base);
     if (tid == 0) {
         misc_u[0] = misc_u[1] = 0;   // sources of this column, deferred cells
@@ -1362,6 +1370,15 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
         ytab[kTileY + tid] = c.y;
         ytab[2 * kTileY + tid] = c.z;
         ytab[3 * kTileY + tid] = c.w;
+    }
+    if (p.nsrc) {   // the sources of this column
+        __syncthreads();
+        for (int e = tid; e < p.nsrc; e += blockDim.x) {
+            const SrcEntry s = p.src[e];
+            if (s.x >= x0 && s.x < x0 + tile_x && s.y >= y0 && s.y < y0 + kTileY && s.z >= z0 &&
+                s.z < z1)
+                csrc[atomicAdd(&misc_u[0], 1u)] = s;
+        }
     }
     if (!REUSE) pdl_wait();
     if (tid == 0) pipe_start(P, tm);
@@ -1387,13 +1404,6 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
         }
     }
     __syncthreads();
-    for (int e = tid; e < p.nsrc; e += blockDim.x) {
-        const SrcEntry s = p.src[e];
-        if (s.x >= x0 && s.x < x0 + tile_x && s.y >= y0 && s.y < y0 + kTileY && s.z >= z0 &&
-            s.z < z1)
-            csrc[atomicAdd(&misc_u[0], 1u)] = s;
-    }
-    if (p.nsrc) __syncthreads();
     const float T2lo = misc[0], T2hi = misc[1];
     const int ncsrc = (int)misc_u[0];
     bool ok = true;
@@ -1477,7 +1487,7 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     if ((above & okb) >> j & 1u)
-                        kS[j] = xr::scalar_s(Ux[j], Uy[j], Uz[j], m2[j], f4(Ev, j), f4(Rv, j));
+                        kS[j] = scalar_s_call(Ux[j], Uy[j], Uz[j], m2[j], f4(Ev, j), f4(Rv, j));
             } else {
                 float S[4];
 #pragma unroll
@@ -1773,18 +1783,19 @@ __device__ __forceinline__ void fix_cell(const PlaneParams &p, float Tf, size_t 
         p.record[(long long)(x - pml) * (ny - 2 * pml) + (y - pml)] = out;
 }
 
-// A block's share of the segments, kThreads at a time: lens of them are
-// scanned to offsets, so that the threads share the cells evenly however the
-// lengths differ.  len(i) is segment i's length (0: none to fix), fix(i, j)
-// handles its entry j.
+// A block's share of the segments, kThreads at a time: their lengths (count)
+// are scanned to offsets, so that the threads share the cells evenly however
+// the lengths differ.  len(i, n) is how many of segment i's n cells to fix (0:
+// none), fix(i, j) handles its entry j.
 template <class Len, class Fix>
-__device__ __forceinline__ void for_segment_cells(int nseg, Len len, Fix fix)
+__device__ __forceinline__ void for_segment_cells(int nseg, const unsigned *count, Len len, Fix fix)
 {
     __shared__ unsigned s_off[kThreads + 1], s_w[kThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     for (int first = 0; first * (int)gridDim.x + (int)blockIdx.x < nseg; first += blockDim.x) {
         const long long i = blockIdx.x + (long long)(first + tid) * gridDim.x;
-        const unsigned c = i < nseg ? len((int)i) : 0u;
+        const unsigned n = i < nseg ? count[i] : 0u;   // beside the loads len asks for
+        const unsigned c = i < nseg ? len((int)i, n) : 0u;
         unsigned incl = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1831,22 +1842,21 @@ __global__ void __launch_bounds__(kStepThreads, 2)
 {
     pdl_trigger();
     pdl_wait();
-    const bool rerun = step_missed(p);
     const int nyt = (p.ny - kRadius - 1) / kTileY + 1;
     const int nxt = (p.nx - 2 * kRadius + p.tile_x - 1) / p.tile_x;
     const int nch = (p.nz - 2 * kRadius + p.chunk_z - 1) / p.chunk_z;
     const int ntiles = nyt * nxt * nch;
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x < 2) step_account(p, spec_err);
-    const float Tf = threshold_of(p.gmax[p.step]);
     for_segment_cells(
-        ntiles,
-        [&](int i) {
-            const unsigned n = p.dcount[i];
+        ntiles, p.dcount,
+        [&](int, unsigned n) {
             if (n) atomicAdd(p.alt_count, n);
-            return rerun ? 0u : n;
+            return step_missed(p) ? 0u : n;
         },
-        [&](int i, unsigned j) { fix_cell<HALF, AR>(p, Tf, (size_t)i * p.dcap + j); });
-    if (!rerun) return;
+        [&](int i, unsigned j) {
+            fix_cell<HALF, AR>(p, threshold_of(p.gmax[p.step]), (size_t)i * p.dcap + j);
+        });
+    if (!step_missed(p)) return;
     extern __shared__ __align__(128) unsigned char smem[];
     const DeferSeg none = {0, 0, nullptr};
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -2109,11 +2119,10 @@ __global__ void __launch_bounds__(kStepThreads, 2)
     for (int s = threadIdx.x; s < b.nshots; s += blockDim.x)
         if (b.pp[s].active && step_missed(b.pp[s])) s_missed = 1;
     for_segment_cells(
-        b.nwork,
-        [&](int i) {
+        b.nwork, b.dcount,
+        [&](int i, unsigned n) {
             const PlaneParams &g = b.pp[b.work[i].shot];
             if (!g.active) return 0u;
-            const unsigned n = b.dcount[i];
             if (n) atomicAdd(g.alt_count, n);
             return n && !step_missed(g) ? n : 0u;
         },
