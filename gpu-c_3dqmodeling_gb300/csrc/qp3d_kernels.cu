@@ -1555,6 +1555,7 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
                 o.w31 = own[6 * nthr]; o.w32 = own[7 * nthr];
                 o.p1 = own[8 * nthr];  o.p2 = own[9 * nthr];
                 o.w21 = own[10 * nthr];
+                if (t + 1 < nzc) prefetch_pml(base + plane, face_of_z(z + 1) >= 0);
                 PmlNew n;
                 const int liz = z < pml ? pml - z : z - nz + pml;
                 if (AR == kArithRef)
@@ -1571,10 +1572,11 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
                 }
             }
         }
-        if (t + 1 < nzc) {
-            const bool z_face = face_of_z(z + 1) >= 0;
-            if (xy_face_warp || z_face) prefetch_pml(base + plane, z_face);
-        }
+        // a quad of the shell has asked for the next plane's state already
+        // (as soon as it had read its own: 2.5 % of a step on 240x240x190
+        // against here)
+        if (t + 1 < nzc && face_of_z(z + 1) >= 0 && !(PML && (xy_face || (row_ok && fz >= 0))))
+            prefetch_pml(base + plane, true);
         if (AR == kArithRef) {   // source injection (CPU_function.c:334): u3 += source * wavelet
             unsigned srcb = 0;
             for (int e = 0; e < ncsrc; ++e) {
