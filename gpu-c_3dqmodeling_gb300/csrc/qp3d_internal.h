@@ -323,6 +323,10 @@ cudaError_t launch_batch_resolve(const BatchArgs &b, int grid, int threads, size
 struct GradmaxScratch {
     unsigned max_bits, done, err;
 };
+cudaError_t launch_gradmax_direct(const float *u, int nx, int ny, int nz, int ldy, const Coefs &k,
+                                  int nsm, cudaStream_t stream, GradmaxScratch *sc, float *out,
+                                  unsigned *host_flags);
+// the same from TMA-staged planes
 cudaError_t configure_gradmax_single();
 cudaError_t launch_gradmax_single(const TileMaps &tm, const PlaneParams &p, dim3 grid,
                                   cudaStream_t stream, GradmaxScratch *sc, float *out,

@@ -285,6 +285,11 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b)
     return __fadd2_rn(a, make_float2(-b.x, -b.y));
 }
 
+__device__ __forceinline__ float2 half2of(const float4 &v, int h)
+{
+    return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+}
+
 // One second-difference tap in the reference's form, (u[+m] - 2u) + u[-m]
 // (CPU_function.c:393-395), two cells at a time.  Summing c2[m] times these
 // keeps a constant field's Laplacian exactly zero; the form with the centre
@@ -853,6 +858,20 @@ __global__ void __launch_bounds__(kThreads, 2)
 // launch finds zero.  The last CTA delivers the result (NaN when a wait ran
 // out) and the error flags, and leaves the scratch zero again.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void gradmax_deliver(GradmaxScratch *sc, float *out,
+                                                unsigned *host_flags)
+{
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&sc->done, 1u) != gridDim.x * gridDim.y * gridDim.z - 1) return;
+    __threadfence();
+    const unsigned flags = atomicExch(&sc->err, 0u), bits = atomicExch(&sc->max_bits, 0u);
+    atomicExch(&sc->done, 0u);
+    out[0] = flags ? __int_as_float(0x7fc00000) : __uint_as_float(bits);
+    *host_flags = flags;
+}
+
 __global__ void __launch_bounds__(kQuadsY * kGradmaxTileX, 4)
     qp3d_gradmax_single_kernel(const __grid_constant__ TileMaps tm, const PlaneParams p,
                                GradmaxScratch *sc, float *out, unsigned *host_flags)
@@ -866,15 +885,83 @@ __global__ void __launch_bounds__(kQuadsY * kGradmaxTileX, 4)
                                         kRadius + blockIdx.y * p.tile_x, z0, z1, smem, mx);
         if ((threadIdx.x & 31) == 0 && mx > 0.0f) atomicMax(&sc->max_bits, __float_as_uint(mx));
     }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    __threadfence();
-    if (atomicAdd(&sc->done, 1u) != gridDim.x * gridDim.y * gridDim.z - 1) return;
-    __threadfence();
-    const unsigned flags = atomicExch(&sc->err, 0u), bits = atomicExch(&sc->max_bits, 0u);
-    atomicExch(&sc->done, 0u);
-    out[0] = flags ? __int_as_float(0x7fc00000) : __uint_as_float(bits);
-    *host_flags = flags;
+    gradmax_deliver(sc, out, host_flags);
+}
+
+// The same without staging: a thread marches along z with one quad, its own
+// column of eleven planes in registers (the loop is unrolled by eleven, so that
+// the queue never moves), and takes the x and y taps through L1: fifteen
+// 16-byte loads a quad and plane instead of the staged form's 25 from shared
+// memory, and no barriers or copies to wait for on a small grid.
+constexpr int kDirectThreads = 128;   // 8 quads by 16 rows
+__global__ void __launch_bounds__(kDirectThreads, 4)
+    qp3d_gradmax_direct_kernel(const float *u, int nx, int ny, int nz, int ldy, int chunk_z,
+                               const __grid_constant__ Coefs k, GradmaxScratch *sc, float *out,
+                               unsigned *host_flags)
+{
+    constexpr int N = 2 * kRadius + 1;
+    const int q = threadIdx.x & 7, x = kRadius + blockIdx.y * (kDirectThreads / 8) + (threadIdx.x >> 3);
+    const int y = blockIdx.x * kTileY + 4 * q;
+    const int z0 = kRadius + blockIdx.z * chunk_z, z1 = min(z0 + chunk_z, nz - kRadius);
+    float mx = 0.0f;
+    unsigned okb = 0;   // bits of the quad's updated cells
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (y + j >= kRadius && y + j < ny - kRadius) okb |= 1u << j;
+    if (okb && x < nx - kRadius) {
+        const size_t plane = (size_t)nx * ldy;
+        const float *c = u + (size_t)z0 * plane + (size_t)x * ldy + y;   // the current plane's quad
+        auto ld = [](const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); };
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 zq[N];   // slot (z - z0 + 5 + d) % 11 holds plane z + d
+#pragma unroll
+        for (int i = 0; i < 2 * kRadius; ++i)
+            zq[i] = ld(c + (ptrdiff_t)(i - kRadius) * (ptrdiff_t)plane);
+        for (int t0 = z0; t0 < z1; t0 += N) {
+#pragma unroll
+            for (int t = 0; t < N; ++t) {
+                if (t0 + t >= z1) break;
+                zq[(t + 2 * kRadius) % N] = ld(c + kRadius * plane);
+                float Y[20];
+#pragma unroll
+                for (int b = 0; b < 5; ++b) {
+                    const int yb = y - 8 + 4 * b;
+                    const float4 v = b == 2 ? zq[(t + kRadius) % N]
+                                   : yb >= 0 && yb < ldy ? ld(c - 8 + 4 * b) : zero;
+                    Y[4 * b] = v.x; Y[4 * b + 1] = v.y; Y[4 * b + 2] = v.z; Y[4 * b + 3] = v.w;
+                }
+                float2 gx[2], gy[2], gz[2];
+#pragma unroll
+                for (int m = 0; m < kRadius; ++m) {
+                    const float4 xp = ld(c + (m + 1) * ldy), xm = ld(c - (m + 1) * ldy);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int j0 = 8 + 2 * h;
+                        const float2 dx = sub2(half2of(xp, h), half2of(xm, h));
+                        const float2 dy = sub2(f2(Y[j0 + m + 1], Y[j0 + m + 2]),
+                                               f2(Y[j0 - m - 1], Y[j0 - m]));
+                        const float2 dz = sub2(half2of(zq[(t + kRadius + m + 1) % N], h),
+                                               half2of(zq[(t + kRadius - m - 1) % N], h));
+                        gx[h] = m == 0 ? __fmul2_rn(k.cx2[0], dx) : __ffma2_rn(k.cx2[m], dx, gx[h]);
+                        gy[h] = m == 0 ? __fmul2_rn(k.cy2[0], dy) : __ffma2_rn(k.cy2[m], dy, gy[h]);
+                        gz[h] = m == 0 ? __fmul2_rn(k.cz2[0], dz) : __ffma2_rn(k.cz2[m], dz, gz[h]);
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if ((okb >> (2 * h)) & 1u)
+                        mx = fmaxf(mx, fmaxf(fabsf(gx[h].x), fmaxf(fabsf(gy[h].x), fabsf(gz[h].x))));
+                    if ((okb >> (2 * h + 1)) & 1u)
+                        mx = fmaxf(mx, fmaxf(fabsf(gx[h].y), fmaxf(fabsf(gy[h].y), fabsf(gz[h].y))));
+                }
+                c += plane;
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0 && mx > 0.0f) atomicMax(&sc->max_bits, __float_as_uint(mx));
+    gradmax_deliver(sc, out, host_flags);
 }
 
 // ---------------------------------------------------------------------------
@@ -893,11 +980,6 @@ struct PmlOwn {   // what a PML quad reads of its split-field state
 struct PmlNew {
     float2 w13[2], w21[2], w33[2], p3[2];
 };
-
-__device__ __forceinline__ float2 half2of(const float4 &v, int h)
-{
-    return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
-}
 
 template <int AX>
 __device__ __forceinline__ float2 pml_pair(float2 na1, float2 a2, float2 a3, float2 dd, float2 KS,
@@ -2744,6 +2826,21 @@ cudaError_t launch_step(const TileMaps &tm, const PlaneParams &p, dim3 grid, siz
 cudaError_t configure_gradmax_single()
 {
     return set_smem(qp3d_gradmax_single_kernel, 200 * 1024);
+}
+
+cudaError_t launch_gradmax_direct(const float *u, int nx, int ny, int nz, int ldy, const Coefs &k,
+                                  int nsm, cudaStream_t stream, GradmaxScratch *sc, float *out,
+                                  unsigned *host_flags)
+{
+    const int rows = kDirectThreads / 8, ncz = nz - 2 * kRadius;
+    const unsigned nyt = (ny - kRadius - 1) / kTileY + 1;
+    const unsigned nxt = (nx - 2 * kRadius + rows - 1) / rows;
+    const int n = plan_chunks((long long)nyt * nxt, ncz, kDirectThreads, 0, nsm);
+    const int chunk = (ncz + n - 1) / n;
+    const unsigned nch = (ncz + chunk - 1) / chunk;
+    qp3d_gradmax_direct_kernel<<<dim3(nyt, nxt, nch), kDirectThreads, 0, stream>>>(
+        u, nx, ny, nz, ldy, chunk, k, sc, out, host_flags);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_gradmax_single(const TileMaps &tm, const PlaneParams &p, dim3 grid,

@@ -4,8 +4,8 @@
 // Some callers cannot let a library allocate device memory: a host program
 // whose framework has already reserved the whole device for its own pool, or
 // a real-time loop that forbids allocation after start-up.
-// qp3d_gradmax_noalloc serves them.  It is the gradmax kernel of the
-// library, with its scratch (the maximum, a count of finished CTAs and an
+// qp3d_gradmax_noalloc serves them.  It has the arithmetic of the library's
+// gradmax kernel, with its scratch (the maximum, a count of finished CTAs and an
 // error word) in a file-scope device variable of this translation unit
 // instead of buffers the library allocates; the caller passes the wavefield
 // and the output location.  A call is one launch and one wait: the last CTA
@@ -36,6 +36,9 @@ namespace {
 // Largest number of 32-cell x 32-row tiles per plane: nx*ny up to about 64 M
 // cells.
 constexpr unsigned kNoAllocMaxTiles = 1u << 16;
+
+// 96 MB of the 129 MB L2
+constexpr long long kDirectMaxCells = 24ll << 20;
 
 static __device__ GradmaxScratch g_noalloc_scratch;
 
@@ -170,7 +173,14 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
     p.hold_plane = g_hold_plane;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     dim3 grid(nyt, nxt, (unsigned)nch);
-    cudaError_t e = launch_gradmax_single(tm, p, grid, s, ds.sc, d_max, ds.flags);
+    // Through L1 as long as the volume stays in L2 (240x240x190: 49 us a call
+    // against 60 from staged planes), from staged planes beyond, where their
+    // loads ahead of use pay (460x460x360: 280 against 264); the hook that
+    // withholds a plane is the staged form's.
+    const bool direct = (long long)nx * ldy * nz <= kDirectMaxCells && g_hold_plane == 0;
+    cudaError_t e = direct
+        ? launch_gradmax_direct(d_u, nx, ny, nz, ldy, p.k, nsm, s, ds.sc, d_max, ds.flags)
+        : launch_gradmax_single(tm, p, grid, s, ds.sc, d_max, ds.flags);
     if (e != cudaSuccess) {
         snprintf(msg, sizeof(msg), "launch failed: %s", cudaGetErrorString(e));
         return report(err, errlen, QP3D_ERR_CUDA, msg);
