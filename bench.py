@@ -434,9 +434,9 @@ def run_gpu_arm(args, dist):
                 "step_kernel_ms": round(ms_step / n_launch, 5),
                 "threshold_overhead_ms": round(ms_grad / n_launch, 5),
                 "threshold_note": "per step: gradmax pre-pass for the first 3 steps, then the "
-                                  "resolution and deferred-cell compaction kernel and the "
-                                  "fix-up (or, when the max left the window, the exact re-run) "
-                                  "of the speculative step; last shot: "
+                                  "resolution of the speculative step (fix-up of the deferred "
+                                  "cells or, when the max left the window, the exact re-run); "
+                                  "last shot: "
                                   "%d re-runs in %d steps, max %d deferred cells per step" %
                                   (int(redo.sum()), nt, int(alt.max()))}
 

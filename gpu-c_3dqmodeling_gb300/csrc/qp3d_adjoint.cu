@@ -1,11 +1,12 @@
 // qp3d_adjoint.cu -- gradient of the L2 record misfit (qp3d_adjoint of
 // include/qp3d.h).  No counterpart in the reference.
 //
-// Operator: the forward step with its scalar operator S frozen per step and
-// cell (decision and unit normal from the forward wavefield, dependence on
-// eps and delta differentiated); with S frozen the step is linear in the
-// state (u, u_prev and the split-field PML state), and the adjoint is its
-// exact transpose (kernels qp3d_adj_a/b_kernel).  The FP64 oracle
+// Operator: the transpose of the forward step's linearization (kernels
+// qp3d_adj_a/b_kernel).  The scalar operator S is differentiated in eps, delta
+// and ("adj_live" = 1, the default) the unit normal of grad u; only its
+// threshold decision is held from the forward.  "adj_live" = 0 holds the unit
+// normal as well: the step is then linear in the state (u, u_prev and the
+// split-field PML state) and the adjoint is its exact transpose.  The FP64 oracle
 // (oracle/qp3d_adjoint.c) implements the same operator and passes
 // dot-product and finite-difference tests.
 //
@@ -28,7 +29,7 @@
 // direction of grad u, a difference of neighbouring values that BF16
 // rounding of a smooth wavefield would destroy.  With "adj_ckpt_bf16" = 0 the
 // checkpoints are FP32 and the recomputation is bit-identical to the forward.
-// Device memory: ~27 volumes plus nt (all kept) or C volumes, the checkpoints
+// Device memory: 26 volumes plus nt (all kept) or C volumes, the checkpoints
 // and nt/32 volumes of decision bits.  Gradients are summed per shot in FP32
 // on the device and added to the caller's FP64 arrays.
 #include "qp3d_ctx.h"

@@ -394,7 +394,7 @@ static bool use_spec(const qp3d_ctx *ctx, int k)
 
 // Enqueue one time step.  ev_* are optional events bracketing the main step
 // kernel (s) and the threshold overhead kernels (g: gradmax, or fix-up plus
-// the gated exact re-run).
+// the exact re-run).
 static int enqueue_step(qp3d_ctx *ctx, cudaEvent_t ev_g0, cudaEvent_t ev_g1, cudaEvent_t ev_s0,
                         cudaEvent_t ev_s1)
 {

@@ -134,8 +134,8 @@ struct PlaneParams {
                               // never loaded, so its waits run out (0: none)
     // threshold handling of the step kernel
     int spec;                 // 1: predicted window, own max, deferred cells
-    const int *gate;          // spec: set to 1 when the step has to be re-run (null: not
-                              // speculative)
+    const int *gate;          // spec: set to 1 by a column whose segment overflowed and by
+                              // the resolution of a step that is re-run (null: not spec)
     float *win;               // spec: kWinFloats of the step: M_lo, M_hi, M_pred and the
                               // thresholds of m2 at M_lo and M_hi
     int win_ready;            // 1: all five are there already
@@ -252,8 +252,8 @@ cudaError_t launch_gradmax(const TileMaps &tm, const PlaneParams &p, dim3 grid,
 cudaError_t launch_step(const TileMaps &tm, const PlaneParams &p, dim3 grid, size_t smem,
                         cudaStream_t stream);
 // resolution of a speculative step: the fix-up of its deferred cells or (when
-// the max fell outside the window) its exact re-run, a persistent grid of nsm
-// CTAs
+// the max fell outside the window or a segment overflowed) its exact re-run, a
+// persistent grid of two CTAs an SM
 cudaError_t launch_fix_or_rerun(const TileMaps &tm, const PlaneParams &p, float *spec_err,
                                 int nsm, size_t smem, cudaStream_t stream);
 cudaError_t launch_band_sources(float *u_new, const float *u_cur,

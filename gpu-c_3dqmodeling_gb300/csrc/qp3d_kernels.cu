@@ -403,7 +403,7 @@ __device__ __forceinline__ float2 div2(float2 p, float h)
 // xr::div_const_scaled in packed form.  IEEE divisions, with their slow path
 // for the subnormal values ahead of a wavefront, were 9300 of the instructions
 // a warp spent on a plane (998 us a step on 140^3; 223 with products in their
-// place).
+// place; 298 with the two forms below).
 enum TapDiv { kDivIeee, kDivConst, kDivScaled };
 
 __device__ __forceinline__ float2 div_const2(float2 p, float h, float y)
@@ -892,7 +892,9 @@ __global__ void __launch_bounds__(kQuadsY * kGradmaxTileX, 4)
 // column of eleven planes in registers (the loop is unrolled by eleven, so that
 // the queue never moves), and takes the x and y taps through L1: fifteen
 // 16-byte loads a quad and plane instead of the staged form's 25 from shared
-// memory, and no barriers or copies to wait for on a small grid.
+// memory, and no barriers or copies to wait for on a small grid.  240x240x190:
+// 49 us a call, 60 staged; held to 3, 5 or 6 CTAs an SM 59, 62 and 75 (fewer warps,
+// or spills).
 constexpr int kDirectThreads = 128;   // 8 quads by 16 rows
 __global__ void __launch_bounds__(kDirectThreads, 4)
     qp3d_gradmax_direct_kernel(const float *u, int nx, int ny, int nz, int ldy, int chunk_z,
@@ -1015,19 +1017,18 @@ __device__ __forceinline__ void cell_face(int fx, int lix, int fy, int liy, int 
 // ---------------------------------------------------------------------------
 // step kernel.
 //   SPEC = false ("exact"): the threshold comes from gmax[step], already
-//     known (gradmax kernel, or a speculative pass of the same step).  With a
-//     gate the kernel runs only when *gate != 0 (the re-run of a step whose
-//     speculation failed).
+//     known (gradmax kernel, or a speculative pass of the same step whose
+//     resolution found that it has to be re-run).
 //   SPEC = true: the max of the step is not known yet.  It is predicted from
 //     the two previous steps with a window [M_lo, M_hi]; a cell whose m2 lies
 //     in (T2(M_lo), T2(M_hi)] has an uncertain decision: the kernel computes
-//     it as "above", marks it in the deferred-cell bitmask with its m2 and
-//     S = 1 value, and reduces the true max of the step into gmax[step] on
-//     the way.  The resolution kernel then gives the
-//     S = 1 result to the marked cells that turn out to be below the
-//     threshold, or ask for the exact re-run when the max fell outside the
-//     window.  The step never overwrites its inputs, so both are possible.
-//     Both modes write bit-identical results.
+//     it as "above", lists it in its column's segment with its m2 and what
+//     gives it its S = 1 result, and reduces the true max of the step into
+//     gmax[step] on the way.  The resolution kernel then gives the S = 1
+//     result to the listed cells that turn out to be below the threshold, or
+//     runs the exact step again when the max fell outside the window or a
+//     segment was too short.  The step never overwrites its inputs, so both
+//     are possible.  Both modes write bit-identical results.
 // ---------------------------------------------------------------------------
 // w = (M_lo, M_hi, M_pred) of step k, from the maxima of the two steps before
 // and the recent prediction errors.
@@ -2332,8 +2333,10 @@ __device__ __forceinline__ void adj_derivs(const Taps &T, const Coefs &k, float 
 // per quad that gathered its 31 taps through L1 held 128 registers with
 // spills, and waited for three dependent groups of loads: 258 us on
 // 240x240x190, 50% of the DRAM peak; this form 199 us with the 80 bytes of
-// storing u_prev's adjoint and Cyy as well.)  Only updated cells are written: the
-// adjoint of the never-updated band reaches no other cell and no output.
+// storing u_prev's adjoint and Cyy as well, 189 now.  Without the stencil it
+// takes 200, without the stores of the six fields 150.)  Only updated cells are
+// written: the adjoint of the never-updated band reaches no other cell and no
+// output.
 constexpr int kAdjStreams = 15;
 constexpr int kAdjThreads = kQuadsY * kAdjTileX;
 
@@ -2606,8 +2609,9 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
 // Pass B: Nu += the transposed stencils of the six coefficient fields, over
 // the updated cells (their taps lie inside the volume; along y the rows are
 // padded to whole quads, and taps before a row's start or past its end read
-// zero).  Bound by the bytes through L1.
-//
+// zero).  Bound by the latency of its 53 16-byte loads a quad through L1:
+// 240x240x190 105 us with every cell of the volume, 89 with the updated cells
+// in 44 registers.
 __device__ __forceinline__ void fma4(float acc[4], float c, const float4 &a, const float4 &b, bool minus)
 {
 #pragma unroll
@@ -2620,7 +2624,9 @@ __device__ __forceinline__ void fma4(float acc[4], float c, const float4 &a, con
 // Cz are zero and Cyy equals Cxx (qp3d_adj_a_kernel), reads two fields.
 // Two rows by two planes of quads per thread, which needs 34 16-byte loads a
 // quad instead of 53, left 16 warps an SM and took 111 us instead of 105 on
-// 240x240x190: the pass waits for latency rather than for the bytes.
+// 240x240x190: the pass waits for latency rather than for the bytes.  Marching
+// along z with the planes of Cz and Czz in registers (33 loads a quad, 168
+// registers, 12 warps an SM) took 117 against 89 us.
 __global__ void __launch_bounds__(256) qp3d_adj_b_kernel(const AdjParams a)
 {
     pdl_trigger();

@@ -103,8 +103,8 @@ int qp3d_forward(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m,
  * depth and nt): the replacement of the main programs' loop of modeling3d
  * calls.  Records are the same, bit for bit, as qp3d_forward's for each shot.
  * All shots that fit in device memory are resident at once and every time
- * step of all of them is one launch of a persistent kernel that takes work
- * items (one tile column of one shot) from a device queue; steps after the
+ * step of all of them is one launch with a CTA per work item (one tile column
+ * of one shot) and one that resolves the step's threshold; steps after the
  * first three are replayed from a captured CUDA graph.  The tile height and
  * the number of z blocks per column are chosen by timing a few candidate
  * shapes on the first steps of the run (results do not depend on the shape;
@@ -134,7 +134,7 @@ typedef struct {
     int graph_steps;      /* steps replayed from the captured graph */
     int redo_steps;       /* shot-steps whose speculation missed (re-run) */
     int work_items;       /* work items per launch (last group) */
-    int ctas;             /* persistent CTAs per launch (last group) */
+    int ctas;             /* persistent CTAs of the resolution (last group) */
     float run_ms;         /* device time of the time loop, summed over groups */
 } qp3d_batch_stats;
 int qp3d_batch_get_stats(const qp3d_ctx *ctx, qp3d_batch_stats *out);
@@ -198,7 +198,7 @@ int qp3d_shot_read_stats(qp3d_ctx *ctx, int k0, int nsteps, int *redo,
 /* Device timing of nsteps further steps with CUDA events on the context's
  * stream.  ms_total: whole interval; ms_step: sum of the fused step kernel's
  * launch durations; ms_gradmax: sum of the threshold overhead per step (the
- * gradmax pre-pass, or the fix-up and gated re-run of a speculative step).
+ * gradmax pre-pass, or the fix-up or exact re-run of a speculative step).
  * NULL per-kernel pointers skip the per-kernel events. */
 int qp3d_shot_time(qp3d_ctx *ctx, int nsteps, float *ms_total, float *ms_step,
                    float *ms_gradmax);
