@@ -2626,7 +2626,8 @@ __device__ __forceinline__ void fma4(float acc[4], float c, const float4 &a, con
 // quad instead of 53, left 16 warps an SM and took 111 us instead of 105 on
 // 240x240x190: the pass waits for latency rather than for the bytes.  Marching
 // along z with the planes of Cz and Czz in registers (33 loads a quad, 168
-// registers, 12 warps an SM) took 117 against 89 us.
+// registers, 12 warps an SM) took 117 against 89 us; CTAs of 16 rows by 2 planes
+// 92, 8 by 4 95, 4 by 8 104, although they halve what misses L1.
 __global__ void __launch_bounds__(256) qp3d_adj_b_kernel(const AdjParams a)
 {
     pdl_trigger();
