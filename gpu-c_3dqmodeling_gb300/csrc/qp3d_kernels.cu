@@ -1361,7 +1361,18 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
     unsigned *misc_u = reinterpret_cast<unsigned *>(smem + L.misc_off + 16);
 
     const int tid = threadIdx.x, lane = tid & 31;
-    const int q = tid & (kQuadsY - 1), r = tid / kQuadsY;
+    // A warp holds four rows of eight quads, or, in a last y tile of no more
+    // than four, two or one quads, eight, sixteen or 32 rows: the warps left
+    // over only pass the planes on.  (Decision words and the reference
+    // arithmetic's classes go by rows of eight.)  A step of 140^3 cells (last
+    // tile 12 wide) 45.3 -> 42.5 us, 38x42x34 10.5 -> 10.1, 191x127x105 (31
+    // wide) 35.7 -> 35.1, 240x240x190 (16) 107.5 -> 106.4.
+    int lq = 3;
+    if (AR == kArithFast && !DEC) {
+        const int nq = (min(p.ny - y0, kTileY) + 3) >> 2;
+        lq = nq > 4 ? 3 : (nq > 2 ? 2 : nq - 1);
+    }
+    const int q = tid & ((1 << lq) - 1), r = tid >> lq, rt = min(r, tile_x - 1);
     const int nzc = z1 - z0;
     Pipe<kGroups> P;
     pipe_setup(P, smem, L, tile_x, y0, x0, z0, nzc);
@@ -1372,6 +1383,7 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
     // quads wholly in the row padding (y >= ny, the last y tile) neither load
     // nor store: their cells are not part of the volume
     const bool mem_ok = row_ok && (yq < ny);
+    const bool idle = !__any_sync(0xffffffffu, mem_ok);   // warps without a cell
     // bits per cell of the quad: updated; of a y face
     unsigned okb = 0, fyb = 0;
 #pragma unroll
@@ -1380,7 +1392,7 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
         if (row_ok && y >= kRadius && y < ny - kRadius) okb |= 1u << j;
         if (y < pml || y >= ny - pml) fyb |= 1u << j;
     }
-    Taps T = taps_start(P, r, q);
+    Taps T = taps_start(P, rt, q);
     // the x face part, constant along z
     const int fx = x < pml ? 0 : (x >= nx - pml ? 1 : -1);
     const int lix = x < pml ? pml - x : x - nx + pml;
@@ -1698,11 +1710,15 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
     for (int t = 0; t < nzc; taps_next(T, P, t), ++t, base += plane) {
         ok = __all_sync(0xffffffffu, pipe_wait(P, t));   // warps stay converged for the collectives below
         if (!ok) break;
+        if (idle) {
+            pipe_release(P, tm, t);
+            continue;
+        }
         if (AR == kArithRef) {
             if (t == 0)
                 for (int i = 0; i < 2 * kRadius; ++i) zhist = (zhist << 2) | window_class(ztap(T, i));
             zhist = (zhist << 2) | window_class(ztap(T, 2 * kRadius));
-            unsigned cls = halo_class(T.pc - ((r + kRadius) * kBoxY + kHaloY + 4 * q), r & ~3, tile_x);
+            unsigned cls = halo_class(T.pc - ((rt + kRadius) * kBoxY + kHaloY + 4 * q), r & ~3, tile_x);
             if (row_ok) cls |= ((zhist & 0x155555u) ? 1u : 0u) | ((zhist & 0x2aaaaau) ? 2u : 0u);
             cls = k.div_ok ? __reduce_or_sync(0xffffffffu, cls) : 2u;
             if (cls == 0) quad_derivs_ref(T, k, Ux, Uy, Uz, Uxx, Uyy, Uzz, u0);
