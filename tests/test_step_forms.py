@@ -47,10 +47,11 @@ def _check(ctx, shot, u_prev, u_cur, pml_state, arith):
 @pytest.mark.parametrize("arith", [1, 0])
 @pytest.mark.parametrize("hx,hy,nz0,pml,tile_x,chunks", [
     (31, 23, 14, 6, 0, 0),      # 43 x 35 x 26: 33 updated rows, shells of 6
-    (18, 19, 17, 7, 32, 1),     # 32 x 33 x 31: one quad of one cell in the last y tile
+    (18, 19, 17, 7, 32, 1),     # 32 x 33 x 31: one quad, of one cell, in the last y tile
     (29, 53, 13, 5, 16, 13),    # 39 x 63 x 23: one plane a chunk, shells of 5
     (40, 25, 22, 0, 11, 2),     # 40 x 25 x 22: no shell
-    (16, 90, 16, 9, 24, 3)])
+    (16, 90, 16, 9, 24, 3),     # 34 x 108 x 34: three quads in the last y tile
+    (37, 26, 15, 6, 0, 0)])     # 49 x 38 x 27: two
 def test_tile_edges(sctx, hx, hy, nz0, pml, tile_x, chunks, arith):
     shot = synthetic.small_case(hx=hx, hy=hy, nz0=nz0, pml=pml, nt=NT, seed=61,
                                 src=(hx // 2, hy // 2, nz0 // 2))
