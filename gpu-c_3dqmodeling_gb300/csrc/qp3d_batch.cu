@@ -245,7 +245,7 @@ int Runner::build_candidate(int c, std::vector<Plan *> &G)
             if (rc) return rc;
         }
     }
-    // longest columns first: the queue hands them out before the short ones
+    // longest columns first: they start before the short ones
     std::stable_sort(items.begin(), items.end(), [](const WorkItem &a, const WorkItem &b) {
         return (a.z1 - a.z0) > (b.z1 - b.z0);
     });
