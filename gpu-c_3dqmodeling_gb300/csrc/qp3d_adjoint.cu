@@ -110,7 +110,8 @@ int alloc_state(qp3d_ctx *ctx, AdjState *s, int C, int nck, int bf16, int keep, 
     for (auto *&p : s->g) CK(cudaMalloc(&p, vb));
     CK(cudaMalloc(&s->seg, vb * C));
     // the row padding of a wavefield is never written by a step: zero it once
-    CK(cudaMemset(s->seg, 0, vb * C));
+    // (on the steps' stream, which does not wait for the default stream)
+    CK(cudaMemsetAsync(s->seg, 0, vb * C, ctx->stream));
     const size_t per = (size_t)s->vol * (bf16 ? 2 * sizeof(float) + 7 * sizeof(__nv_bfloat16)
                                               : 9 * sizeof(float));
     if (nck) CK(cudaMalloc(&s->ck, per * nck));
@@ -119,7 +120,7 @@ int alloc_state(qp3d_ctx *ctx, AdjState *s, int C, int nck, int bf16, int keep, 
     if (nck) {   // one bit per cell and step: the forward's threshold decisions
         const size_t db = (size_t)s->nt * (size_t)(s->vol / 32) * sizeof(unsigned);
         CK(cudaMalloc(&s->dec, db));
-        CK(cudaMemset(s->dec, 0, db));
+        CK(cudaMemsetAsync(s->dec, 0, db, ctx->stream));
     }
     CK(cudaMalloc(&s->misfit, sizeof(double)));
     s->C = C;
