@@ -51,6 +51,10 @@ int qp3d_internal_restore_wavefields(qp3d_ctx *ctx, float *const U[3]);
 namespace qp3d {
 
 struct AdjState {
+    // the shape the buffers were made for.  Equal volumes are not enough: the
+    // record's size follows the shell, and the outer planes of a kept u^k, which
+    // no step writes, lie elsewhere in another shape.
+    int nx = 0, ny = 0, nz = 0, pml = 0;
     long long vol = 0;
     int nt = 0, C = 0, nck = 0, bf16 = 1, keep = 0;
     // adjoint of u: this step's, the step after's, the step before's; the seven
@@ -154,7 +158,8 @@ extern "C" int qp3d_adjoint(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model 
     const size_t vb = (size_t)vol * sizeof(float);
     // state buffers, reused when the geometry and the schedule repeat
     AdjState *&S = ctx->adj;
-    if (S && (S->vol != vol || S->nt != nt || S->bf16 != ctx->adj_bf16 ||
+    if (S && (S->nx != g->nx || S->ny != g->ny || S->nz != g->nz || S->pml != g->pml ||
+              S->nt != nt || S->bf16 != ctx->adj_bf16 ||
               (ctx->adj_keep >= 0 && S->keep != ctx->adj_keep))) {
         adjoint_free(S);
         S = nullptr;
@@ -172,6 +177,10 @@ extern "C" int qp3d_adjoint(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model 
     if (!S) {
         S = new (std::nothrow) AdjState();
         if (!S) return ctx_fail(ctx, QP3D_ERR_NOMEM, "out of host memory");
+        S->nx = g->nx;
+        S->ny = g->ny;
+        S->nz = g->nz;
+        S->pml = g->pml;
         S->vol = vol;
         S->nt = nt;
         if ((rc = alloc_state(ctx, S, C, nck, ctx->adj_bf16, keep, rec))) {
