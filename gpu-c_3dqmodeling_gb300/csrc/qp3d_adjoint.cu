@@ -43,6 +43,7 @@
 using namespace qp3d;
 
 // qp3d_api.cu
+int qp3d_internal_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m);
 int qp3d_internal_enqueue_step(qp3d_ctx *ctx);
 int qp3d_internal_restore_step(qp3d_ctx *ctx, int step);
 int qp3d_internal_bind_wavefields(qp3d_ctx *ctx, float *u_prev, float *u_cur, float *u_next);
@@ -143,7 +144,8 @@ extern "C" int qp3d_adjoint(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model 
     if (!ctx) return QP3D_ERR_ARG;
     if (!g || !m || !d_obs) return ctx_fail(ctx, QP3D_ERR_ARG, "missing input");
     if (ctx->param_fp16) return ctx_fail(ctx, QP3D_ERR_ARG, "qp3d_adjoint needs FP32 parameters");
-    int rc = qp3d_shot_load(ctx, g, m);
+    const StreamDrain drain{ctx};   // for m's volumes and d_obs
+    int rc = qp3d_internal_load(ctx, g, m);
     if (rc) return rc;
     if (!ctx->fuse_sources || ctx->n_band > 0 || !ctx->rec_fused)
         return ctx_fail(ctx, QP3D_ERR_ARG,

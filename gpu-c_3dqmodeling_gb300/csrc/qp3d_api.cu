@@ -99,6 +99,7 @@ extern "C" int qp3d_ctx_create(int device, qp3d_ctx **out)
         return QP3D_ERR_CUDA;
     }
     for (auto &ev : ctx->ev) cudaEventCreate(&ev);
+    cudaEventCreateWithFlags(&ctx->load_ev, cudaEventDisableTiming);
     for (auto &ev : ctx->uev) cudaEventCreate(&ev);
     void *fn = nullptr;
     cudaDriverEntryPointQueryResult q;
@@ -133,6 +134,7 @@ extern "C" void qp3d_ctx_destroy(qp3d_ctx *ctx)
     }
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->copy_ev) cudaEventDestroy(ctx->copy_ev);
+    if (ctx->load_ev) cudaEventDestroy(ctx->load_ev);
     for (auto &ev : ctx->ev)
         if (ev) cudaEventDestroy(ev);
     for (auto &ev : ctx->uev)
@@ -223,9 +225,11 @@ static int download_vol(qp3d_ctx *ctx, float *dst, const float *src)
     return QP3D_OK;
 }
 
-extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m)
+// The load without its last wait, for the calls that wait for the context's
+// stream before they return (StreamDrain): the device may still be reading m's
+// volumes (page-locked ones).
+int qp3d_internal_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m)
 {
-    if (!ctx) return QP3D_ERR_ARG;
     int rc = check_geom(ctx, g);
     if (rc) return rc;
     if (!m || !m->vp || !m->epsilon || !m->delta || !m->wavelet || !m->c || !m->c2)
@@ -309,7 +313,7 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
     // coefficient tables
     derive_coefs(m->c, m->c2, g->dx, g->dy, g->dz, &ctx->coefs);
     if (g->pml > 0) {
-        std::vector<float4> &tab = ctx->layers_host;   // the copy may still read it on return
+        std::vector<float4> &tab = ctx->layers_host;   // outlives the copy
         tab.resize(3 * g->pml);
         derive_layers(m->dlr, m->ddlr, g->pml, g->dt, tab.data());
         derive_layers(m->dfb, m->ddfb, g->pml, g->dt, tab.data() + g->pml);
@@ -319,7 +323,10 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
     }
     ctx->wavelet.assign(m->wavelet, m->wavelet + g->nt);
     // sparse source: every non-zero sample (CPU_function.c:326-338 adds all)
-    std::vector<SrcEntry> fused, band, all;
+    std::vector<SrcEntry> &fused = ctx->host_fused, &band = ctx->host_band, &all = ctx->host_all;
+    fused.clear();
+    band.clear();
+    all.clear();
     if (m->source) scan_source_volume(m->source, g->nx, g->ny, g->nz, all);
     for (const SrcEntry &e : all) {
         const bool inside = e.x >= kRadius && e.x < g->nx - kRadius && e.y >= kRadius &&
@@ -340,7 +347,8 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
             CK(cudaMalloc(d, v.size() * sizeof(SrcEntry)));
             *cap = v.size();
         }
-        CK(cudaMemcpy(*d, v.data(), v.size() * sizeof(SrcEntry), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(*d, v.data(), v.size() * sizeof(SrcEntry), cudaMemcpyHostToDevice,
+                           ctx->stream));
         return QP3D_OK;
     };
     if (ctx->fuse_sources) {
@@ -358,8 +366,19 @@ extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_mode
     if ((rc = ensure_defer(ctx))) return rc;
     for (int i = 0; i < 3; ++i)
         if ((rc = make_tmap(ctx, ctx->U[i], &ctx->tm[i]))) return rc;
+    CK(cudaEventRecord(ctx->load_ev, ctx->stream));   // the inputs have been read
     ctx->loaded = true;
     return qp3d_shot_reset(ctx);
+}
+
+extern "C" int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m)
+{
+    if (!ctx) return QP3D_ERR_ARG;
+    const int rc = qp3d_internal_load(ctx, g, m);
+    // the caller may write the next model into its buffers, or free them, after this
+    if (rc) (void)cudaStreamSynchronize(ctx->stream);
+    else CK(cudaEventSynchronize(ctx->load_ev));
+    return rc;
 }
 
 extern "C" int qp3d_shot_reset(qp3d_ctx *ctx)
@@ -886,7 +905,8 @@ extern "C" int qp3d_forward(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model 
                             const qp3d_snap *snap)
 {
     if (!ctx || !record) return QP3D_ERR_ARG;
-    int rc = qp3d_shot_load(ctx, g, m);
+    const StreamDrain drain{ctx};   // for m's volumes
+    int rc = qp3d_internal_load(ctx, g, m);
     if (rc) return rc;
     // A page-locked record buffer is filled while the time loop runs: the
     // planes of each finished piece of steps go to the host on a second

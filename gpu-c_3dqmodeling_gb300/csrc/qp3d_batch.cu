@@ -524,6 +524,7 @@ extern "C" int qp3d_batch(qp3d_ctx *ctx, int nshots, const qp3d_shot *shots)
     if (nshots < 0 || (nshots > 0 && !shots)) return ctx_fail(ctx, QP3D_ERR_ARG, "bad shot list");
     CK(cudaSetDevice(ctx->device));
     CK(cudaStreamSynchronize(ctx->stream));
+    const StreamDrain drain{ctx};   // for the shots' volumes
     if (!ctx->batch) ctx->batch = new (std::nothrow) BatchState();
     if (!ctx->batch) return ctx_fail(ctx, QP3D_ERR_NOMEM, "out of host memory");
     BatchState *B = ctx->batch;

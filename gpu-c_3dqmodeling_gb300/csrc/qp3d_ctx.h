@@ -66,7 +66,10 @@ struct qp3d_ctx {
     qp3d::SrcEntry *src_fused = nullptr, *src_band = nullptr, *src_all = nullptr;
     int n_fused = 0, n_band = 0, n_all = 0;
     size_t cap_fused = 0, cap_band = 0, cap_all = 0;   // entries allocated
+    // sources of the load's copies, and the event behind the last of them
     std::vector<float4> layers_host;
+    std::vector<qp3d::SrcEntry> host_fused, host_band, host_all;
+    cudaEvent_t load_ev = nullptr;
     bool fuse_sources = true;
     unsigned *errword = nullptr;
     qp3d::TileMaps tm[3];
@@ -131,6 +134,13 @@ struct qp3d_ctx {
     int adj_keep = -1;               // 1: keep every u^k, 0: checkpoints, -1: by free memory
     int adj_live = 1;                // 1: gradient of the live operator (dS/du included), 0: S frozen
 };
+// For a call that hands the caller's buffers to asynchronous copies: none may be
+// read or written after the call has returned, also on an error.
+struct StreamDrain {
+    qp3d_ctx *ctx;
+    ~StreamDrain() { (void)cudaStreamSynchronize(ctx->stream); }
+};
+
 inline int ctx_fail(qp3d_ctx *c, int code, const char *fmt, ...)
 {
     if (c) {

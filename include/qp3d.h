@@ -166,7 +166,9 @@ int qp3d_adjoint(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m,
                  const float *d_obs, double *grad_vp, double *grad_eps,
                  double *grad_del, double *misfit);
 
-/* Staged form of the same shot. */
+/* Staged form of the same shot.  qp3d_shot_load has read the model when it
+ * returns, page-locked volumes too (as qp3d_forward, qp3d_adjoint and
+ * qp3d_batch have): the caller may then write the next one into them. */
 int qp3d_shot_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m);
 int qp3d_shot_reset(qp3d_ctx *ctx);                 /* zero state, step 0 */
 int qp3d_shot_advance(qp3d_ctx *ctx, int nsteps);   /* enqueue, asynchronous */
