@@ -706,7 +706,11 @@ extern "C" int qp3d_shot_write_state(qp3d_ctx *ctx, int step, const float *u_pre
                         tmp[(size_t)z * ctx->plane + (size_t)x * ctx->ldy + y] =
                             pml_state[L.off[f][a] + fi];
                     }
-            CK(cudaMemcpy(arr[a], tmp.data(), tmp.size() * sizeof(float), cudaMemcpyHostToDevice));
+            // on the steps' stream, which does not wait for the default stream;
+            // tmp is filled again
+            CK(cudaMemcpyAsync(arr[a], tmp.data(), tmp.size() * sizeof(float),
+                               cudaMemcpyHostToDevice, ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
         }
     }
     CK(cudaStreamSynchronize(ctx->stream));
