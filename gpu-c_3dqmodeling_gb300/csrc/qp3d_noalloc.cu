@@ -157,7 +157,12 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
     }
 
     TileMaps tm;
-    if (encode_tile_maps(g_encode, d_u, nx, ny, nz, ldy, tile_x, &tm) != CUDA_SUCCESS)
+    CUresult cr = encode_tile_maps(g_encode, d_u, nx, ny, nz, ldy, tile_x, &tm);
+    if (cr == CUDA_ERROR_INVALID_CONTEXT) {   // a host thread that has used no CUDA yet
+        (void)cudaFree(nullptr);              // gives it the device's context
+        cr = encode_tile_maps(g_encode, d_u, nx, ny, nz, ldy, tile_x, &tm);
+    }
+    if (cr != CUDA_SUCCESS)
         return report(err, errlen, QP3D_ERR_CUDA, "cuTensorMapEncodeTiled failed");
 
     PlaneParams p;
