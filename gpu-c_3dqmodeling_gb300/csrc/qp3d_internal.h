@@ -320,7 +320,7 @@ cudaError_t launch_batch_resolve(const BatchArgs &b, int grid, int threads, size
                                  cudaStream_t stream);
 // max|grad u| in one launch: sc starts zero and is left zero, out receives the
 // maximum (NaN on a timed-out wait) and *host_flags (mapped) the error bits.
-struct GradmaxScratch {
+struct alignas(64) GradmaxScratch {
     unsigned max_bits, done, err;
 };
 cudaError_t launch_gradmax_direct(const float *u, int nx, int ny, int nz, int ldy, const Coefs &k,

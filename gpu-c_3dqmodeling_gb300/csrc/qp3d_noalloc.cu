@@ -14,14 +14,17 @@
 // over partial maxima and a copy of the flags).
 //
 // The scratch exists once per device that loads the library and is held until
-// the process exits.  Every call shares it and leaves it zero, so calls that
-// overlap on the GPU (different streams, or host threads without ordering)
-// race.  The call waits for its stream before it returns, so that a bounded
-// device wait that ran out is reported as QP3D_ERR_TIMEOUT.
+// the process exits: kSlots entries, one for each call under way.  A call waits
+// for its stream before it returns (so that a bounded device wait that ran out
+// is reported as QP3D_ERR_TIMEOUT) and keeps its entry until then, so host
+// threads may call at the same time; the last CTA leaves the entry zero for the
+// next call.  (One entry for all: two calls whose kernels overlapped could each
+// miss the last of its CTAs, and the count stayed wrong for the process.)
 #include "qp3d.h"
 #include "qp3d_internal.h"
 
 #include <algorithm>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -40,16 +43,43 @@ constexpr unsigned kNoAllocMaxTiles = 1u << 16;
 // 96 MB of the 129 MB L2
 constexpr long long kDirectMaxCells = 24ll << 20;
 
-static __device__ GradmaxScratch g_noalloc_scratch;
+constexpr int kSlots = 32;       // a bit each in DeviceScratch::busy
+constexpr int kFlagStride = 16;  // a 64-byte line each
+static __device__ GradmaxScratch g_noalloc_scratch[kSlots];
 
 struct DeviceScratch {
     bool ready;
     GradmaxScratch *sc;
-    unsigned *flags;      // mapped host word
+    unsigned *flags;      // mapped host words
+    unsigned busy;
 };
 constexpr int kMaxDevices = 64;
 DeviceScratch g_dev[kMaxDevices];
 std::mutex g_mutex;
+std::condition_variable g_slot_free;
+
+// A call's entry of its device's scratch, from its launch to the end of its
+// wait; with all of them taken the call waits for one.
+struct Slot {
+    DeviceScratch &d;
+    int i = 0;
+    explicit Slot(DeviceScratch &dev) : d(dev)
+    {
+        std::unique_lock<std::mutex> lock(g_mutex);
+        g_slot_free.wait(lock, [&] { return d.busy != ~0u; });
+        while (d.busy >> i & 1u) ++i;
+        d.busy |= 1u << i;
+    }
+    ~Slot()
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        d.busy &= ~(1u << i);
+        g_slot_free.notify_all();
+    }
+    GradmaxScratch *scratch() const { return d.sc + i; }
+    unsigned *flags() const { return d.flags + kFlagStride * i; }
+};
+static_assert(kSlots == 32, "one bit of busy each");
 
 EncodeTiledFn g_encode = nullptr;
 
@@ -126,7 +156,6 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
     // once per device, with that device current: the scratch addresses and
     // the kernel's shared-memory limit.  The first call on a device does this
     // set-up; make it before any stream capture.
-    DeviceScratch ds;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         if (!g_encode) {
@@ -146,14 +175,13 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
                 return report(err, errlen, QP3D_ERR_CUDA, "cudaGetSymbolAddress failed");
             if (configure_gradmax_single() != cudaSuccess)
                 return report(err, errlen, QP3D_ERR_CUDA, "cannot set the kernel's shared memory");
-            if (cudaHostAlloc((void **)&flags, sizeof(unsigned),
+            if (cudaHostAlloc((void **)&flags, kSlots * kFlagStride * sizeof(unsigned),
                               cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
-                return report(err, errlen, QP3D_ERR_NOMEM, "cannot allocate the host flag word");
+                return report(err, errlen, QP3D_ERR_NOMEM, "cannot allocate the host flag words");
             d.sc = sc;
             d.flags = flags;
             d.ready = true;
         }
-        ds = d;
     }
 
     TileMaps tm;
@@ -173,7 +201,8 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
     p.plane = (long long)nx * ldy;
     derive_coefs(c, c, dx, dy, dz, &p.k);   // first-derivative weights only
     p.arith = kArithFast;   // the library's default arithmetic
-    p.err = &ds.sc->err;
+    const Slot slot(g_dev[dev]);
+    p.err = &slot.scratch()->err;
     p.wait_ns = g_wait_ns;
     p.hold_plane = g_hold_plane;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -184,8 +213,9 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
     // withholds a plane is the staged form's.
     const bool direct = (long long)nx * ldy * nz <= kDirectMaxCells && g_hold_plane == 0;
     cudaError_t e = direct
-        ? launch_gradmax_direct(d_u, nx, ny, nz, ldy, p.k, nsm, s, ds.sc, d_max, ds.flags)
-        : launch_gradmax_single(tm, p, grid, s, ds.sc, d_max, ds.flags);
+        ? launch_gradmax_direct(d_u, nx, ny, nz, ldy, p.k, nsm, s, slot.scratch(), d_max,
+                                slot.flags())
+        : launch_gradmax_single(tm, p, grid, s, slot.scratch(), d_max, slot.flags());
     if (e != cudaSuccess) {
         snprintf(msg, sizeof(msg), "launch failed: %s", cudaGetErrorString(e));
         return report(err, errlen, QP3D_ERR_CUDA, msg);
@@ -196,7 +226,7 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
         snprintf(msg, sizeof(msg), "%s", cudaGetErrorString(e));
         return report(err, errlen, QP3D_ERR_CUDA, msg);
     }
-    const unsigned flags = *const_cast<volatile unsigned *>(ds.flags);
+    const unsigned flags = *const_cast<volatile unsigned *>(slot.flags());
     if (flags) return report(err, errlen, QP3D_ERR_TIMEOUT, "a device wait timed out");
     return QP3D_OK;
 }

@@ -273,8 +273,9 @@ void qp3d_host_free(void *p);
  * (nx*ny up to about 64 M cells), and at most 65535 tiles along x and z
  * chunks; larger grids return QP3D_ERR_ARG.
  * Its scratch is a fixed device array that every GPU loading the library
- * holds until exit and that all calls share: calls that overlap on the GPU
- * race.  The first call on each device sets up the scratch addresses and the
+ * holds until exit, with an entry for each of up to 32 calls under way on the
+ * device (further ones wait for an entry): host threads may call at the same
+ * time.  The first call on each device sets up the scratch addresses and the
  * kernel attributes; make it before any stream capture.  Test hooks, set with
  * qp3d_tune(NULL, key, value): "noalloc_wait_limit_us" (limit of the bounded
  * waits, 0: 2 s) and "noalloc_test_hold_plane" (a plane the first CTA never
