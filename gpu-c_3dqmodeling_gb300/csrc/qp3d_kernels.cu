@@ -877,12 +877,15 @@ __global__ void __launch_bounds__(kQuadsY * kGradmaxTileX, 4)
                                GradmaxScratch *sc, float *out, unsigned *host_flags)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    // tiles of a plane in the grid's first dimension, which has no limit of 65535
+    const int nyt = (p.ny - kRadius - 1) / kTileY + 1;
+    const int yt = blockIdx.x % nyt, xt = blockIdx.x / nyt;
     const int z0 = kRadius + blockIdx.z * p.chunk_z;
     const int z1 = min(z0 + p.chunk_z, p.nz - kRadius);
     if (z0 < z1) {
         float mx;
-        gradmax_tile<false, kArithFast>(&tm, p, p.k, p.tile_x, blockIdx.x * kTileY,
-                                        kRadius + blockIdx.y * p.tile_x, z0, z1, smem, mx);
+        gradmax_tile<false, kArithFast>(&tm, p, p.k, p.tile_x, yt * kTileY,
+                                        kRadius + xt * p.tile_x, z0, z1, smem, mx);
         if ((threadIdx.x & 31) == 0 && mx > 0.0f) atomicMax(&sc->max_bits, __float_as_uint(mx));
     }
     gradmax_deliver(sc, out, host_flags);

@@ -134,7 +134,8 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
     const int nxt = (ncx + tile_x - 1) / tile_x;
     const int nyt = (ny - kRadius - 1) / kTileY + 1;
     const long long tiles = (long long)nxt * nyt;
-    const long long tiles32 = (long long)((ncx + 31) / 32) * nyt;
+    const int nxt32 = (ncx + 31) / 32;
+    const long long tiles32 = (long long)nxt32 * nyt;
     if (tiles32 > kNoAllocMaxTiles) {
         snprintf(msg, sizeof(msg),
                  "grid %dx%d needs %lld tiles per z chunk; qp3d_gradmax_noalloc holds at most %u",
@@ -144,12 +145,13 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
     long long nch = plan_chunks(tiles, ncz, plane_threads(tile_x), gradmax_smem_bytes(tile_x), nsm);
     const int chunk_z = (int)((ncz + nch - 1) / nch);
     nch = (ncz + chunk_z - 1) / chunk_z;
-    // the launch grid is (y tiles, x tiles, z chunks); CUDA limits its second
-    // and third dimensions to 65535
-    if (nxt > 65535 || nch > 65535) {
+    // the documented limits, in tiles of 32 x 32 cells and z chunks (the launch
+    // grid is (tiles of a plane, 1, z chunks), and CUDA limits its third
+    // dimension to 65535)
+    if (nxt32 > 65535 || nch > 65535) {
         snprintf(msg, sizeof(msg),
-                 "grid %dx%dx%d needs %d x tiles and %lld z chunks; the launch allows at most 65535",
-                 nx, ny, nz, nxt, nch);
+                 "grid %dx%dx%d needs %d x tiles and %lld z chunks; a call takes at most 65535",
+                 nx, ny, nz, nxt32, nch);
         return report(err, errlen, QP3D_ERR_ARG, msg);
     }
 
@@ -206,7 +208,7 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
     p.wait_ns = g_wait_ns;
     p.hold_plane = g_hold_plane;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    dim3 grid(nyt, nxt, (unsigned)nch);
+    dim3 grid((unsigned)tiles, 1, (unsigned)nch);
     // Through L1 as long as the volume stays in L2 (240x240x190: 49 us a call
     // against 60 from staged planes), from staged planes beyond, where their
     // loads ahead of use pay (460x460x360: 280 against 264); the hook that
