@@ -200,6 +200,7 @@ static int ensure_defer(qp3d_ctx *ctx)
     if (n <= ctx->defer_entries && segs <= ctx->defer_segs) return QP3D_OK;
     CK(cudaStreamSynchronize(ctx->stream));
     free_defer(ctx);
+    if (ctx->fail_alloc) CK(cudaErrorMemoryAllocation);   // test hook
     CK(cudaMalloc(&ctx->dkey, n * sizeof(uint2)));
     CK(cudaMalloc(&ctx->dval, n * sizeof(float4)));
     CK(cudaMalloc(&ctx->dcount, segs * sizeof(unsigned)));
@@ -243,6 +244,7 @@ int qp3d_internal_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m)
     bool same = ctx->loaded && ctx->g.nx == g->nx && ctx->g.ny == g->ny && ctx->g.nz == g->nz &&
                 ctx->g.nt == g->nt && ctx->g.pml == g->pml && ctx->half_loaded == half;
     if (!same) free_shot(ctx);
+    ctx->loaded = false;   // until everything below has succeeded
     ctx->g = *g;
     ctx->ldy = (g->ny + 31) & ~31;
     ctx->plane = (long long)g->nx * ctx->ldy;
@@ -344,6 +346,7 @@ int qp3d_internal_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m)
             if (*d) cudaFree(*d);
             *d = nullptr;
             *cap = 0;
+            if (ctx->fail_alloc) CK(cudaErrorMemoryAllocation);   // test hook
             CK(cudaMalloc(d, v.size() * sizeof(SrcEntry)));
             *cap = v.size();
         }
@@ -1075,6 +1078,7 @@ extern "C" int qp3d_tune(qp3d_ctx *ctx, const char *key, int value)
     else if (!strcmp(key, "arith") && (value == kArithRef || value == kArithFast)) ctx->arith = value;
     else if (!strcmp(key, "wait_limit_us") && value >= 0) ctx->wait_ns = 1000ull * (unsigned)value;
     else if (!strcmp(key, "test_hold_plane") && value >= -1) ctx->hold_plane = value + 1;
+    else if (!strcmp(key, "test_fail_alloc") && (value == 0 || value == 1)) ctx->fail_alloc = value;
     else if (!strcmp(key, "adj_ckpt_bf16") && (value == 0 || value == 1)) ctx->adj_bf16 = value;
     else if (!strcmp(key, "adj_keep_all") && value >= -1 && value <= 1) ctx->adj_keep = value;
     else if (!strcmp(key, "adj_live") && (value == 0 || value == 1)) ctx->adj_live = value;
@@ -1084,9 +1088,9 @@ extern "C" int qp3d_tune(qp3d_ctx *ctx, const char *key, int value)
         CK(cudaStreamSynchronize(ctx->stream));
         plan_launch(ctx);
         int rc = ensure_defer(ctx);
-        if (rc) return rc;
-        for (int i = 0; i < 3; ++i)
-            if ((rc = make_tmap(ctx, ctx->U[i], &ctx->tm[i]))) return rc;
+        for (int i = 0; i < 3 && !rc; ++i) rc = make_tmap(ctx, ctx->U[i], &ctx->tm[i]);
+        if (rc) ctx->loaded = false;   // its lists or maps are not those of the plan
+        return rc;
     }
     return QP3D_OK;
 }
@@ -1105,6 +1109,7 @@ extern "C" int qp3d_tune_get(const qp3d_ctx *ctx, const char *key)
     if (!strcmp(key, "wait_limit_us"))
         return (int)((ctx->wait_ns ? ctx->wait_ns : 2000000000ull) / 1000ull);
     if (!strcmp(key, "test_hold_plane")) return ctx->hold_plane - 1;
+    if (!strcmp(key, "test_fail_alloc")) return ctx->fail_alloc;
     if (!strcmp(key, "adj_ckpt_bf16")) return ctx->adj_bf16;
     if (!strcmp(key, "adj_keep_all")) return ctx->adj_keep;
     if (!strcmp(key, "adj_live")) return ctx->adj_live;

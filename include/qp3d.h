@@ -240,7 +240,9 @@ long long qp3d_ctx_launch_count(const qp3d_ctx *ctx);
  * "wait_limit_us" (limit of the kernels' bounded waits, 0: 2 s) and
  * "test_hold_plane" (test hook: a plane index that the first CTA of each
  * launch never loads, so that its waits run out and the step reports
- * QP3D_ERR_TIMEOUT; -1: none). */
+ * QP3D_ERR_TIMEOUT; -1: none).  "test_fail_alloc" (test hook, 1: the lists of a
+ * loaded shot cannot grow).  When a re-plan of the loaded shot ("tile_x",
+ * "chunks") or a load fails, no shot is loaded afterwards. */
 int qp3d_tune(qp3d_ctx *ctx, const char *key, int value);
 int qp3d_tune_get(const qp3d_ctx *ctx, const char *key);
 
