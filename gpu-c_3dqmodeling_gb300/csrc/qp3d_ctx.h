@@ -153,12 +153,16 @@ inline int ctx_fail(qp3d_ctx *c, int code, const char *fmt, ...)
     return code;
 }
 
+// The runtime's last error is taken back: the next call's launches would
+// otherwise report it as theirs.
 #define CK(call)                                                                           \
     do {                                                                                   \
         cudaError_t e_ = (call);                                                           \
-        if (e_ != cudaSuccess)                                                             \
+        if (e_ != cudaSuccess) {                                                           \
+            (void)cudaGetLastError();                                                      \
             return ctx_fail(ctx, e_ == cudaErrorMemoryAllocation ? QP3D_ERR_NOMEM : QP3D_ERR_CUDA, \
                         "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+        }                                                                                  \
     } while (0)
 
 // launch a library kernel: check it and count it
