@@ -20,11 +20,9 @@
 #include "qp3d_ctx.h"
 
 #include <algorithm>
-#include <atomic>
 #include <cstring>
 #include <map>
 #include <string>
-#include <thread>
 #include <vector>
 
 using namespace qp3d;
@@ -547,30 +545,15 @@ extern "C" int qp3d_batch(qp3d_ctx *ctx, int nshots, const qp3d_shot *shots)
         if (g.pml > 0 && (!m.dlr || !m.ddlr || !m.dtb || !m.ddtb || !m.dfb || !m.ddfb))
             return ctx_fail(ctx, QP3D_ERR_ARG, "shot %d: missing PML profiles", i);
     }
-    // the shots' sources, one shot per host thread at a time
+    // the shots' sources
     std::vector<std::vector<SrcEntry>> sources(nshots);
-    {
-        std::atomic<int> next{0};
-        auto scan = [&] {
-            for (int i; (i = next++) < nshots;)
-                if (shots[i].model.source)
-                    scan_source_volume(shots[i].model.source, shots[i].geom.nx, shots[i].geom.ny,
-                                       shots[i].geom.nz, sources[i], 1);
-        };
-        long long cells = 0;
-        for (int i = 0; i < nshots; ++i)
-            cells += (long long)shots[i].geom.nx * shots[i].geom.ny * shots[i].geom.nz;
-        const unsigned hw = std::thread::hardware_concurrency();
-        const int nth = (int)std::min({16ll, (long long)(hw ? hw : 1u), (long long)nshots,
-                                       (cells + (1 << 22) - 1) >> 22});
-        std::vector<std::thread> th;
-        try {
-            for (int t = 1; t < nth; ++t) th.emplace_back(scan);
-        } catch (...) {   // no more threads: the ones there are scan all
-        }
-        scan();
-        for (auto &t : th) t.join();
+    std::vector<SourceVolume> volumes;
+    for (int i = 0; i < nshots; ++i) {
+        const qp3d_geom &g = shots[i].geom;
+        if (const float *s = shots[i].model.source)
+            volumes.push_back({s, g.nx, g.ny, g.nz, &sources[i]});
     }
+    scan_source_volumes(volumes);
     for (int i = 0; i < nshots; ++i) {
         const qp3d_geom &g = shots[i].geom;
         const qp3d_model &m = shots[i].model;

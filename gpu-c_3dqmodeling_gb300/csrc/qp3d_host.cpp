@@ -11,6 +11,7 @@
 #include "qp3d_exact.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -23,52 +24,73 @@ namespace qp3d {
 
 // The reference adds the whole source volume every step
 // (CPU_function.c:326-338); its non-zero samples are the sparse source.
-// Planes are split over threads and the lists joined in plane order, so the
+// Every volume is cut into slabs of planes of up to 4 M samples, which host
+// threads take in turn, and the slabs' lists are joined in plane order, so the
 // order is that of one sequential scan.  A thread costs 50 us to start and
 // scans 4 M samples in about 1 ms, so a small volume takes none (with 16
 // threads for every volume a shot of 26x22x18 cells spent half of its load
-// here, 0.8 ms).  Rows are passed over 16 samples at a time: a sample is
+// here, 0.8 ms), and one large volume among small ones takes as many as all
+// of them together.  Rows are passed over 16 samples at a time: a sample is
 // non-zero when any bit but its sign is set.
-void scan_source_volume(const float *s, int nx, int ny, int nz, std::vector<SrcEntry> &out,
-                        int max_threads)
+void scan_source_volumes(const std::vector<SourceVolume> &vols)
 {
-    out.clear();
-    const unsigned hw = std::thread::hardware_concurrency();
-    const long long n = (long long)nx * ny * nz;
-    const int nth = (int)std::max(1ll, std::min({(long long)max_threads, (long long)(hw ? hw : 1u),
-                                                 (n + (1 << 22) - 1) >> 22}));
-    std::vector<std::vector<SrcEntry>> part(nth);
-    auto work = [&](int t) {
-        const int z0 = (int)((long long)nz * t / nth), z1 = (int)((long long)nz * (t + 1) / nth);
-        for (int z = z0; z < z1; ++z)
-            for (int x = 0; x < nx; ++x) {
-                const float *row = s + ((size_t)z * nx + x) * ny;
-                for (int y = 0; y < ny;) {
-                    if (y + 16 <= ny) {
-                        uint32_t b[16], any = 0;
-                        memcpy(b, row + y, sizeof(b));
-                        for (int i = 0; i < 16; ++i) any |= b[i] << 1;
+    struct Slab {
+        const SourceVolume *v;
+        int z0, z1;
+        std::vector<SrcEntry> found;
+    };
+    std::vector<Slab> slabs;
+    long long all = 0;
+    for (const SourceVolume &v : vols) {
+        v.out->clear();
+        const long long n = (long long)v.nx * v.ny * v.nz;
+        const int parts = (int)std::min((long long)v.nz, (n + (1 << 22) - 1) >> 22);
+        for (int t = 0; t < parts; ++t)
+            slabs.push_back({&v, (int)((long long)v.nz * t / parts),
+                             (int)((long long)v.nz * (t + 1) / parts), {}});
+        all += n;
+    }
+    auto scan = [](Slab &b) {
+        const SourceVolume &v = *b.v;
+        for (int z = b.z0; z < b.z1; ++z)
+            for (int x = 0; x < v.nx; ++x) {
+                const float *row = v.s + ((size_t)z * v.nx + x) * v.ny;
+                for (int y = 0; y < v.ny;) {
+                    if (y + 16 <= v.ny) {
+                        uint32_t u[16], any = 0;
+                        memcpy(u, row + y, sizeof(u));
+                        for (int i = 0; i < 16; ++i) any |= u[i] << 1;
                         if (!any) {
                             y += 16;
                             continue;
                         }
                     }
-                    const int e = std::min(ny, y + 16);
+                    const int e = std::min(v.ny, y + 16);
                     for (; y < e; ++y)
-                        if (row[y] != 0.0f) part[t].push_back(SrcEntry{x, y, z, row[y]});
+                        if (row[y] != 0.0f) b.found.push_back(SrcEntry{x, y, z, row[y]});
                 }
             }
     };
+    std::atomic<size_t> next{0};
+    auto work = [&] {
+        for (size_t i; (i = next++) < slabs.size();) scan(slabs[i]);
+    };
+    const unsigned hw = std::thread::hardware_concurrency();
+    const long long nth = std::min({16ll, (long long)(hw ? hw : 1u), (all + (1 << 22) - 1) >> 22,
+                                    (long long)slabs.size()});
     std::vector<std::thread> th;
-    int started = 1;
     try {
-        for (int t = 1; t < nth; ++t, ++started) th.emplace_back(work, t);
-    } catch (...) {   // no more threads: this one scans the rest
+        for (long long t = 1; t < nth; ++t) th.emplace_back(work);
+    } catch (...) {   // no more threads: the ones there scan all
     }
-    work(0);
+    work();
     for (auto &t : th) t.join();
-    for (int t = started; t < nth; ++t) work(t);
-    for (auto &p : part) out.insert(out.end(), p.begin(), p.end());
+    for (Slab &b : slabs) b.v->out->insert(b.v->out->end(), b.found.begin(), b.found.end());
+}
+
+void scan_source_volume(const float *s, int nx, int ny, int nz, std::vector<SrcEntry> &out)
+{
+    scan_source_volumes({{s, nx, ny, nz, &out}});
 }
 
 // FD tables with the 1/h factors folded in.  The reference divides every tap

@@ -278,10 +278,15 @@ cudaError_t launch_params_dense(const float *vp, const float *eps, const float *
                                 cudaStream_t stream);
 cudaError_t launch_to_half_dense(const float *a, __half *h, int nx, int ny, int nz, int ldy,
                                  cudaStream_t stream);
-// Every non-zero sample of a dense [nz][nx][ny] source volume, in index order
-// (z, then x, then y), scanned by up to max_threads host threads.
-void scan_source_volume(const float *s, int nx, int ny, int nz, std::vector<SrcEntry> &out,
-                        int max_threads = 16);
+// Every non-zero sample of dense [nz][nx][ny] source volumes, of each in index
+// order (z, then x, then y), scanned by several host threads.
+struct SourceVolume {
+    const float *s;
+    int nx, ny, nz;
+    std::vector<SrcEntry> *out;
+};
+void scan_source_volumes(const std::vector<SourceVolume> &vols);
+void scan_source_volume(const float *s, int nx, int ny, int nz, std::vector<SrcEntry> &out);
 // Dynamic shared memory of a step kernel; nsrc = fused sources of the shot
 // (the per-CTA source list has room for all of them); and of a gradmax kernel.
 size_t plane_smem_bytes(int tile_x, int pml, int nsrc);
