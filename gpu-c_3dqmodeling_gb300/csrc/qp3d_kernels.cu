@@ -1365,15 +1365,15 @@ __device__ __forceinline__ bool step_tile(const TileMaps *tm, const PlaneParams 
 
     const int tid = threadIdx.x, lane = tid & 31;
     // A warp holds four rows of eight quads, or, in a last y tile of no more
-    // than four, two or one quads, eight, sixteen or 32 rows: the warps left
-    // over only pass the planes on.  (Decision words and the reference
+    // than four or two quads, eight or sixteen rows: the warps left over only
+    // pass the planes on.  (A last tile starts at ny - 6 or before: two quads.)  (Decision words and the reference
     // arithmetic's classes go by rows of eight.)  A step of 140^3 cells (last
     // tile 12 wide) 45.3 -> 42.5 us, 38x42x34 10.5 -> 10.1, 191x127x105 (31
     // wide) 35.7 -> 35.1, 240x240x190 (16) 107.5 -> 106.4.
     int lq = 3;
     if (AR == kArithFast && !DEC) {
         const int nq = (min(p.ny - y0, kTileY) + 3) >> 2;
-        lq = nq > 4 ? 3 : (nq > 2 ? 2 : nq - 1);
+        lq = nq > 4 ? 3 : (nq > 2 ? 2 : 1);
     }
     const int q = tid & ((1 << lq) - 1), r = tid >> lq, rt = min(r, tile_x - 1);
     const int nzc = z1 - z0;
