@@ -196,6 +196,7 @@ static int ensure_defer(qp3d_ctx *ctx)
 {
     const size_t segs = (size_t)ctx->nyt * ctx->nxt * ctx->nchunks;
     ctx->dcap = (unsigned)(ctx->tile_x * kTileY / 4 * ctx->chunk_z);
+    if (ctx->defer_cap > 0) ctx->dcap = std::min(ctx->dcap, (unsigned)ctx->defer_cap);
     const size_t n = segs * ctx->dcap;
     if (n <= ctx->defer_entries && segs <= ctx->defer_segs) return QP3D_OK;
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1078,6 +1079,7 @@ extern "C" int qp3d_tune(qp3d_ctx *ctx, const char *key, int value)
     else if (!strcmp(key, "arith") && (value == kArithRef || value == kArithFast)) ctx->arith = value;
     else if (!strcmp(key, "wait_limit_us") && value >= 0) ctx->wait_ns = 1000ull * (unsigned)value;
     else if (!strcmp(key, "test_hold_plane") && value >= -1) ctx->hold_plane = value + 1;
+    else if (!strcmp(key, "test_defer_cap") && value >= 0) ctx->defer_cap = value;
     else if (!strcmp(key, "test_fail_alloc") && (value == 0 || value == 1)) ctx->fail_alloc = value;
     else if (!strcmp(key, "adj_ckpt_bf16") && (value == 0 || value == 1)) ctx->adj_bf16 = value;
     else if (!strcmp(key, "adj_keep_all") && value >= -1 && value <= 1) ctx->adj_keep = value;
@@ -1109,6 +1111,7 @@ extern "C" int qp3d_tune_get(const qp3d_ctx *ctx, const char *key)
     if (!strcmp(key, "wait_limit_us"))
         return (int)((ctx->wait_ns ? ctx->wait_ns : 2000000000ull) / 1000ull);
     if (!strcmp(key, "test_hold_plane")) return ctx->hold_plane - 1;
+    if (!strcmp(key, "test_defer_cap")) return ctx->defer_cap;
     if (!strcmp(key, "test_fail_alloc")) return ctx->fail_alloc;
     if (!strcmp(key, "adj_ckpt_bf16")) return ctx->adj_bf16;
     if (!strcmp(key, "adj_keep_all")) return ctx->adj_keep;

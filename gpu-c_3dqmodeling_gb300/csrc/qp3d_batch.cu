@@ -232,6 +232,7 @@ int Runner::build_candidate(int c, std::vector<Plan *> &G)
                     w.z0 = z0;
                     w.z1 = std::min(z0 + cz, P.g.nz - kRadius);
                     w.dcap = (unsigned)(tx * kTileY / 4 * (w.z1 - w.z0));
+                    if (ctx->defer_cap > 0) w.dcap = std::min(w.dcap, (unsigned)ctx->defer_cap);
                     w.dbase = (unsigned)dbase;
                     dbase += w.dcap;
                     items.push_back(w);

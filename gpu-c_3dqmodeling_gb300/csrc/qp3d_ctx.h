@@ -116,6 +116,7 @@ struct qp3d_ctx {
     // (plane index + 1 in the first CTA of each grid launch; 0: none)
     unsigned long long wait_ns = 0;
     int hold_plane = 0;
+    int defer_cap = 0;               // test hook: entries per segment at the most (0: the plan's)
     int fail_alloc = 0;              // test hook: a loaded shot's lists cannot grow
     // threshold decisions of each step (qp3d_adjoint): 1 = record them into
     // dec_base + step * dec_words, 2 = replay them (no maximum is needed then)

@@ -241,7 +241,9 @@ long long qp3d_ctx_launch_count(const qp3d_ctx *ctx);
  * "test_hold_plane" (test hook: a plane index that the first CTA of each
  * launch never loads, so that its waits run out and the step reports
  * QP3D_ERR_TIMEOUT; -1: none).  "test_fail_alloc" (test hook, 1: the lists of a
- * loaded shot cannot grow).  When a re-plan of the loaded shot ("tile_x",
+ * loaded shot cannot grow), "test_defer_cap" (test hook, from the next load or
+ * qp3d_batch: room for so many undecided cells per tile column, so that steps
+ * with more are re-run; 0: a quarter of the column).  When a re-plan of the loaded shot ("tile_x",
  * "chunks") or a load fails, no shot is loaded afterwards. */
 int qp3d_tune(qp3d_ctx *ctx, const char *key, int value);
 int qp3d_tune_get(const qp3d_ctx *ctx, const char *key);
