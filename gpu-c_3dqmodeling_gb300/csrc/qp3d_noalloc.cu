@@ -186,14 +186,21 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
         }
     }
 
-    TileMaps tm;
-    CUresult cr = encode_tile_maps(g_encode, d_u, nx, ny, nz, ldy, tile_x, &tm);
-    if (cr == CUDA_ERROR_INVALID_CONTEXT) {   // a host thread that has used no CUDA yet
-        (void)cudaFree(nullptr);              // gives it the device's context
-        cr = encode_tile_maps(g_encode, d_u, nx, ny, nz, ldy, tile_x, &tm);
+    // Through L1 as long as the volume stays in L2 (240x240x190: 49 us a call
+    // against 60 from staged planes), from staged planes beyond, where their
+    // loads ahead of use pay (460x460x360: 280 against 264); the hook that
+    // withholds a plane is the staged form's.
+    const bool direct = (long long)nx * ldy * nz <= kDirectMaxCells && g_hold_plane == 0;
+    TileMaps tm{};
+    if (!direct) {   // the tensor maps of the staged form
+        CUresult cr = encode_tile_maps(g_encode, d_u, nx, ny, nz, ldy, tile_x, &tm);
+        if (cr == CUDA_ERROR_INVALID_CONTEXT) {   // a host thread that has used no CUDA yet
+            (void)cudaFree(nullptr);              // gives it the device's context
+            cr = encode_tile_maps(g_encode, d_u, nx, ny, nz, ldy, tile_x, &tm);
+        }
+        if (cr != CUDA_SUCCESS)
+            return report(err, errlen, QP3D_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     }
-    if (cr != CUDA_SUCCESS)
-        return report(err, errlen, QP3D_ERR_CUDA, "cuTensorMapEncodeTiled failed");
 
     PlaneParams p;
     memset(&p, 0, sizeof(p));
@@ -209,11 +216,6 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
     p.hold_plane = g_hold_plane;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     dim3 grid((unsigned)tiles, 1, (unsigned)nch);
-    // Through L1 as long as the volume stays in L2 (240x240x190: 49 us a call
-    // against 60 from staged planes), from staged planes beyond, where their
-    // loads ahead of use pay (460x460x360: 280 against 264); the hook that
-    // withholds a plane is the staged form's.
-    const bool direct = (long long)nx * ldy * nz <= kDirectMaxCells && g_hold_plane == 0;
     cudaError_t e = direct
         ? launch_gradmax_direct(d_u, nx, ny, nz, ldy, p.k, nsm, s, slot.scratch(), d_max,
                                 slot.flags())

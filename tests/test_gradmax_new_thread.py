@@ -13,8 +13,8 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-def test_first_call_of_a_thread():
-    n = 32
+@pytest.mark.parametrize("n", [32, 300])    # through L1; from staged planes
+def test_first_call_of_a_thread(n):
     u = torch.zeros((n, n, n), device="cuda")
     u[16, 16, 16] = 2.0
     c = np.zeros(36, np.float32)
