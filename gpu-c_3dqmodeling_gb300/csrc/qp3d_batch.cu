@@ -49,6 +49,7 @@ struct Plan {
     int ldy = 0, hx = 0, hy = 0;
     long long plane = 0, vol = 0;
     std::vector<SrcEntry> src;
+    std::vector<float4> layers;     // PML layer coefficients
     size_t bytes = 0;               // device bytes of this shot
     size_t defer_entries = 0;
     BatchShot d{};                  // device pointers, filled per group
@@ -184,6 +185,11 @@ class Runner {
     Launch L[kNumCands];
     int nshots = 0;
     Coefs coefs{};
+    // sources of copies, kept until the group has run: a device that reads
+    // pageable memory itself need not have read them when the copy call returns
+    std::vector<WorkItem> items[kNumCands];
+    std::vector<TileMaps> maps[kNumCands];
+    std::vector<BatchShot> hshots;
 
     int build_candidate(int c, std::vector<Plan *> &G);
     BatchArgs args(int c, int queue, bool spec) const
@@ -206,8 +212,10 @@ class Runner {
 
 int Runner::build_candidate(int c, std::vector<Plan *> &G)
 {
-    std::vector<WorkItem> items;
-    std::vector<TileMaps> tms(3 * G.size());
+    std::vector<WorkItem> &items = this->items[c];
+    std::vector<TileMaps> &tms = maps[c];
+    items.clear();
+    tms.resize(3 * G.size());
     int max_tile = 1;
     size_t smem = 0;
     for (size_t s = 0; s < G.size(); ++s) {
@@ -282,6 +290,7 @@ int Runner::enqueue_step(int c, bool spec)
 
 int Runner::run_group(std::vector<Plan *> &G, const Coefs &kc, const qp3d_shot *shots)
 {
+    const StreamDrain drain{ctx};   // for hshots, the items and the maps
     int rc;
     nshots = (int)G.size();
     coefs = kc;
@@ -311,7 +320,7 @@ int Runner::run_group(std::vector<Plan *> &G, const Coefs &kc, const qp3d_shot *
 
     // ---- per shot: layout, model upload, derived inputs, zero state
     Carver cv{static_cast<char *>(B->arena)};
-    std::vector<BatchShot> hshots(nshots);
+    hshots.resize(nshots);
     int nt_max = 0;
     for (int s = 0; s < nshots; ++s) {
         Plan &P = *G[s];
@@ -346,11 +355,11 @@ int Runner::run_group(std::vector<Plan *> &G, const Coefs &kc, const qp3d_shot *
         CK(cudaMemcpyAsync(d.spec_err, first, sizeof(first), cudaMemcpyHostToDevice,
                            ctx->stream));
         if (P.g.pml > 0) {
-            std::vector<float4> tab(3 * P.g.pml);
+            std::vector<float4> &tab = P.layers;   // outlives the copy
+            tab.resize(3 * P.g.pml);
             derive_layers(m.dlr, m.ddlr, P.g.pml, P.g.dt, tab.data());
             derive_layers(m.dfb, m.ddfb, P.g.pml, P.g.dt, tab.data() + P.g.pml);
             derive_layers(m.dtb, m.ddtb, P.g.pml, P.g.dt, tab.data() + 2 * P.g.pml);
-            // pageable source: staged before the call returns, ordered on the stream
             CK(cudaMemcpyAsync(const_cast<float4 *>(d.layers), tab.data(),
                                sizeof(float4) * tab.size(), cudaMemcpyHostToDevice, ctx->stream));
         }
