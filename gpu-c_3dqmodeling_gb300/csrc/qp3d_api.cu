@@ -252,8 +252,9 @@ int qp3d_internal_load(qp3d_ctx *ctx, const qp3d_geom *g, const qp3d_model *m)
     ctx->vol = ctx->plane * g->nz;
     ctx->hx = g->nx - 2 * g->pml;
     ctx->hy = g->ny - 2 * g->pml;
-    // the kernels index cells with 32 bits; the state of 2^32 cells (14 volumes
-    // and the parameters) is more than the device holds anyway
+    // the kernels index cells with 32 bits; 2^32 cells take 272 GiB with half
+    // parameters (14 volumes of state, the parameters, the deferred-cell lists),
+    // about all the device has
     if (ctx->vol >= (1ll << 32)) {
         free_shot(ctx);
         return ctx_fail(ctx, QP3D_ERR_NOMEM, "grid of %lld padded cells", ctx->vol);

@@ -63,7 +63,7 @@ struct BatchState {
     BatchShot *d_shots = nullptr;
     PlaneParams *d_pp = nullptr;
     int shots_cap = 0;
-    int *d_ctr = nullptr;           // [0] step counter, [4..8) work queues
+    int *d_ctr = nullptr;           // [0] step counter, [1] re-run queue
     WorkItem *d_work[kNumCands] = {};
     size_t work_cap[kNumCands] = {};
     unsigned *d_count = nullptr;    // deferred cells per work item
@@ -192,7 +192,7 @@ class Runner {
     std::vector<BatchShot> hshots;
 
     int build_candidate(int c, std::vector<Plan *> &G);
-    BatchArgs args(int c, int queue, bool spec) const
+    BatchArgs args(int c) const
     {
         BatchArgs a;
         a.k = coefs;
@@ -202,8 +202,7 @@ class Runner {
         a.nwork = L[c].nwork;
         a.dcount = B->d_count;
         a.nshots = nshots;
-        a.spec = spec ? 1 : 0;
-        a.queue = B->d_ctr + 4 + queue;
+        a.queue = B->d_ctr + 1;
         a.arith = ctx->arith;
         return a;
     }
@@ -276,14 +275,14 @@ int Runner::build_candidate(int c, std::vector<Plan *> &G)
 int Runner::enqueue_step(int c, bool spec)
 {
     const Launch &l = L[c];
-    CKL(launch_batch_prepare(B->d_shots, nshots, B->d_pp, B->d_ctr, B->d_ctr + 4, spec ? 1 : 0,
+    CKL(launch_batch_prepare(B->d_shots, nshots, B->d_pp, B->d_ctr, B->d_ctr + 1, spec ? 1 : 0,
                              ctx->stream));
     if (spec) {
-        CKL(launch_batch_plane(2, args(c, 1, true), l.threads, l.smem, ctx->stream));
-        CKL(launch_batch_resolve(args(c, 2, true), l.grid, l.threads, l.smem, ctx->stream));
+        CKL(launch_batch_plane(2, args(c), l.threads, l.smem, ctx->stream));
+        CKL(launch_batch_resolve(args(c), l.grid, l.threads, l.smem, ctx->stream));
     } else {
-        CKL(launch_batch_plane(0, args(c, 0, false), l.threads, l.smem, ctx->stream));
-        CKL(launch_batch_plane(1, args(c, 1, false), l.threads, l.smem, ctx->stream));
+        CKL(launch_batch_plane(0, args(c), l.threads, l.smem, ctx->stream));
+        CKL(launch_batch_plane(1, args(c), l.threads, l.smem, ctx->stream));
     }
     return QP3D_OK;
 }
@@ -314,7 +313,7 @@ int Runner::run_group(std::vector<Plan *> &G, const Coefs &kc, const qp3d_shot *
         CK(cudaMalloc(&B->d_pp, sizeof(PlaneParams) * nshots));
         B->shots_cap = nshots;
     }
-    if (!B->d_ctr) CK(cudaMalloc(&B->d_ctr, 8 * sizeof(int)));
+    if (!B->d_ctr) CK(cudaMalloc(&B->d_ctr, 2 * sizeof(int)));
     if (!ctx->errword) CK(cudaMalloc(&ctx->errword, sizeof(unsigned)));
     CK(cudaMemsetAsync(ctx->errword, 0, sizeof(unsigned), ctx->stream));
 
@@ -374,7 +373,7 @@ int Runner::run_group(std::vector<Plan *> &G, const Coefs &kc, const qp3d_shot *
     }
     CK(cudaMemcpyAsync(B->d_shots, hshots.data(), sizeof(BatchShot) * nshots,
                        cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemsetAsync(B->d_ctr, 0, 8 * sizeof(int), ctx->stream));
+    CK(cudaMemsetAsync(B->d_ctr, 0, 2 * sizeof(int), ctx->stream));
     for (int c = 0; c < kNumCands; ++c)
         if ((rc = build_candidate(c, G))) return rc;
 

@@ -199,8 +199,8 @@ struct BatchArgs {
     const WorkItem *work;
     int nwork;
     unsigned *dcount;         // deferred cells per work item
-    int nshots, spec;
-    int *queue;               // next work item (zeroed by the prepare kernel)
+    int nshots;
+    int *queue;               // next item of the re-run (zeroed by the prepare kernel)
     int arith;                // Arith of every shot of the batch
 };
 
@@ -318,7 +318,7 @@ inline CUresult encode_tile_maps(EncodeTiledFn encode, const float *base, int nx
 // resolution of a speculative step runs on grid persistent CTAs.
 size_t batch_smem_bytes(int tile_x, int pml, int nsrc);
 cudaError_t launch_batch_prepare(const BatchShot *shots, int nshots, PlaneParams *pp, int *ctr,
-                                 int *queues, int spec, cudaStream_t stream);
+                                 int *queue, int spec, cudaStream_t stream);
 cudaError_t launch_batch_plane(int kind, const BatchArgs &b, int threads, size_t smem,
                                cudaStream_t stream);
 cudaError_t launch_batch_resolve(const BatchArgs &b, int grid, int threads, size_t smem,

@@ -779,12 +779,10 @@ __device__ __forceinline__ void taps_next(Taps &T, const Pipe<G> &P, int t)   //
 }
 
 // ---------------------------------------------------------------------------
-// max|grad u| over one tile column [z0, z1), a thread's own maximum in mx.
-// The grid kernels run one column per CTA; the batched kernel runs many
-// (REUSE: barriers invalidated at the end).  Returns false (in every thread)
-// when a wait timed out.
+// max|grad u| over one tile column [z0, z1), one per CTA, a warp's maximum in
+// mx.  Returns false (in every thread) when a wait timed out.
 // ---------------------------------------------------------------------------
-template <bool REUSE, int AR>
+template <int AR>
 __device__ __forceinline__ bool gradmax_tile(const TileMaps *tm, const PlaneParams &p,
                                              const Coefs &k, int tile_x, int y0, int x0, int z0,
                                              int z1, unsigned char *smem, float &mx)
@@ -795,7 +793,7 @@ __device__ __forceinline__ bool gradmax_tile(const TileMaps *tm, const PlanePara
     const SmemLayout L = smem_layout(tile_x, 0, 0, 0, kGradmaxGroups);
     Pipe<kGradmaxGroups> P;
     pipe_setup(P, smem, L, tile_x, y0, x0, z0, nzc);
-    if (!REUSE) pipe_hooks(P, p.wait_ns, p.hold_plane);
+    pipe_hooks(P, p.wait_ns, p.hold_plane);
     if (tid == 0) {
         pipe_init(P);
         pipe_start(P, tm);
@@ -824,7 +822,6 @@ __device__ __forceinline__ bool gradmax_tile(const TileMaps *tm, const PlanePara
         pipe_release(P, tm, t);
     }
     ok = pipe_finish(P, ok, p.err);
-    if (REUSE && tid == 0 && ok) pipe_inval(P);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     return ok;
@@ -847,8 +844,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int z1 = min(z0 + p.chunk_z, p.nz - kRadius);
     if (z0 >= z1) return;
     float mx;
-    gradmax_tile<false, AR>(&tm, p, p.k, p.tile_x, blockIdx.x * kTileY,
-                            kRadius + blockIdx.y * p.tile_x, z0, z1, smem, mx);
+    gradmax_tile<AR>(&tm, p, p.k, p.tile_x, blockIdx.x * kTileY,
+                     kRadius + blockIdx.y * p.tile_x, z0, z1, smem, mx);
     gradmax_publish(p, mx);
 }
 
@@ -884,8 +881,8 @@ __global__ void __launch_bounds__(kQuadsY * kGradmaxTileX, 4)
     const int z1 = min(z0 + p.chunk_z, p.nz - kRadius);
     if (z0 < z1) {
         float mx;
-        gradmax_tile<false, kArithFast>(&tm, p, p.k, p.tile_x, yt * kTileY,
-                                        kRadius + xt * p.tile_x, z0, z1, smem, mx);
+        gradmax_tile<kArithFast>(&tm, p, p.k, p.tile_x, yt * kTileY,
+                                 kRadius + xt * p.tile_x, z0, z1, smem, mx);
         if ((threadIdx.x & 31) == 0 && mx > 0.0f) atomicMax(&sc->max_bits, __float_as_uint(mx));
     }
     gradmax_deliver(sc, out, host_flags);
@@ -1343,9 +1340,10 @@ __device__ __noinline__ float scalar_s_call(float Ux, float Uy, float Uz, float 
     return xr::scalar_s(Ux, Uy, Uz, m2, e, r);
 }
 
-// One tile column [z0, z1) of the step.  The grid kernel below runs one per
-// CTA; the batched kernel runs many per CTA (REUSE: barriers invalidated at
-// the end, return value uniform over the CTA; false = a wait timed out).
+// One tile column [z0, z1) of the step.  The step kernels, single and batched,
+// run one per CTA; the re-runs in the resolution kernels run many (REUSE:
+// barriers invalidated at the end).  The return value is the same in every
+// thread; false = a wait timed out.
 // AR: kArithRef (the reference CPU operators' roundings, qp3d_exact.h) or
 // kArithFast (folded coefficients, fused multiply-adds, one reciprocal in S).
 // DEC: the step's threshold decisions are kept or replayed (p.dec_out,
@@ -2074,7 +2072,7 @@ __global__ void qp3d_to_half_dense_kernel(const float *a, __half *h, int ny, lon
 //   qp3d_batch_prepare_kernel   reads the step counter k, writes every shot's
 //                               PlaneParams of step k (buffer rotation,
 //                               wavelet[k], record plane, per-step slots),
-//                               zeroes the work queues, sets the counter to
+//                               zeroes the re-run queue, sets the counter to
 //                               k + 1.  The step is therefore the same
 //                               sequence of launches for every k and can be
 //                               captured once in a CUDA graph.
@@ -2085,7 +2083,7 @@ __global__ void qp3d_to_half_dense_kernel(const float *a, __half *h, int ny, lon
 //   qp3d_batch_resolve_kernel   the resolution of a speculative step.
 // ---------------------------------------------------------------------------
 __global__ void qp3d_batch_prepare_kernel(const BatchShot *shots, int nshots, PlaneParams *pp,
-                                          int *ctr, int *queues, int spec)
+                                          int *ctr, int *queue, int spec)
 {
     pdl_trigger();
     pdl_wait();
@@ -2142,7 +2140,7 @@ __global__ void qp3d_batch_prepare_kernel(const BatchShot *shots, int nshots, Pl
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        queues[0] = queues[1] = queues[2] = queues[3] = 0;
+        *queue = 0;
         *ctr = k + 1;
     }
 }
@@ -2181,7 +2179,7 @@ __device__ __forceinline__ bool batch_item(const BatchArgs &b, int it, unsigned 
     tm += p.ucur;
     if (KIND == 0) {
         float mx;
-        const bool ok = gradmax_tile<REUSE, AR>(tm, p, b.k, w.tile_x, w.y0, w.x0, w.z0, w.z1, body, mx);
+        const bool ok = gradmax_tile<AR>(tm, p, b.k, w.tile_x, w.y0, w.x0, w.z0, w.z1, body, mx);
         gradmax_publish(p, mx);
         return ok;
     }
@@ -2258,25 +2256,23 @@ __global__ void __launch_bounds__(kStepThreads, 2)
 // ---------------------------------------------------------------------------
 // Adjoint (qp3d_adjoint.cu drives them).  Pass A, per cell: the residual of
 // the step is injected at the receivers; the scalar operator of step k is
-// rebuilt from u^k (frozen: its decision and unit normal are those of the
-// forward, its eps/delta dependence is differentiated); the PML recursions
-// and the interior leapfrog are transposed term by term; each derivative the
-// update took of u^k leaves a coefficient field; the gradient terms
-// lambda * (d update / d m) are summed.  Pass B, per cell: the transposed
+// rebuilt from u^k (its decision is the forward's; its dependence on eps, delta
+// and, with the live operator, the unit normal is differentiated); the PML
+// recursions and the interior leapfrog are transposed term by term; each
+// derivative the update took of u^k leaves a coefficient field; the gradient
+// terms lambda * (d update / d m) are summed.  Pass B, per cell: the transposed
 // stencils of the six coefficient fields (second derivatives: the stencil
 // itself; first derivatives: its negative), zero outside the volume.
-// Pass A writes only what a cell can make non-zero (PML state and first-
-// derivative fields at PML cells, u_prev and second-derivative fields at
-// updated cells); the caller zeroes every buffer once, so the entries never
-// written stay zero in both buffers of each pair.
+// Pass A writes the quads with updated cells: the adjoint of u, Cxx and Czz; Cyy
+// where it can differ from Cxx; Cx, Cy, Cz with the live operator, otherwise
+// where a cell is of the shell, as the PML state.  (The adjoint of u_prev is not
+// kept, see AdjParams.)  The caller zeroes every buffer once, so the entries
+// never written stay zero in all buffers that take turns.
 // The gradient is checked against the FP64 adjoint by cosine, not bit for
 // bit, so these kernels take the cheaper arithmetic: fast division
 // (__fdividef, 2 ulp) in S and its derivatives, fused multiply-adds in the
-// transposed stencils.  Both passes are bound by the L1 load path and
-// instruction issue (31 and 63 gathered taps per cell), so each thread takes
-// four consecutive y cells with 16-byte loads (a quarter of the load
-// instructions); a shared-memory z-marching form (register queue along z)
-// was measured slower on GB300.
+// transposed stencils.  Pass A is bound by HBM, pass B by the latency of the
+// taps it gathers through L1 (see each).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float4 ldg4_or0(const float *f, long long j, bool ok)
 {
@@ -2898,10 +2894,10 @@ cudaError_t launch_fix_or_rerun(const TileMaps &tm, const PlaneParams &p, float 
 }
 
 cudaError_t launch_batch_prepare(const BatchShot *shots, int nshots, PlaneParams *pp, int *ctr,
-                                 int *queues, int spec, cudaStream_t stream)
+                                 int *queue, int spec, cudaStream_t stream)
 {
     return launch_pdl(qp3d_batch_prepare_kernel, dim3(1), 128, 0, stream, shots, nshots, pp, ctr,
-                      queues, spec);
+                      queue, spec);
 }
 
 template <int AR>
@@ -2978,7 +2974,12 @@ void plan_adjoint(AdjParams &a, int nsm)
     const size_t smem = smem_layout(a.tile_x, a.pml, 0, kAdjStreams).total;
     // Where there are several waves either way, short chunks keep more loads
     // and stores in flight: 5 planes 189 us on 240x240x190, 12 planes (the
-    // estimate's choice) 199.
+    // estimate's choice) 199.  On either side of the line, whole gradients of 120
+    // steps with 5 planes and with the estimate's: 300x300x200 (32 CTAs an SM)
+    // 80.7 and 83.4 ms, 240x240x190 (19) 54.3 and 56.0; below it, where the
+    // estimate is taken, 200x200x150 (10) 33.1 and 36.0, 150x150x150 (5.5) 20.9
+    // and 22.5, 130x130x110 (2.6) 13.4 and 12.8, 100x100x100 (1.4) 9.0 and 8.5: the
+    // crossover is near 4, and the line could lie there.
     const int n = tiles * ((ncz + 4) / 5) >= 12ll * nsm
                       ? (ncz + 4) / 5
                       : plan_chunks(tiles, ncz, std::max(192, plane_threads(a.tile_x)), smem, nsm);

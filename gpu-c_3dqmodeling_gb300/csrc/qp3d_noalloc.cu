@@ -186,10 +186,13 @@ extern "C" int qp3d_gradmax_noalloc(const float *d_u, int nx, int ny, int nz, in
         }
     }
 
-    // Through L1 as long as the volume stays in L2 (240x240x190: 49 us a call
-    // against 60 from staged planes), from staged planes beyond, where their
-    // loads ahead of use pay (460x460x360: 280 against 264); the hook that
-    // withholds a plane is the staged form's.
+    // Through L1 as long as the volume stays in L2, from staged planes beyond,
+    // where their loads ahead of use pay.  Calls in a loop, through L1 and staged:
+    // 240x240x190 (11 Mi cells) 42 and 56 us, 300x300x200 (18) 63 and 80,
+    // 300x300x262 (24) 99 and 99, 320x320x260 (25) 107 and 103, 400x400x300 (48)
+    // 185 and 173, 460x460x360 (76) 271 and 259.  (With L2 full of other data the
+    // two are closer, staged ahead: 65 and 63, 97 and 87, 121 and 105.)  The hook
+    // that withholds a plane is the staged form's.
     const bool direct = (long long)nx * ldy * nz <= kDirectMaxCells && g_hold_plane == 0;
     TileMaps tm{};
     if (!direct) {   // the tensor maps of the staged form
